@@ -355,6 +355,11 @@ k_spmv_wmerge_hot(MergeTables mt, const int64_t *__restrict__ offsets,
 constexpr int LOR_W = 4;
 constexpr int LOR_HEAD = 32;
 constexpr int LOR_CHUNK = 256;
+// general path (k_spmv_vector_general): rows longer than GEN_LONG run in
+// chunks of GEN_CHUNK, a lane's loads in batches of GEN_BATCH
+constexpr int GEN_LONG = 64;
+constexpr int GEN_CHUNK = 256;
+constexpr int GEN_BATCH = 4;
 
 template <bool VALUED>
 __global__ void __launch_bounds__(256)
@@ -420,63 +425,89 @@ k_lor_tail(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ ind
 	}
 }
 
-// chunk list of the lor path: per row beyond LOR_HEAD, ceil((len - HEAD) /
-// CHUNK) chunks; pass 1 counts (out == nullptr), pass 2 writes them at
-// positions taken from *count (any order: the results do not depend on it)
-__global__ void k_lor_chunks(const int64_t *__restrict__ offsets, int64_t m,
-	unsigned long long *count, int64_t *rows, int64_t *k0s) {
+// Chunk lists of the plan: per row of more than `longer` nonzeroes, its
+// nonzeroes from `head` on in chunks of `chunk`, consecutive in the list.
+// Pass 1 counts (rows == nullptr), pass 2 writes them at positions taken from
+// *count (any order of the rows: no result depends on it); first, when given,
+// lists each row's first chunk at a position from *nrows.
+__global__ void k_row_chunks(const int64_t *__restrict__ offsets, int64_t m, int64_t longer,
+	int64_t head, int64_t chunk, unsigned long long *count, unsigned long long *nrows,
+	int64_t *rows, int64_t *k0s, int64_t *first) {
 	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m;
 		 i += int64_t(gridDim.x) * blockDim.x) {
-		const int64_t b = offsets[i] + LOR_HEAD, e = offsets[i + 1];
-		if (e <= b) continue;
-		const int64_t n = (e - b + LOR_CHUNK - 1) / LOR_CHUNK;
+		const int64_t b = offsets[i] + head, e = offsets[i + 1];
+		if (e - offsets[i] <= longer) continue;
+		const int64_t n = (e - b + chunk - 1) / chunk;
 		const unsigned long long at = atomicAdd(count, (unsigned long long) n);
-		if (rows)
+		const unsigned long long l = atomicAdd(nrows, 1ull);
+		if (rows) {
 			for (int64_t c = 0; c < n; ++c) {
 				rows[at + c] = i;
-				k0s[at + c] = b + c * LOR_CHUNK;
+				k0s[at + c] = b + c * chunk;
 			}
+			if (first) first[l] = int64_t(at);
+		}
 	}
 }
 
-static void lor_release(alpb_spmv_plan_s *p) {
+static void lists_release(alpb_spmv_plan_s *p) {
 	cudaFree(p->lor_row);
 	cudaFree(p->lor_k0);
-	p->lor_row = nullptr;
-	p->lor_k0 = nullptr;
+	cudaFree(p->gen_row);
+	cudaFree(p->gen_k0);
+	cudaFree(p->gen_first);
+	p->lor_row = p->lor_k0 = p->gen_row = p->gen_k0 = p->gen_first = nullptr;
 	p->lor_n = -1;
+	p->gen_n = p->gen_rows = 0;
 }
 
-static int lor_build(alpb_spmv_plan_s *p, cudaStream_t s) {
-	lor_release(p);
+// the lor path's list (rows beyond their first LOR_HEAD nonzeroes) and the
+// general path's (rows of more than GEN_LONG, whole)
+static int lists_build(alpb_spmv_plan_s *p, cudaStream_t s) {
+	lists_release(p);
 	if (p->m == 0) {
 		p->lor_n = 0;
 		return ALPB_SUCCESS;
 	}
-	unsigned long long *cnt = nullptr, h = 0;
-	ALPB_CUDA(cudaMallocAsync(&cnt, 8, s));
-	ALPB_CUDA(cudaMemsetAsync(cnt, 0, 8, s));
-	k_lor_chunks<<<grid_for(p->m, 256, 4), 256, 0, s>>>(p->offsets, p->m, cnt, nullptr, nullptr);
+	const unsigned grid = grid_for(p->m, 256, 4);
+	unsigned long long *cnt = nullptr, h[4] = {0, 0, 0, 0};  // lor chunks, rows; general chunks, rows
+	ALPB_CUDA(cudaMallocAsync(&cnt, sizeof(h), s));
+	ALPB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(h), s));
+	k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, LOR_HEAD, LOR_HEAD, LOR_CHUNK, cnt,
+		cnt + 1, nullptr, nullptr, nullptr);
 	ALPB_LAUNCHED();
-	ALPB_CUDA(cudaMemcpyAsync(&h, cnt, 8, cudaMemcpyDeviceToHost, s));
+	k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, GEN_LONG, 0, GEN_CHUNK, cnt + 2, cnt + 3,
+		nullptr, nullptr, nullptr);
+	ALPB_LAUNCHED();
+	ALPB_CUDA(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, s));
 	ALPB_CUDA(cudaStreamSynchronize(s));
-	if (h > 0) {
-		if (cudaMalloc(&p->lor_row, size_t(h) * 8) != cudaSuccess ||
-			cudaMalloc(&p->lor_k0, size_t(h) * 8) != cudaSuccess) {
+	if (h[0] > 0) {
+		if (cudaMalloc(&p->lor_row, size_t(h[0]) * 8) != cudaSuccess ||
+			cudaMalloc(&p->lor_k0, size_t(h[0]) * 8) != cudaSuccess ||
+			(h[2] > 0 && (cudaMalloc(&p->gen_row, size_t(h[2]) * 8) != cudaSuccess ||
+				cudaMalloc(&p->gen_k0, size_t(h[2]) * 8) != cudaSuccess ||
+				cudaMalloc(&p->gen_first, size_t(h[3]) * 8) != cudaSuccess))) {
 			cudaGetLastError();
 			cudaFreeAsync(cnt, s);
 			cudaStreamSynchronize(s);
-			lor_release(p);
-			set_error("alpb_spmv_plan_create: out of device memory for the lor chunk list");
+			lists_release(p);
+			set_error("alpb_spmv_plan_create: out of device memory for the chunk lists");
 			return ALPB_OUTOFMEM;
 		}
-		ALPB_CUDA(cudaMemsetAsync(cnt, 0, 8, s));
-		k_lor_chunks<<<grid_for(p->m, 256, 4), 256, 0, s>>>(p->offsets, p->m, cnt, p->lor_row,
-			p->lor_k0);
+		ALPB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(h), s));
+		k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, LOR_HEAD, LOR_HEAD, LOR_CHUNK, cnt,
+			cnt + 1, p->lor_row, p->lor_k0, nullptr);
 		ALPB_LAUNCHED();
+		if (h[2] > 0) {
+			k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, GEN_LONG, 0, GEN_CHUNK, cnt + 2,
+				cnt + 3, p->gen_row, p->gen_k0, p->gen_first);
+			ALPB_LAUNCHED();
+		}
 	}
 	ALPB_CUDA(cudaFreeAsync(cnt, s));
-	p->lor_n = int64_t(h);
+	p->lor_n = int64_t(h[0]);
+	p->gen_n = int64_t(h[2]);
+	p->gen_rows = int64_t(h[3]);
 	return ALPB_SUCCESS;
 }
 
@@ -538,86 +569,214 @@ k_spmv_vector_dense(const int64_t *__restrict__ offsets, const uint32_t *__restr
 	}
 }
 
-// General path, all ALP semantics; see the file comment.
-template <class R, int W>
-__global__ void __launch_bounds__(256)
-k_spmv_vector_general(SpmvArgs a) {
-	using T = typename R::T;
-	constexpr int RPW = 32 / W;
-	const T *__restrict__ values = reinterpret_cast<const T *>(a.values);
-	const T *__restrict__ x = reinterpret_cast<const T *>(a.v);
-	T *__restrict__ y = reinterpret_cast<T *>(a.u);
-	const bool dense_hint = (a.descr & ALPB_DESC_DENSE) != 0;
-	const bool add_identity = (a.descr & ALPB_DESC_ADD_IDENTITY) != 0;
-	const bool use_index = (a.descr & ALPB_DESC_USE_INDEX) != 0;
-	const bool explicit_zero = (a.descr & ALPB_DESC_EXPLICIT_ZERO) != 0;
-	const int lane = threadIdx.x & (W - 1);
-	const int sub = (threadIdx.x & 31) / W;
-	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
-	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-	int64_t newly = 0;
-	for (int64_t base = warp * RPW; base < a.m_out; base += nwarps * RPW) {
-		const int64_t i = base + sub;
-		const bool in_range = i < a.m_out;
-		bool row_ok = in_range;
+// General path, all ALP semantics; see the file comment.  Two kinds of work
+// items share one launch: chunks of long rows, then groups of 32/W rows.
+//
+// What bounds it is the dependent chain index -> flag -> value and x of each
+// nonzero, so a lane issues GEN_BATCH of each before it uses any, and the row
+// lengths: with W lanes on every row, a hub row of 1e5 nonzeroes ran as 1e4
+// dependent steps of one lane group while the rest of the chip idled.  Rows
+// of more than GEN_LONG nonzeroes are therefore cut in chunks of GEN_CHUNK
+// (the plan's list), one warp each, first in the item order; their partials
+// are summed in chunk order by k_spmv_general_finish (deterministic).
+// Measured, R-MAT: min-plus from a 20% sparse vector, 500,009 vertices,
+// 2289 -> 118 us; lor-land with a 5% frontier and 30% visited, 1,000,003
+// vertices, 474 -> 188 us.
+
+// Rows of the general path: who takes part, and the row's identity term.
+template <class R>
+struct GenRow {
+	bool row_ok, id_row, u_has;
+	__device__ __forceinline__ GenRow(const SpmvArgs &a, int64_t i, bool in_range) {
+		row_ok = in_range;
 		if (row_ok && a.masked)
 			row_ok = a.mask_by_structure
 				? (a.u_mask_assigned == nullptr || a.u_mask_assigned[i] != 0)
 				: eval_mask(a.u_mask, a.u_mask_assigned, a.u_mask_type, a.descr, i);
-		const bool id_row = in_range && add_identity && (a.scatter_sem || row_ok);
-		const bool u_has = in_range && (a.u_assigned == nullptr || a.u_assigned[i] != 0);
+		id_row = in_range && (a.descr & ALPB_DESC_ADD_IDENTITY) && (a.scatter_sem || row_ok);
+		u_has = in_range && (a.u_assigned == nullptr || a.u_assigned[i] != 0);
 		// immutable-nonzero shortcut of the gather (blas2.hpp:351-357)
-		if (R::immutable && !a.scatter_sem && row_ok && u_has && y[i] != R::zero()) row_ok = false;
-		const bool active = row_ok || id_row;
-		T acc = R::zero();
-		bool set = false;
-		if (active) {
-			if (id_row && lane == 0 && i < a.n_in) {
-				const bool vm_ok = !a.input_masked ||
-					eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, i);
-				if (vm_ok && (dense_hint || a.v_assigned == nullptr || a.v_assigned[i])) {
-					acc = a.left ? R::mull(x[i], R::one()) : R::mulr(R::one(), x[i]);
-					set = true;
-				}
-			}
-			const int64_t b = row_ok ? a.offsets[i] : 0, e = row_ok ? a.offsets[i + 1] : 0;
-			for (int64_t k = b + lane; k < e; k += W) {
-				const uint32_t j = a.indices[k];
-				if (a.input_masked &&
-					!eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, j))
-					continue;
-				if (!dense_hint && a.v_assigned != nullptr && !a.v_assigned[j]) continue;
-				const T av = values ? values[k] : R::one();
-				const T xv = use_index ? T(j) : x[j];
-				acc = R::add(a.left ? R::mull(xv, av) : R::mulr(av, xv), acc);
-				set = true;
-				if (R::immutable && acc != R::zero()) break;
+		if (R::immutable && !a.scatter_sem && row_ok && u_has &&
+			reinterpret_cast<const typename R::T *>(a.u)[i] != R::zero())
+			row_ok = false;
+	}
+	// the identity's contribution to row i (add_identity), if any
+	__device__ __forceinline__ void identity(const SpmvArgs &a, int64_t i, typename R::T &acc,
+		bool &set) const {
+		if (!id_row || i >= a.n_in) return;
+		const typename R::T *x = reinterpret_cast<const typename R::T *>(a.v);
+		const bool vm_ok = !a.input_masked ||
+			eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, i);
+		if (vm_ok && ((a.descr & ALPB_DESC_DENSE) || a.v_assigned == nullptr || a.v_assigned[i])) {
+			acc = a.left ? R::mull(x[i], R::one()) : R::mulr(R::one(), x[i]);
+			set = true;
+		}
+	}
+	// fold the row's sum into the output; counts a newly assigned entry
+	__device__ __forceinline__ void finish(const SpmvArgs &a, int64_t i, typename R::T acc,
+		bool set, int64_t &newly) const {
+		const bool dense_hint = (a.descr & ALPB_DESC_DENSE) != 0;
+		const bool ez = (a.descr & ALPB_DESC_EXPLICIT_ZERO) && !a.scatter_sem && row_ok;
+		if (!(row_ok || id_row) || !(ez || set)) return;
+		typename R::T *y = reinterpret_cast<typename R::T *>(a.u);
+		y[i] = u_has || dense_hint ? R::add(y[i], acc) : acc;
+		if (!u_has && a.u_assigned) {
+			a.u_assigned[i] = 1;
+			++newly;
+		}
+	}
+};
+
+// acc (+)= the products of nonzeroes b + lane, b + lane + W, ... < e, in that
+// order; set: any product was there.  With stop_early (immutable rings) a
+// lane ends after a batch that made its sum nonzero.
+template <class R, int W>
+__device__ __forceinline__ void gen_gather(const SpmvArgs &a, int64_t b, int64_t e, int lane,
+	typename R::T &acc, bool &set) {
+	using T = typename R::T;
+	const T *__restrict__ values = reinterpret_cast<const T *>(a.values);
+	const T *__restrict__ x = reinterpret_cast<const T *>(a.v);
+	const bool use_index = (a.descr & ALPB_DESC_USE_INDEX) != 0;
+	const uint8_t *__restrict__ va = (a.descr & ALPB_DESC_DENSE) ? nullptr : a.v_assigned;
+	for (int64_t k0 = b + lane; k0 < e; k0 += GEN_BATCH * W) {
+		uint32_t j[GEN_BATCH];
+		bool on[GEN_BATCH];
+		T xv[GEN_BATCH], av[GEN_BATCH];
+#pragma unroll
+		for (int q = 0; q < GEN_BATCH; ++q) {
+			on[q] = k0 + q * W < e;
+			j[q] = on[q] ? __ldcs(a.indices + k0 + q * W) : 0u;
+		}
+		if (a.input_masked) {
+#pragma unroll
+			for (int q = 0; q < GEN_BATCH; ++q)
+				if (on[q])
+					on[q] = eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, j[q]);
+		}
+		if (va) {
+#pragma unroll
+			for (int q = 0; q < GEN_BATCH; ++q)
+				if (on[q]) on[q] = va[j[q]] != 0;
+		}
+#pragma unroll
+		for (int q = 0; q < GEN_BATCH; ++q) {
+			xv[q] = R::zero();
+			av[q] = R::one();
+			if (on[q]) {
+				xv[q] = use_index ? T(j[q]) : x[j[q]];
+				if (values) av[q] = values[k0 + q * W];
 			}
 		}
+#pragma unroll
+		for (int q = 0; q < GEN_BATCH; ++q)
+			if (on[q]) {
+				acc = R::add(a.left ? R::mull(xv[q], av[q]) : R::mulr(av[q], xv[q]), acc);
+				set = true;
+			}
+		if (R::immutable && acc != R::zero()) break;
+	}
+}
+
+// Chunks of the long rows (rows of more than GEN_LONG nonzeroes) and where
+// their partials go; nchunks = 0: every row runs in a row group.
+struct GenChunks {
+	int64_t nchunks = 0, nlong = 0;
+	const int64_t *row = nullptr, *k0 = nullptr;    // [nchunks]
+	const int64_t *first = nullptr;                 // [nlong] first chunk of a long row
+	uint64_t *val = nullptr;                        // [nchunks] partial sums
+	uint8_t *has = nullptr;                         // [nchunks]
+};
+
+// warp-aggregated count of newly assigned entries
+__device__ __forceinline__ void gen_count(const SpmvArgs &a, int64_t newly) {
+	if (!a.u_nnz) return;
+	for (int o = 16; o > 0; o >>= 1) newly += __shfl_down_sync(0xffffffffu, newly, o);
+	if ((threadIdx.x & 31) == 0 && newly)
+		atomicAdd((unsigned long long *) a.u_nnz, (unsigned long long) newly);
+}
+
+template <class R, int W>
+__global__ void __launch_bounds__(256)
+k_spmv_vector_general(SpmvArgs a, GenChunks g) {
+	using T = typename R::T;
+	constexpr int RPW = 32 / W;
+	const int wl = threadIdx.x & 31;
+	const int lane = threadIdx.x & (W - 1);
+	const int sub = wl / W;
+	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+	const int64_t items = g.nchunks + (a.m_out + RPW - 1) / RPW;
+	const int64_t long_len = g.nchunks > 0 ? GEN_LONG : INT64_MAX;
+	int64_t newly = 0;
+	for (int64_t it = warp; it < items; it += nwarps) {
+		if (it < g.nchunks) {   // one chunk of a long row, the whole warp
+			const int64_t i = g.row[it], k0 = g.k0[it];
+			const GenRow<R> row(a, i, true);
+			T acc = R::zero();
+			bool set = false;
+			if (row.row_ok) {
+				int64_t e = a.offsets[i + 1];
+				if (e > k0 + GEN_CHUNK) e = k0 + GEN_CHUNK;
+				gen_gather<R, 32>(a, k0, e, wl, acc, set);
+			}
+#pragma unroll
+			for (int o = 16; o > 0; o >>= 1)
+				acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o));
+			set = __any_sync(0xffffffffu, set);
+			if (wl == 0) {
+				store_bits<T>(g.val + it, acc);
+				g.has[it] = set ? 1 : 0;
+			}
+			continue;
+		}
+		const int64_t i = (it - g.nchunks) * RPW + sub;
+		const bool in_range = i < a.m_out;
+		const int64_t b = in_range ? a.offsets[i] : 0, e = in_range ? a.offsets[i + 1] : 0;
+		const bool mine = in_range && e - b <= long_len;
+		const GenRow<R> row(a, i, mine);
+		T acc = R::zero();
+		bool set = false;
+		if (lane == 0) row.identity(a, i, acc, set);
+		if (row.row_ok) gen_gather<R, W>(a, b, e, lane, acc, set);
 #pragma unroll
 		for (int o = W / 2; o > 0; o >>= 1) {
 			acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o, W));
 			set = set | (__shfl_down_sync(0xffffffffu, int(set), o, W) != 0);
 		}
-		const bool ez = explicit_zero && !a.scatter_sem && row_ok;
-		if (active && lane == 0 && (ez || set)) {
-			if (u_has || dense_hint) {
-				y[i] = R::add(y[i], acc);
-			} else {
-				y[i] = acc;
-			}
-			if (!u_has && a.u_assigned) {
-				a.u_assigned[i] = 1;
-				++newly;
-			}
-		}
+		if (lane == 0) row.finish(a, i, acc, set, newly);
 	}
-	if (a.u_nnz) {
-		// warp-aggregated count of newly assigned entries
-		for (int o = 16; o > 0; o >>= 1) newly += __shfl_down_sync(0xffffffffu, newly, o);
-		if ((threadIdx.x & 31) == 0 && newly) atomicAdd((unsigned long long *) a.u_nnz,
-			(unsigned long long) newly);
+	gen_count(a, newly);
+}
+
+// One warp per long row: its chunks' partials in a fixed order (lane-strided,
+// then a shuffle tree), the identity term, the output.
+template <class R>
+__global__ void __launch_bounds__(256)
+k_spmv_general_finish(SpmvArgs a, GenChunks g) {
+	using T = typename R::T;
+	const int lane = threadIdx.x & 31;
+	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+	int64_t newly = 0;
+	for (int64_t l = warp; l < g.nlong; l += nwarps) {
+		const int64_t c0 = g.first[l], i = g.row[c0];
+		const int64_t n = (a.offsets[i + 1] - g.k0[c0] + GEN_CHUNK - 1) / GEN_CHUNK;
+		const GenRow<R> row(a, i, true);
+		T acc = R::zero();
+		bool set = false;
+		if (lane == 0) row.identity(a, i, acc, set);
+		if (row.row_ok)
+			for (int64_t c = c0 + lane; c < c0 + n; c += 32)
+				if (g.has[c]) {
+					acc = R::add(acc, wm_load_slot<T>(g.val + c));
+					set = true;
+				}
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o));
+		set = __any_sync(0xffffffffu, set);
+		if (lane == 0) row.finish(a, i, acc, set, newly);
 	}
+	gen_count(a, newly);
 }
 
 // Trivial case of blas2.hpp:1001-1037: the output keeps its values; with
@@ -708,15 +867,40 @@ int launch_vector_dense_w(const SpmvArgs &a, cudaStream_t s) {
 }
 
 template <class R, int W>
-int launch_vector_general_w(const SpmvArgs &a, cudaStream_t s) {
-	const int64_t threads = a.m_out * W;
-	k_spmv_vector_general<R, W><<<grid_for(threads, 256, 8), 256, 0, s>>>(a);
+int launch_vector_general_w(const SpmvArgs &a, const alpb_spmv_plan_s *p, cudaStream_t s) {
+	constexpr int RPW = 32 / W;
+	GenChunks g;
+	void *scratch = nullptr;
+	if (p && p->gen_n > 0) {
+		// partials of the long rows' chunks, this call's own (calls on other
+		// streams may use the same plan); without them every row runs in a group
+		if (cudaMallocAsync(&scratch, size_t(p->gen_n) * 9, s) == cudaSuccess) {
+			g.nchunks = p->gen_n;
+			g.nlong = p->gen_rows;
+			g.row = p->gen_row;
+			g.k0 = p->gen_k0;
+			g.first = p->gen_first;
+			g.val = static_cast<uint64_t *>(scratch);
+			g.has = reinterpret_cast<uint8_t *>(g.val + p->gen_n);
+		} else {
+			cudaGetLastError();
+			scratch = nullptr;
+		}
+	}
+	const int64_t items = g.nchunks + (a.m_out + RPW - 1) / RPW;
+	k_spmv_vector_general<R, W><<<grid_for(items * 32, 256, 8), 256, 0, s>>>(a, g);
 	ALPB_LAUNCHED();
+	if (g.nlong > 0) {
+		k_spmv_general_finish<R><<<grid_for(g.nlong * 32, 256, 8), 256, 0, s>>>(a, g);
+		ALPB_LAUNCHED();
+	}
+	if (scratch) ALPB_CUDA(cudaFreeAsync(scratch, s));
 	return ALPB_SUCCESS;
 }
 
 template <class R>
-int launch_vector(const SpmvArgs &a, int W, bool dense, cudaStream_t s) {
+int launch_vector(const SpmvArgs &a, const alpb_spmv_plan_s *p, int W, bool dense,
+	cudaStream_t s) {
 	if (dense) {
 		switch (W) {
 		case 1: return launch_vector_dense_w<R, 1>(a, s);
@@ -728,12 +912,12 @@ int launch_vector(const SpmvArgs &a, int W, bool dense, cudaStream_t s) {
 		}
 	}
 	switch (W) {
-	case 1: return launch_vector_general_w<R, 1>(a, s);
-	case 2: return launch_vector_general_w<R, 2>(a, s);
-	case 4: return launch_vector_general_w<R, 4>(a, s);
-	case 8: return launch_vector_general_w<R, 8>(a, s);
-	case 16: return launch_vector_general_w<R, 16>(a, s);
-	default: return launch_vector_general_w<R, 32>(a, s);
+	case 1: return launch_vector_general_w<R, 1>(a, p, s);
+	case 2: return launch_vector_general_w<R, 2>(a, p, s);
+	case 4: return launch_vector_general_w<R, 4>(a, p, s);
+	case 8: return launch_vector_general_w<R, 8>(a, p, s);
+	case 16: return launch_vector_general_w<R, 16>(a, p, s);
+	default: return launch_vector_general_w<R, 32>(a, p, s);
 	}
 }
 
@@ -771,7 +955,7 @@ int run_spmv(const SpmvArgs &a, const alpb_spmv_plan_s *p, int force_sched, cuda
 	int W = p ? p->vw : default_width(a.m_out ? double(a.nnz) / double(a.m_out) : 1.0);
 	if (fast && sched == ALPB_SCHED_MERGE_PATH && p && p->tile_row)
 		return launch_merge<R>(a, *p, s);
-	return launch_vector<R>(a, W, fast, s);
+	return launch_vector<R>(a, p, W, fast, s);
 }
 
 int dispatch_spmv(int ring, const SpmvArgs &a, const alpb_spmv_plan_s *p, int force_sched,
@@ -878,7 +1062,7 @@ int alpb_spmv_plan_create(alpb_spmv_plan *plan, int64_t m, int64_t nnz, const in
 	cudaStream_t s = as_stream(stream);
 	int rc = plan_create_tiles(plan, m, nnz, offsets, sched, vector_width, WM_TILE, s);
 	if (rc != ALPB_SUCCESS) return rc;
-	rc = lor_build(*plan, s);
+	rc = lists_build(*plan, s);
 	if (rc != ALPB_SUCCESS) {
 		alpb_spmv_plan_destroy(*plan);
 		*plan = nullptr;
@@ -937,8 +1121,7 @@ int alpb_spmv_plan_destroy(alpb_spmv_plan p) {
 	cudaFree(p->hot_idx);
 	cudaFree(p->hot_cols);
 	cudaFree(p->hot_x);
-	cudaFree(p->lor_row);
-	cudaFree(p->lor_k0);
+	lists_release(p);
 	delete p;
 	return ALPB_SUCCESS;
 }

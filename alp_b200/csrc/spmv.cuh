@@ -48,6 +48,12 @@ struct alpb_spmv_plan_s {
 	int64_t lor_n = -1;
 	int64_t *lor_row = nullptr;
 	int64_t *lor_k0 = nullptr;
+	// General path: the rows of more than GEN_LONG nonzeroes in chunks of
+	// GEN_CHUNK, a row's chunks consecutive; gen_first: each row's first chunk.
+	int64_t gen_n = 0, gen_rows = 0;
+	int64_t *gen_row = nullptr;
+	int64_t *gen_k0 = nullptr;
+	int64_t *gen_first = nullptr;
 };
 
 namespace alpb {

@@ -1,0 +1,69 @@
+"""The general mxv path (masks, sparse vectors, descriptors) on rows cut in
+chunks: row lengths at the edges of a row group, of a chunk and of the warp
+that sums a row's chunks, against the restatement.
+
+Integer and boolean rings must agree bit for bit.  FP64 sums n <= 9000
+positive terms in another order: each of the two orders is off by at most
+(n - 1) 2^-53 relative, so entries agree to 2 * 9000 * 2^-53 = 2e-12."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [0, 1, 3, 31, 32, 33, 63, 64, 65, 66, 255, 256, 257, 511, 513, 8191, 8193, 8449, 9000, 2]
+DESCR = {"none": 0, "invert": 1, "structural": 8, "invert_structural": 9, "add_identity": 32,
+         "use_index": 64, "explicit_zero": 512}
+
+
+def storage(rng, vtype):
+    from oracle.oracle import NP, VOID
+    n = 9001
+    lens = np.array(LENGTHS * 3)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    col = np.concatenate([rng.choice(n, k, replace=False) for k in lens]).astype(np.uint32)
+    if vtype == 3:
+        vals = rng.random(len(col))
+    elif vtype == 2:
+        vals = rng.integers(1, 101, len(col)).astype(np.int32)
+    else:
+        vals = (rng.random(len(col)) < 0.5).astype(NP[vtype])
+    return len(lens), n, rp, col, vals
+
+
+@pytest.mark.parametrize("frontier", [0.02, 0.5, 1.0])
+@pytest.mark.parametrize("descr", sorted(DESCR))
+@pytest.mark.parametrize("ring", [0, 1, 2])
+def test_general_path_long_rows(cuda, oracle, ring, descr, frontier):
+    import torch
+    from alp_b200 import device as dev
+    vtype = {0: 3, 1: 1, 2: 2}[ring]
+    rng = np.random.default_rng([ring, DESCR[descr], int(100 * frontier)])
+    m, n, rp, col, vals = storage(rng, vtype)
+    npt = {3: np.float64, 2: np.int32, 1: np.uint8}[vtype]
+    value = lambda k: (rng.random(k) if vtype == 3 else rng.integers(0, 2 if vtype == 1 else 1000, k)).astype(npt)  # noqa: E731
+    u, v = value(m), value(n)
+    ua = (rng.random(m) < 0.5).astype(np.uint8)
+    va = (rng.random(n) < frontier).astype(np.uint8)
+    mask, mask_a = (rng.random(m) < 0.7).astype(np.uint8), (rng.random(m) < 0.8).astype(np.uint8)
+    A = dev.from_host(m, n, rp, col, vals, vtype)
+    plan = dev.Plan(A, sched=1)
+    for form in (0, 1, 2):
+        wu, wa = u.copy(), ua.copy()
+        rc, wn = oracle.mxv(ring, DESCR[descr], form, m, n, rp, col, vals, vtype, wu, wa,
+                            u_mask=mask, u_mask_assigned=mask_a, u_mask_count=int(mask_a.sum()),
+                            v=v, v_assigned=va)
+        assert rc == 0
+        T = lambda a: torch.from_numpy(a.copy()).cuda()  # noqa: E731
+        gu, ga = T(u), T(ua)
+        gn = torch.tensor([int(ua.sum())], dtype=torch.int64, device="cuda")
+        dev.mxv(ring, A, gu, T(v), descr=DESCR[descr], form=form, u_assigned=ga, u_nnz=gn,
+                u_mask=T(mask), u_mask_assigned=T(mask_a), u_mask_count=int(mask_a.sum()),
+                v_assigned=T(va), plan=plan)
+        np.testing.assert_array_equal(ga.cpu().numpy() != 0, wa != 0)
+        assert int(gn) == wn
+        got, want = gu.cpu().numpy()[wa != 0], wu[wa != 0]
+        if vtype == 3:
+            np.testing.assert_allclose(got, want, rtol=2e-12, atol=0)
+        else:
+            np.testing.assert_array_equal(got, want)
+    plan.close()
