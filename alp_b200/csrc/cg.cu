@@ -40,6 +40,12 @@ struct CgState {
 	int converged;
 };
 
+} // namespace alpb
+
+#include "cg_rows.cuh"
+
+namespace alpb {
+
 struct CgArgs {
 	MergeTables mt;
 	const int64_t *offsets;
@@ -232,6 +238,134 @@ __global__ void __launch_bounds__(32 * CG_WARPS, 24 / CG_WARPS) k_cg(CgArgs a) {
 	}
 }
 
+// Launch shape of k_cg_rows for n rows of at most maxlen nonzeroes.
+struct CgRowsShape {
+	int L = 1, nb = 0, grid = 0, steps = 0, items = 0, resident = 0, vec_smem = 0;
+	size_t smem = 0;
+};
+
+// One lane per row gathers best (32 consecutive rows on one line after another:
+// 64^3 17 us an iteration, 20 with two lanes a row, 27 with four); more lanes
+// only while every other warp would have no item (32^3: four lanes a row).
+// Vectors go to shared memory while they leave room for the matrix.
+static CgRowsShape cg_rows_shape(int64_t n, int maxlen) {
+	CgRowsShape c;
+	const size_t cap = CGR_SMEM;
+	const int64_t sms = sm_count() < 256 ? sm_count() : 256;   // partials of GridReduce
+	const int64_t per = (n + sms - 1) / sms;
+	if (per > (1 << 24) || maxlen < 1) return c;
+	while (c.L < 8 && c.L * 2 <= maxlen && (per * c.L + 31) / 32 * 2 <= CGR_WARPS) c.L *= 2;
+	const int H = 32 / c.L;
+	c.nb = int((per + H - 1) / H * H);
+	c.grid = int((n + c.nb - 1) / c.nb);
+	c.steps = (maxlen + c.L - 1) / c.L;
+	c.items = c.nb / H;
+	const size_t vec = size_t(c.nb) * 32;
+	c.vec_smem = vec <= cap * 5 / 8;
+	const size_t item = size_t(c.steps) * 32 * 12;
+	const size_t left = cap - (c.vec_smem ? vec : 0);
+	c.resident = int(left / item < size_t(c.items) ? left / item : size_t(c.items));
+	c.smem = (c.vec_smem ? vec : 0) + size_t(c.resident) * item;
+	return c;
+}
+
+// The solve on k_cg_rows; ALPB_UNSUPPORTED (nothing launched) when its
+// workspace cannot be had, and the caller runs k_cg instead.
+template <int L>
+static int cg_rows_solve(const CgRowsShape &c, CgRowsArgs a, double *wk, cudaStream_t s,
+	CgState *h) {
+	static std::atomic<bool> ready[64];
+	int dev = 0;
+	ALPB_CUDA(cudaGetDevice(&dev));
+	if (dev >= 64 || !ready[dev].load()) {
+		ALPB_CUDA(cudaFuncSetAttribute(k_cg_rows<L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			CGR_SMEM));
+		if (dev < 64) ready[dev].store(true);
+	}
+	const int64_t n = a.n;
+	const size_t ell = size_t(c.grid) * size_t(c.items - c.resident) * size_t(c.steps) * 32;
+	// one allocation: state, partials, the items outside shared memory, r
+	const size_t head = (sizeof(GridReduce) + sizeof(CgState) + 255) / 256 * 256;
+	const size_t bytes = head + ell * 12 + (c.vec_smem ? 0 : size_t(n) * 8);
+	unsigned char *ws = nullptr;
+	if (cudaMallocAsync(&ws, bytes, s) != cudaSuccess) {
+		cudaGetLastError();
+		return ALPB_UNSUPPORTED;
+	}
+	a.gr = reinterpret_cast<GridReduce *>(ws);
+	a.st = reinterpret_cast<CgState *>(ws + sizeof(GridReduce));
+	a.ell_val = reinterpret_cast<double *>(ws + head);
+	a.g_r = a.ell_val + ell;
+	a.ell_idx = reinterpret_cast<uint32_t *>(a.g_r + (c.vec_smem ? 0 : n));
+	a.pr = reinterpret_cast<double2 *>(wk);
+	a.g_u = wk + 2 * n;
+	a.g_t = wk + 3 * n;
+	a.r_out = wk;
+	a.nb = c.nb;
+	a.steps = c.steps;
+	a.items = c.items;
+	a.resident = c.resident;
+	a.vec_smem = c.vec_smem;
+	ALPB_CUDA(cudaMemsetAsync(ws, 0, head, s));
+	void *args[] = {&a};
+	ALPB_CUDA(cudaLaunchCooperativeKernel((void *) k_cg_rows<L>, dim3(c.grid), dim3(CGR_THREADS),
+		args, c.smem, s));
+	ALPB_LAUNCHED();
+	ALPB_CUDA(cudaMemcpyAsync(h, a.st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
+	ALPB_CUDA(cudaFreeAsync(ws, s));
+	return ALPB_SUCCESS;
+}
+
+// The solve on warp merge tiles (k_cg): any row lengths.  *h is filled once
+// the stream has run.
+static int cg_tiles_solve(int64_t n, const int64_t *row_ptr, const uint32_t *col_idx,
+	const double *values, const double *b, double *x, int64_t max_iter, double tol, double *wk,
+	alpb_spmv_plan plan, cudaStream_t s, CgState *h) {
+	const bool few = plan->ntiles <= CG_FEW_TILES;
+	const int warps = few ? 16 : 8;
+	const size_t smem = sizeof(CgWarpSmem) * warps;
+	static bool smem_set = false;
+	if (!smem_set) {
+		ALPB_CUDA(cudaFuncSetAttribute(k_cg<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			int(sizeof(CgWarpSmem) * 16)));
+		ALPB_CUDA(cudaFuncSetAttribute(k_cg<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			int(sizeof(CgWarpSmem) * 8)));
+		smem_set = true;
+	}
+	const int grid = few ? solver_grid(k_cg<16>, 32 * 16, plan->ntiles, 16, smem)
+						 : solver_grid(k_cg<8>, 32 * 8, plan->ntiles, 8, smem);
+	ALPB_CHECK(grid > 0, ALPB_PANIC, "alpb_cg_solve: no cooperative occupancy");
+	double *scratch = nullptr;
+	CgState *st = nullptr;
+	ALPB_CUDA(cudaMallocAsync(&scratch, size_t(4 * grid) * 8, s));
+	ALPB_CUDA(cudaMallocAsync(&st, sizeof(CgState), s));
+	ALPB_CUDA(cudaMemsetAsync(st, 0, sizeof(CgState), s));
+	CgArgs a;
+	a.mt = merge_tables(*plan);
+	a.offsets = row_ptr;
+	a.indices = col_idx;
+	a.values = values;
+	a.b = b;
+	a.x = x;
+	a.pr = reinterpret_cast<double2 *>(wk);
+	a.u_new = wk + 2 * n;
+	a.temp = wk + 3 * n;
+	a.r_out = wk;
+	a.blk = scratch;
+	a.n = n;
+	a.max_iter = max_iter;
+	a.tol = tol;
+	a.st = st;
+	void *args[] = {&a};
+	ALPB_CUDA(cudaLaunchCooperativeKernel(few ? (void *) k_cg<16> : (void *) k_cg<8>, dim3(grid),
+		dim3(32 * warps), args, smem, s));
+	ALPB_LAUNCHED();
+	ALPB_CUDA(cudaMemcpyAsync(h, st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
+	ALPB_CUDA(cudaFreeAsync(scratch, s));
+	ALPB_CUDA(cudaFreeAsync(st, s));
+	return ALPB_SUCCESS;
+}
+
 } // namespace alpb
 
 using namespace alpb;
@@ -259,58 +393,44 @@ extern "C" int alpb_cg_solve(int64_t n, const int64_t *row_ptr, const uint32_t *
 		if (rc != ALPB_SUCCESS) return rc;
 		plan = own_plan;
 	}
-	const bool few = plan->ntiles <= CG_FEW_TILES;
-	const int warps = few ? 16 : 8;
-	const size_t smem = sizeof(CgWarpSmem) * warps;
-	static bool smem_set = false;
-	if (!smem_set) {
-		ALPB_CUDA(cudaFuncSetAttribute(k_cg<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			int(sizeof(CgWarpSmem) * 16)));
-		ALPB_CUDA(cudaFuncSetAttribute(k_cg<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			int(sizeof(CgWarpSmem) * 8)));
-		smem_set = true;
-	}
-	const int grid = few ? solver_grid(k_cg<16>, 32 * 16, plan->ntiles, 16, smem)
-						 : solver_grid(k_cg<8>, 32 * 8, plan->ntiles, 8, smem);
-	ALPB_CHECK(grid > 0, ALPB_PANIC, "alpb_cg_solve: no cooperative occupancy");
 	// the (r, u) pairs take 16-byte loads: a work space that is not 16-byte
 	// aligned is replaced by an internal one
 	double *wk = (reinterpret_cast<uintptr_t>(work) & 15) ? nullptr : work;
-	double *own_work = nullptr, *scratch = nullptr;
-	CgState *st = nullptr;
+	double *own_work = nullptr;
 	if (!wk) {
 		ALPB_CUDA(cudaMallocAsync(&own_work, size_t(4 * n) * 8, s));
 		wk = own_work;
 	}
-	ALPB_CUDA(cudaMallocAsync(&scratch, size_t(4 * grid) * 8, s));
-	ALPB_CUDA(cudaMallocAsync(&st, sizeof(CgState), s));
-	ALPB_CUDA(cudaMemsetAsync(st, 0, sizeof(CgState), s));
-	CgArgs a;
-	a.mt = merge_tables(*plan);
-	a.offsets = row_ptr;
-	a.indices = col_idx;
-	a.values = values;
-	a.b = b;
-	a.x = x;
-	a.pr = reinterpret_cast<double2 *>(wk);
-	a.u_new = wk + 2 * n;
-	a.temp = wk + 3 * n;
-	a.r_out = wk;
-	a.blk = scratch;
-	a.n = n;
-	a.max_iter = max_iter;
-	a.tol = tol;
-	a.st = st;
-	void *args[] = {&a};
-	ALPB_CUDA(cudaLaunchCooperativeKernel(few ? (void *) k_cg<16> : (void *) k_cg<8>, dim3(grid),
-		dim3(32 * warps), args, smem, s));
-	ALPB_LAUNCHED();
 	CgState h;
-	ALPB_CUDA(cudaMemcpyAsync(&h, st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
-	ALPB_CUDA(cudaFreeAsync(scratch, s));
-	ALPB_CUDA(cudaFreeAsync(st, s));
+	int rc = ALPB_UNSUPPORTED;
+	// short regular rows (the plan's tiles hold whole rows): fixed rows per
+	// block.  Measured us per iteration, k_cg -> k_cg_rows, 27-point grids:
+	// 10^3 11.6 -> 7.7, 32^3 13.9 -> 7.6, 48^3 26 -> 11, 64^3 47 -> 17,
+	// 80^3 78 -> 50, 128^3 311 -> 199
+	const CgRowsShape c = plan->tile_d ? cg_rows_shape(n, int(plan->maxlen)) : CgRowsShape{};
+	if (c.grid > 0 && n < int64_t(CGR_NONE)) {
+		CgRowsArgs a{};
+		a.offsets = row_ptr;
+		a.indices = col_idx;
+		a.values = values;
+		a.b = b;
+		a.x = x;
+		a.n = n;
+		a.max_iter = max_iter;
+		a.tol = tol;
+		rc = c.L == 1 ? cg_rows_solve<1>(c, a, wk, s, &h)
+			: c.L == 2 ? cg_rows_solve<2>(c, a, wk, s, &h)
+			: c.L == 4 ? cg_rows_solve<4>(c, a, wk, s, &h)
+					   : cg_rows_solve<8>(c, a, wk, s, &h);
+	}
+	if (rc == ALPB_UNSUPPORTED)
+		rc = cg_tiles_solve(n, row_ptr, col_idx, values, b, x, max_iter, tol, wk, plan, s, &h);
 	if (own_work) ALPB_CUDA(cudaFreeAsync(own_work, s));
 	ALPB_CUDA(cudaStreamSynchronize(s));
+	if (rc != ALPB_SUCCESS) {
+		alpb_spmv_plan_destroy(own_plan);
+		return rc;
+	}
 	if (own_plan) alpb_spmv_plan_destroy(own_plan);
 	ALPB_CHECK(h.gs.err == 0, ALPB_PANIC, "alpb_cg_solve: a grid barrier or tile wait timed out");
 	*iterations = h.iterations;

@@ -17,8 +17,9 @@ struct alignas(128) GridSync {
 	unsigned int pad1[30];
 };
 
-// ~1 s at the sleep granularity below: far beyond any legitimate wait of a
-// co-resident grid, short enough to keep the context usable on a fault.
+// A few seconds of polls (each an L2 round trip of about 0.2 us): far beyond any
+// legitimate wait of a co-resident grid, short enough to keep the context
+// usable on a fault.
 constexpr long long kSpinLimit = 1ll << 24;
 
 // All blocks of a cooperative launch call this the same number of times.
@@ -30,31 +31,31 @@ constexpr long long kSpinLimit = 1ll << 24;
 // then leave their loop.
 __device__ __forceinline__ bool grid_sync(GridSync *gs) {
 	__syncthreads();
+	int bad = 0;
 	if (threadIdx.x == 0) {
 		const unsigned long long G = gridDim.x;
 		unsigned long long old;
 		asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;"
 					 : "=l"(old) : "l"(&gs->count) : "memory");
 		const unsigned long long target = (old / G + 1) * G;
-		if (old + 1 != target) {
-			volatile int *verr = &gs->err;
-			long long spins = 0;
-			for (;;) {
-				unsigned long long c;
-				asm volatile("ld.acquire.gpu.global.u64 %0, [%1];"
-							 : "=l"(c) : "l"(&gs->count) : "memory");
-				if (c >= target) break;
-				if ((++spins & 63) == 0 && *verr) break;
-				if (spins > kSpinLimit) {
-					atomicExch(&gs->err, 1);
-					break;
-				}
-				__nanosleep(32);
+		volatile int *verr = &gs->err;
+		for (long long spins = 0;; ++spins) {
+			// the error flag's load is in flight with the counter's: read after
+			// the barrier it cost every thread one more L2 round trip
+			const int e = *verr;
+			unsigned long long c;
+			asm volatile("ld.acquire.gpu.global.u64 %0, [%1];"
+						 : "=l"(c) : "l"(&gs->count) : "memory");
+			bad = e;
+			if (c >= target || bad) break;
+			if (spins > kSpinLimit) {
+				atomicExch(&gs->err, 1);
+				bad = 1;
+				break;
 			}
 		}
 	}
-	__syncthreads();
-	return *((volatile int *) &gs->err) == 0;
+	return !__syncthreads_or(bad);
 }
 
 // Sum over the block in a fixed order (warp trees, then warp 0 over the warp
@@ -80,6 +81,70 @@ __device__ __forceinline__ double block_sum_array(const double *a, int64_t n, do
 	double v = 0.0;
 	for (int64_t k = threadIdx.x; k < n; k += blockDim.x) v += ((const volatile double *) a)[k];
 	return block_sum(v, smem);
+}
+
+// Grid barrier and sum in one: every block leaves its partial beside the
+// counter and the blocks read all partials once the counter is complete.
+// What bounds it is latency across the chip: about 700 cycles for the atomic
+// (300-700 by the die that holds the line), 300-400 each for a poll and for
+// the partials.  Measured with 148 blocks of 512 threads, fences included:
+// 2.0 us; value-carrying slots polled by every block took 3.8 us (the polls
+// contend with the stores), pushed to every block's own lines 2.9 us, and
+// gathered and broadcast by one block 3.1 us.
+struct alignas(128) GridReduce {
+	unsigned long long count;
+	unsigned int pad[30];
+	double part[2][256];     // [epoch parity][block]
+};
+
+// All threads call, with epoch = 1, 2, ... ; v: this thread's term; *sum: the
+// grid's total in a fixed order (lanes, warps, blocks), the same bits in every
+// thread.  Needs gridDim.x <= min(blockDim.x, 256), *g zeroed before the
+// launch.  Global writes of any block before the call are visible to plain
+// loads of all after it.  false: a wait gave up (*err is set).
+__device__ __forceinline__ bool grid_reduce(GridReduce *g, unsigned epoch, double v,
+	double *sum, double *smem /* >= 64 */, int *err) {
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	const int nwarps = blockDim.x >> 5, G = gridDim.x;
+	double *part = g->part[epoch & 1];
+	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+	if (lane == 0) smem[w] = v;
+	__syncthreads();
+	int bad = 0;
+	if (w == 0) {
+		double t = lane < nwarps ? smem[lane] : 0.0;
+		for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+		if (lane == 0) {
+			part[blockIdx.x] = t;
+			unsigned long long c;
+			asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;"
+						 : "=l"(c) : "l"(&g->count) : "memory");
+			const unsigned long long target = (unsigned long long) epoch * G;
+			for (long long spins = 0;; ++spins) {
+				asm volatile("ld.acquire.gpu.global.u64 %0, [%1];"
+							 : "=l"(c) : "l"(&g->count) : "memory");
+				if (c >= target) break;
+				if ((spins & 255) == 255 && *reinterpret_cast<volatile int *>(err)) bad = 1;
+				if (spins > kSpinLimit / 8) {
+					atomicExch(err, 1);
+					bad = 1;
+				}
+				if (bad) break;
+			}
+		}
+	}
+	if (__syncthreads_or(bad)) return false;
+	const int gw = (G + 31) >> 5;
+	if (w < gw) {
+		double t = int(threadIdx.x) < G ? __ldcg(part + threadIdx.x) : 0.0;
+		for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+		if (lane == 0) smem[32 + w] = t;
+	}
+	__syncthreads();
+	double r = 0.0;
+	for (int k = 0; k < gw; ++k) r += smem[32 + k];
+	*sum = r;
+	return true;
 }
 
 // Largest grid of `kernel` whose blocks are all co-resident.
