@@ -7,6 +7,7 @@
 // count only) forms block partials in a fixed order, and one block sums them.
 #include "common.cuh"
 #include "persist.cuh"
+#include "scalar.cuh"
 
 namespace alpb {
 
@@ -83,6 +84,45 @@ __global__ void __launch_bounds__(RB) k_dot_partial(int add_op, int mul_op, int6
 	if (threadIdx.x == 0) partials[blockIdx.x] = acc;
 }
 
+// The same to a host scalar, in one launch: a thread's entries i, i + S, ...
+// in that order, four of them loaded at a time.
+__global__ void __launch_bounds__(SCALAR_BLOCK) k_dot_scalar(int add_op, int mul_op, int64_t n,
+	const double *__restrict__ x, const uint8_t *__restrict__ xa, const double *__restrict__ y,
+	const uint8_t *__restrict__ ya, uint64_t *part, unsigned *arrived, uint64_t *out) {
+	const double ident = op_identity(add_op);
+	double acc = ident;
+	const int64_t S = int64_t(gridDim.x) * SCALAR_BLOCK;
+	for (int64_t i0 = blockIdx.x * int64_t(SCALAR_BLOCK) + threadIdx.x; i0 < n; i0 += 4 * S) {
+		double xv[4], yv[4];
+		bool on[4];
+#pragma unroll
+		for (int q = 0; q < 4; ++q) {
+			const int64_t i = i0 + q * S;
+			on[q] = i < n && !(xa && !xa[i]) && !(ya && !ya[i]);
+			xv[q] = on[q] ? x[i] : 0.0;
+			yv[q] = on[q] ? y[i] : 0.0;
+		}
+#pragma unroll
+		for (int q = 0; q < 4; ++q)
+			if (on[q]) acc = apply_op(add_op, acc, apply_op(mul_op, xv[q], yv[q]));
+	}
+	scalar_finish(acc, ident, ident, true,
+		[&](double a, double b) { return apply_op(add_op, a, b); }, part, arrived, out);
+}
+
+static int dot_scalar(double *h, int add_op, int mul_op, int64_t n, const double *x,
+	const uint8_t *xa, const double *y, const uint8_t *ya, cudaStream_t s) {
+	ScalarScratch sc;
+	const int rc = scalar_scratch(&sc, s);
+	if (rc != ALPB_SUCCESS) return rc;
+	k_dot_scalar<<<scalar_grid(n), SCALAR_BLOCK, 0, s>>>(add_op, mul_op, n, x, xa, y, ya, sc.part,
+		sc.arrived, sc.host_dev);
+	ALPB_LAUNCHED();
+	ALPB_CUDA(cudaStreamSynchronize(s));
+	*h = *reinterpret_cast<const double *>(sc.host);
+	return ALPB_SUCCESS;
+}
+
 __global__ void __launch_bounds__(RB) k_reduce_partials(int add_op, const double *__restrict__ p,
 	int np, double *__restrict__ out, int accumulate) {
 	__shared__ double sm[33];
@@ -142,11 +182,23 @@ __global__ void k_ewise_muladd(double *__restrict__ out, int add_op, int mul_op,
 		out[i] = apply_op(add_op, out[i], apply_op(mul_op, a ? a[i] : sa, b ? b[i] : sb));
 }
 
+// four entries of a thread in flight at a time (one wave of threads over 1e6
+// entries used to walk three or four of them one after the other)
 __global__ void k_foldl(double *__restrict__ x, int op, int64_t n, const double *__restrict__ y,
 	double sy) {
-	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
-		 i += int64_t(gridDim.x) * blockDim.x)
-		x[i] = apply_op(op, x[i], y ? y[i] : sy);
+	const int64_t S = int64_t(gridDim.x) * blockDim.x;
+	for (int64_t i0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i0 < n; i0 += 4 * S) {
+		double a[4], b[4];
+#pragma unroll
+		for (int q = 0; q < 4; ++q)
+			if (i0 + q * S < n) {
+				a[q] = x[i0 + q * S];
+				b[q] = y ? y[i0 + q * S] : sy;
+			}
+#pragma unroll
+		for (int q = 0; q < 4; ++q)
+			if (i0 + q * S < n) x[i0 + q * S] = apply_op(op, a[q], b[q]);
+	}
 }
 
 } // namespace alpb
@@ -162,15 +214,10 @@ int alpb_dot_f64(double *result, int add_op, int mul_op, int64_t n, const double
 		"alpb_dot_f64: operators (%d, %d) are not a monoid and an operator", add_op, mul_op);
 	ALPB_CHECK(n >= 0, ALPB_ILLEGAL, "alpb_dot_f64: negative size");
 	if (n == 0) return ALPB_SUCCESS;
-	cudaStream_t s = as_stream(stream);
-	double *d = nullptr;
-	ALPB_CUDA(cudaMallocAsync(&d, 8, s));
-	int rc = dot_device(d, add_op, mul_op, n, x, x_assigned, y, y_assigned, 0, s);
-	if (rc != ALPB_SUCCESS) return rc;
 	double h = 0;
-	ALPB_CUDA(cudaMemcpyAsync(&h, d, 8, cudaMemcpyDeviceToHost, s));
-	ALPB_CUDA(cudaFreeAsync(d, s));
-	ALPB_CUDA(cudaStreamSynchronize(s));
+	const int rc = dot_scalar(&h, add_op, mul_op, n, x, x_assigned, y, y_assigned,
+		as_stream(stream));
+	if (rc != ALPB_SUCCESS) return rc;
 	// z = z (+) dot: the reference folds the dot into the given scalar (blas1.hpp:9334-9336)
 	double z = *result;
 	switch (add_op) {
@@ -241,15 +288,10 @@ int alpb_reduce_f64(double *result, int op, int64_t n, const double *x, const ui
 	ALPB_CHECK(is_monoid(op), ALPB_UNSUPPORTED, "alpb_reduce_f64: op %d is not a monoid", op);
 	if (n == 0) return ALPB_SUCCESS;
 	// fold(x) = dot(x, 1) under (op, left_assign)
-	cudaStream_t s = as_stream(stream);
-	double *d = nullptr;
-	ALPB_CUDA(cudaMallocAsync(&d, 8, s));
-	int rc = dot_device(d, op, ALPB_OP_LEFT_ASSIGN, n, x, assigned, x, nullptr, 0, s);
-	if (rc != ALPB_SUCCESS) return rc;
 	double h = 0;
-	ALPB_CUDA(cudaMemcpyAsync(&h, d, 8, cudaMemcpyDeviceToHost, s));
-	ALPB_CUDA(cudaFreeAsync(d, s));
-	ALPB_CUDA(cudaStreamSynchronize(s));
+	const int rc = dot_scalar(&h, op, ALPB_OP_LEFT_ASSIGN, n, x, assigned, x, nullptr,
+		as_stream(stream));
+	if (rc != ALPB_SUCCESS) return rc;
 	double z = *result;
 	switch (op) {
 	case ALPB_OP_ADD: z = z + h; break;

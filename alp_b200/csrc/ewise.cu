@@ -10,6 +10,7 @@
 // cast their operands (graphblas/ops.hpp): integer operators compute exactly,
 // with two's-complement wrap-around.
 #include "common.cuh"
+#include "scalar.cuh"
 
 #include <cstring>
 #include <type_traits>
@@ -261,49 +262,45 @@ __global__ void k_count_assigned(const uint8_t *a, int64_t n, int64_t *cnt) {
 	if ((threadIdx.x & 31) == 0 && c) atomicAdd((unsigned long long *) cnt, (unsigned long long) c);
 }
 
-template <class T>
-__device__ __forceinline__ T shfl_down_t(T v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
+// entries a thread loads before it uses any
+constexpr int VEC_BATCH = 4;
 
-// Typed reduction: partial[b] = (+)_i x_i (*) y_i over i where x, y (and the
-// mask) are present; y == nullptr means "no second operand" (plain fold).
+// Where a reduction leaves its partials and its result (scalar.cuh).
+struct VecOut {
+	uint64_t *part;
+	unsigned *arrived;
+	uint64_t *out;
+};
+
+// Typed reduction: init (+) [(+)_i x_i (*) y_i] over i where x, y (and the
+// mask) are present; y == nullptr means "no second operand" (plain fold).  A
+// thread takes the entries i, i + S, i + 2S, ... (S threads in all) in that
+// order, VEC_BATCH of them loaded at a time.
 template <class T>
-__global__ void k_vec_dot(int add_op, T ident, int mul_op, int64_t n, const void *x, int xt,
+__global__ void __launch_bounds__(SCALAR_BLOCK)
+k_vec_dot(int add_op, T ident, int mul_op, int64_t n, const void *x, int xt,
 	const uint8_t *xa, const void *y, int yt, const uint8_t *ya, const void *m,
-	const uint8_t *ma, int mt, int masked, uint32_t descr, T *partials) {
-	__shared__ T sm[32];
+	const uint8_t *ma, int mt, int masked, uint32_t descr, T init, VecOut out) {
 	T acc = ident;
-	bool any = false;
-	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
-		 i += int64_t(gridDim.x) * blockDim.x) {
-		if (xa && !xa[i]) continue;
-		if (y && ya && !ya[i]) continue;
-		if (masked && !eval_mask(m, ma, mt, descr, i)) continue;
-		const T xv = ld_as<T>(x, xt, i);
-		const T yv = y ? ld_as<T>(y, yt, i) : T(0);
-		if (y && opv_skips(mul_op, yv)) continue;
-		const T t = y ? opv(mul_op, xv, yv) : xv;
-		acc = any ? opv(add_op, acc, t) : opv(add_op, ident, t);
-		any = true;
+	const int64_t S = int64_t(gridDim.x) * blockDim.x;
+	for (int64_t i0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i0 < n; i0 += VEC_BATCH * S) {
+		T xv[VEC_BATCH], yv[VEC_BATCH];
+		bool on[VEC_BATCH];
+#pragma unroll
+		for (int q = 0; q < VEC_BATCH; ++q) {
+			const int64_t i = i0 + q * S;
+			on[q] = i < n && !(xa && !xa[i]) && !(y && ya && !ya[i]) &&
+				!(masked && !eval_mask(m, ma, mt, descr, i));
+			xv[q] = on[q] ? ld_as<T>(x, xt, i) : T(0);
+			yv[q] = on[q] && y ? ld_as<T>(y, yt, i) : T(0);
+		}
+#pragma unroll
+		for (int q = 0; q < VEC_BATCH; ++q)
+			if (on[q] && !(y && opv_skips(mul_op, yv[q])))
+				acc = opv(add_op, acc, y ? opv(mul_op, xv[q], yv[q]) : xv[q]);
 	}
-	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-	for (int o = 16; o > 0; o >>= 1) acc = opv(add_op, acc, shfl_down_t(acc, o));
-	if (lane == 0) sm[wid] = acc;
-	__syncthreads();
-	if (wid == 0) {
-		T w = lane < int(blockDim.x >> 5) ? sm[lane] : ident;
-		for (int o = 16; o > 0; o >>= 1) w = opv(add_op, w, shfl_down_t(w, o));
-		if (lane == 0) partials[blockIdx.x] = w;
-	}
-}
-
-// *result = *result (+) partial[0] (+) ... (+) partial[g-1], in block order,
-// by one thread (the reference folds into the given scalar).
-template <class T>
-__global__ void k_vec_dot_finish(int add_op, const T *partials, int g, T *result) {
-	if (blockIdx.x != 0 || threadIdx.x != 0) return;
-	T acc = *result;
-	for (int b = 0; b < g; ++b) acc = opv(add_op, acc, partials[b]);
-	*result = acc;
+	scalar_finish(acc, ident, init, scalar_groups(add_op),
+		[&](T a, T b) { return opv(add_op, a, b); }, out.part, out.arrived, out.out);
 }
 
 template <class T>
@@ -318,21 +315,18 @@ static int vec_reduce_run(void *result, int add_op, uint64_t identity, int mul_o
 	uint32_t descr, int64_t n, const void *x, int x_type, const uint8_t *x_assigned,
 	const void *y, int y_type, const uint8_t *y_assigned, const void *mask,
 	const uint8_t *mask_assigned, int mask_type, int masked, cudaStream_t s) {
-	int64_t g64 = (n + 256 * 8 - 1) / (256 * 8);
-	if (g64 > int64_t(sm_count()) * 4) g64 = int64_t(sm_count()) * 4;
-	const int g = int(g64 < 1 ? 1 : g64);
-	T *part = nullptr;
-	ALPB_CUDA(cudaMallocAsync(&part, size_t(g + 1) * sizeof(T), s));
-	k_vec_dot<T><<<g, 256, 0, s>>>(add_op, from_bits<T>(identity), mul_op, n, x, x_type,
-		x_assigned, y, y_type, y_assigned, mask, mask_assigned,
-		mask == nullptr ? ALPB_VOID : mask_type, masked, descr, part);
+	ScalarScratch sc;
+	int rc = scalar_scratch(&sc, s);
+	if (rc != ALPB_SUCCESS) return rc;
+	T init;
+	memcpy(&init, result, sizeof(T));
+	k_vec_dot<T><<<scalar_grid(n), SCALAR_BLOCK, 0, s>>>(add_op, from_bits<T>(identity), mul_op, n,
+		x, x_type, x_assigned, y, y_type, y_assigned, mask, mask_assigned,
+		mask == nullptr ? ALPB_VOID : mask_type, masked, descr, init,
+		VecOut{sc.part, sc.arrived, sc.host_dev});
 	ALPB_LAUNCHED();
-	ALPB_CUDA(cudaMemcpyAsync(part + g, result, sizeof(T), cudaMemcpyHostToDevice, s));
-	k_vec_dot_finish<T><<<1, 32, 0, s>>>(add_op, part, g, part + g);
-	ALPB_LAUNCHED();
-	ALPB_CUDA(cudaMemcpyAsync(result, part + g, sizeof(T), cudaMemcpyDeviceToHost, s));
-	ALPB_CUDA(cudaFreeAsync(part, s));
 	ALPB_CUDA(cudaStreamSynchronize(s));
+	memcpy(result, sc.host, sizeof(T));
 	return ALPB_SUCCESS;
 }
 
@@ -377,8 +371,7 @@ static int vec_op_run(int kind, int op, int monoid, uint64_t identity, int mul_o
 }
 
 // ------------------------------------------------------ fused chains --
-// Steps of alpb_vec_chain, with the domain's values decoded; slot values live
-// in a per-thread array for the element being processed.
+// Steps of alpb_vec_chain, with the domain's values decoded.
 template <class T>
 struct ChainStep {
 	int32_t kind, op, mul_op, use_index, z, x, y;
@@ -397,47 +390,92 @@ struct ChainArgs {
 	T rident;
 };
 
-template <class T>
-__global__ void __launch_bounds__(256) k_vec_chain(ChainArgs<T> c, T *partials) {
-	__shared__ T sm[32];
-	T acc = c.rident;
-	bool any = false;
-	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < c.n;
-		 i += int64_t(gridDim.x) * blockDim.x) {
-		T v[ALPB_CHAIN_SLOTS];
+// op applied to VEC_BATCH pairs: one decision per step, not one per entry
+template <class T, class F>
+__device__ __forceinline__ void chain_each(T (&z)[VEC_BATCH], const T (&a)[VEC_BATCH],
+	const T (&b)[VEC_BATCH], const F &f) {
 #pragma unroll
-		for (int q = 0; q < ALPB_CHAIN_SLOTS; ++q)
-			if (q < c.nslots && ((c.load >> q) & 1)) v[q] = ld_as<T>(c.val[q], c.type[q], i);
+	for (int q = 0; q < VEC_BATCH; ++q) z[q] = f(a[q], b[q]);
+}
+template <class T>
+__device__ __forceinline__ void chain_op(int op, T (&z)[VEC_BATCH], const T (&a)[VEC_BATCH],
+	const T (&b)[VEC_BATCH]) {
+	switch (op) {
+	case ALPB_OP_ADD: chain_each(z, a, b, [](T u, T v) { return opv(ALPB_OP_ADD, u, v); }); break;
+	case ALPB_OP_SUB: chain_each(z, a, b, [](T u, T v) { return opv(ALPB_OP_SUB, u, v); }); break;
+	case ALPB_OP_MUL: chain_each(z, a, b, [](T u, T v) { return opv(ALPB_OP_MUL, u, v); }); break;
+	default: chain_each(z, a, b, [op](T u, T v) { return opv(op, u, v); }); break;
+	}
+}
+
+// The entries i, i + S, ... of a thread, VEC_BATCH at a time.  The slots'
+// values wait in shared memory, [slot][batch][thread]: the steps name their
+// slots by number, and an array indexed so in registers went to local memory
+// (40 us for two updates and a dot on 1e6 entries; 48 MB of vectors).
+template <class T>
+__global__ void __launch_bounds__(SCALAR_BLOCK) k_vec_chain(ChainArgs<T> c, T init, VecOut out) {
+	extern __shared__ __align__(16) unsigned char chain_smem[];
+	T *v = reinterpret_cast<T *>(chain_smem) + threadIdx.x;
+	const auto at = [&](int slot, int q) -> T & {
+		return v[(slot * VEC_BATCH + q) * SCALAR_BLOCK];
+	};
+	T acc = c.rident;
+	const int64_t S = int64_t(gridDim.x) * blockDim.x;
+	for (int64_t i0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i0 < c.n;
+		 i0 += VEC_BATCH * S) {
+		for (int s = 0; s < c.nslots; ++s)
+			if ((c.load >> s) & 1) {
+				T t[VEC_BATCH];
+#pragma unroll
+				for (int q = 0; q < VEC_BATCH; ++q)
+					t[q] = i0 + q * S < c.n ? ld_as<T>(c.val[s], c.type[s], i0 + q * S) : T(0);
+#pragma unroll
+				for (int q = 0; q < VEC_BATCH; ++q) at(s, q) = t[q];
+			}
+		const auto get = [&](int slot, T scalar, T (&t)[VEC_BATCH]) {
+#pragma unroll
+			for (int q = 0; q < VEC_BATCH; ++q) t[q] = slot >= 0 ? at(slot, q) : scalar;
+		};
 		for (int k = 0; k < c.nsteps; ++k) {
 			const ChainStep<T> &o = c.step[k];
-			const T xv = o.x >= 0 ? v[o.x] : o.alpha;
-			const T yv = o.y >= 0 ? v[o.y] : o.beta;
+			T x[VEC_BATCH], y[VEC_BATCH], z[VEC_BATCH];
+			get(o.x, o.alpha, x);
+			if (o.kind != ALPB_VEC_SET) get(o.z, T(0), z);
 			switch (o.kind) {
-			case ALPB_VEC_SET: v[o.z] = o.use_index ? T(i) : xv; break;
-			case ALPB_VEC_FOLDL: v[o.z] = opv(o.op, v[o.z], xv); break;
-			case ALPB_VEC_FOLDR: v[o.z] = opv(o.op, xv, v[o.z]); break;
-			default: v[o.z] = opv(o.op, v[o.z], opv(o.mul_op, xv, yv)); break;  // MULADD
+			case ALPB_VEC_SET:
+#pragma unroll
+				for (int q = 0; q < VEC_BATCH; ++q) z[q] = o.use_index ? T(i0 + q * S) : x[q];
+				break;
+			case ALPB_VEC_FOLDL: chain_op(o.op, z, z, x); break;
+			case ALPB_VEC_FOLDR: chain_op(o.op, z, x, z); break;
+			default:   // MULADD
+				get(o.y, o.beta, y);
+				chain_op(o.mul_op, x, x, y);
+				chain_op(o.op, z, z, x);
+				break;
 			}
+#pragma unroll
+			for (int q = 0; q < VEC_BATCH; ++q) at(o.z, q) = z[q];
 		}
 		if (c.reduce) {   // as k_vec_dot on dense operands
-			const T t = c.ry >= 0 ? opv(c.rmul, v[c.rx], v[c.ry]) : v[c.rx];
-			acc = any ? opv(c.radd, acc, t) : opv(c.radd, c.rident, t);
-			any = true;
-		}
+			T x[VEC_BATCH], y[VEC_BATCH];
+			get(c.rx, T(0), x);
+			get(c.ry, T(0), y);
+			if (c.ry >= 0) chain_op(c.rmul, x, x, y);
 #pragma unroll
-		for (int q = 0; q < ALPB_CHAIN_SLOTS; ++q)
-			if (q < c.nslots && ((c.store >> q) & 1)) st_as<T>(c.val[q], c.type[q], i, v[q]);
+			for (int q = 0; q < VEC_BATCH; ++q)
+				if (i0 + q * S < c.n) acc = opv(c.radd, acc, x[q]);
+		}
+		for (int s = 0; s < c.nslots; ++s)
+			if ((c.store >> s) & 1) {
+#pragma unroll
+				for (int q = 0; q < VEC_BATCH; ++q)
+					if (i0 + q * S < c.n) st_as<T>(c.val[s], c.type[s], i0 + q * S, at(s, q));
+			}
 	}
 	if (!c.reduce) return;
-	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-	for (int o = 16; o > 0; o >>= 1) acc = opv(c.radd, acc, shfl_down_t(acc, o));
-	if (lane == 0) sm[wid] = acc;
-	__syncthreads();
-	if (wid == 0) {
-		T w = lane < int(blockDim.x >> 5) ? sm[lane] : c.rident;
-		for (int o = 16; o > 0; o >>= 1) w = opv(c.radd, w, shfl_down_t(w, o));
-		if (lane == 0) partials[blockIdx.x] = w;
-	}
+	scalar_finish(acc, c.rident, init, scalar_groups(c.radd),
+		[&](T a, T b) { return opv(c.radd, a, b); }, out.part, out.arrived, out.out);
 }
 
 static bool domain_type(int domain, int type) {
@@ -506,25 +544,27 @@ static int vec_chain_run(int domain, int64_t n, int nslots, void *const *values,
 		d.beta = from_bits<T>(o.beta);
 	}
 	c.store = written;
+	const size_t smem = size_t(nslots) * VEC_BATCH * SCALAR_BLOCK * sizeof(T);
+	if (smem > 48 * 1024)   // seven or eight slots of 8 bytes
+		ALPB_CUDA(cudaFuncSetAttribute(k_vec_chain<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			int(smem)));
 	if (!c.reduce) {
-		k_vec_chain<T><<<grid_for(n, 256), 256, 0, s>>>(c, nullptr);
+		k_vec_chain<T><<<grid_for((n + VEC_BATCH - 1) / VEC_BATCH, SCALAR_BLOCK), SCALAR_BLOCK, smem,
+			s>>>(c, T(0), VecOut{});
 		ALPB_LAUNCHED();
 		return ALPB_SUCCESS;
 	}
 	// the reduction's grid and order are those of alpb_vec_reduce_dom
-	int64_t g64 = (n + 256 * 8 - 1) / (256 * 8);
-	if (g64 > int64_t(sm_count()) * 4) g64 = int64_t(sm_count()) * 4;
-	const int g = int(g64 < 1 ? 1 : g64);
-	T *part = nullptr;
-	ALPB_CUDA(cudaMallocAsync(&part, size_t(g + 1) * sizeof(T), s));
-	k_vec_chain<T><<<g, 256, 0, s>>>(c, part);
+	ScalarScratch sc;
+	const int rc = scalar_scratch(&sc, s);
+	if (rc != ALPB_SUCCESS) return rc;
+	T init;
+	memcpy(&init, result, sizeof(T));
+	k_vec_chain<T><<<scalar_grid(n), SCALAR_BLOCK, smem, s>>>(c, init,
+		VecOut{sc.part, sc.arrived, sc.host_dev});
 	ALPB_LAUNCHED();
-	ALPB_CUDA(cudaMemcpyAsync(part + g, result, sizeof(T), cudaMemcpyHostToDevice, s));
-	k_vec_dot_finish<T><<<1, 32, 0, s>>>(c.radd, part, g, part + g);
-	ALPB_LAUNCHED();
-	ALPB_CUDA(cudaMemcpyAsync(result, part + g, sizeof(T), cudaMemcpyDeviceToHost, s));
-	ALPB_CUDA(cudaFreeAsync(part, s));
 	ALPB_CUDA(cudaStreamSynchronize(s));
+	memcpy(result, sc.host, sizeof(T));
 	return ALPB_SUCCESS;
 }
 

@@ -1,6 +1,7 @@
 // Runtime entry points: init/finalize, error reporting, device memory and
 // copies used by the container classes of the grb::b200 backend.
 #include "common.cuh"
+#include "scalar.cuh"
 
 #include <cstdarg>
 #include <mutex>
@@ -44,6 +45,55 @@ size_t type_size(int type) {
 	case ALPB_UINT64: return 8;
 	}
 	return 0;
+}
+
+// A thread's reduction scratch on each device; the destructor runs when the
+// thread ends (at process exit the runtime may already be gone: its errors are
+// of no consequence then).
+struct ScalarPool {
+	static constexpr int kDevices = 64;
+	ScalarScratch dev[kDevices];
+	~ScalarPool() {
+		for (int d = 0; d < kDevices; ++d) {
+			if (dev[d].part) cudaFree(dev[d].part);
+			if (dev[d].host) cudaFreeHost(dev[d].host);
+		}
+	}
+};
+static thread_local ScalarPool t_scalar;
+
+int scalar_scratch(ScalarScratch *out, cudaStream_t s) {
+	int d = 0;
+	ALPB_CUDA(cudaGetDevice(&d));
+	ALPB_CHECK(d < ScalarPool::kDevices, ALPB_UNSUPPORTED, "device ordinal %d", d);
+	ScalarScratch &p = t_scalar.dev[d];
+	if (!p.part) {
+		// allocations of a first call must not disturb a capture that another
+		// thread has under way
+		cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+		cudaThreadExchangeStreamCaptureMode(&mode);
+		ScalarScratch n;
+		const size_t bytes = size_t(SCALAR_MAX_BLOCKS) * 8 + 8;
+		cudaError_t e = cudaMalloc(&n.part, bytes);
+		if (e == cudaSuccess) e = cudaMemsetAsync(n.part, 0, bytes, s);
+		if (e == cudaSuccess)
+			e = cudaHostAlloc(reinterpret_cast<void **>(&n.host), 64, cudaHostAllocMapped);
+		if (e == cudaSuccess)
+			e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&n.host_dev), n.host, 0);
+		if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+		cudaThreadExchangeStreamCaptureMode(&mode);
+		if (e != cudaSuccess) {
+			cudaGetLastError();
+			if (n.part) cudaFree(n.part);
+			if (n.host) cudaFreeHost(n.host);
+			set_error("reduction scratch: %s", cudaGetErrorString(e));
+			return e == cudaErrorMemoryAllocation ? ALPB_OUTOFMEM : ALPB_PANIC;
+		}
+		n.arrived = reinterpret_cast<unsigned *>(n.part + SCALAR_MAX_BLOCKS);
+		p = n;
+	}
+	*out = p;
+	return ALPB_SUCCESS;
 }
 
 } // namespace alpb

@@ -1,0 +1,122 @@
+"""Reductions to a host scalar in one launch: sizes at the edges of a thread's
+batch, of a block and of the largest grid, every monoid, an initial value, the
+scratch of several threads and streams at once, and chains of eight slots.
+
+Integers must be exact (64-bit wrap-around).  FP64 sums of n values in [0, 1)
+in two orders agree to 2 n 2^-53 of the sum."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 31, 255, 256, 1023, 1025, 2047, 2048, 2049, 8193, 592 * 2048, 592 * 2048 + 1, 3000001]
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_integer_reductions(cuda, n):
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    rng = np.random.default_rng(n)
+    x = rng.integers(-2 ** 62, 2 ** 62, n)
+    y = rng.integers(-2 ** 62, 2 ** 62, n)
+    m = (rng.random(n) < 0.4).astype(np.uint8)
+    tx, ty, tm = (torch.from_numpy(a).cuda() for a in (x, y, m))
+    with np.errstate(over="ignore"):
+        cases = {abi.OP_ADD: (0, lambda v, i: np.add.reduce(v, initial=i)),
+                 abi.OP_MUL: (1, lambda v, i: np.multiply.reduce(v, initial=i)),
+                 abi.OP_MIN: (2 ** 63 - 1, lambda v, i: min(i, v.min(initial=2 ** 63 - 1))),
+                 abi.OP_MAX: (-2 ** 63, lambda v, i: max(i, v.max(initial=-2 ** 63)))}
+        for op, (ident, fold) in cases.items():
+            for masked in (0, 1):
+                keep = m != 0 if masked else slice(None)
+                for two in (False, True):
+                    terms = (x * y if two else x)[keep]
+                    res = C.c_int64(12345)
+                    abi.call("alpb_vec_reduce_dom", C.byref(res), op, ident % 2 ** 64, abi.OP_MUL, 0,
+                             abi.INT64, n, dev.ptr(tx), abi.INT64, None,
+                             dev.ptr(ty) if two else None, abi.INT64, None, dev.ptr(tm), None,
+                             abi.BOOL, masked, dev.stream_ptr())
+                    assert res.value == int(fold(terms, np.int64(12345))), (op, masked, two)
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_dot_and_fold(cuda, n):
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    rng = np.random.default_rng(n)
+    x, y = rng.random(n), rng.random(n)
+    xa = (rng.random(n) < 0.7).astype(np.uint8)
+    tx, ty, ta = (torch.from_numpy(a).cuda() for a in (x, y, xa))
+    tol = 2 * n * 2.0 ** -53
+    for flags, keep in ((None, slice(None)), (dev.ptr(ta), xa != 0)):
+        d = C.c_double(0.5)
+        abi.call("alpb_dot_f64", C.byref(d), abi.OP_ADD, abi.OP_MUL, n, dev.ptr(tx), flags,
+                 dev.ptr(ty), None, dev.stream_ptr())
+        want = 0.5 + np.dot(x[keep], y[keep])
+        assert abs(d.value - want) <= tol * want
+        d = C.c_double(2.0)
+        abi.call("alpb_reduce_f64", C.byref(d), abi.OP_MIN, n, dev.ptr(tx), flags, dev.stream_ptr())
+        assert d.value == min(2.0, x[keep].min(initial=np.inf))
+    abi.call("alpb_foldl_f64", dev.ptr(tx), abi.OP_SUB, n, dev.ptr(ty), 0.0, dev.stream_ptr())
+    assert np.array_equal(tx.cpu().numpy(), x - y)
+
+
+def test_threads_and_streams(cuda):
+    """Each thread reduces its own vectors on its own stream, many times."""
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    bad = []
+
+    def work(k):
+        torch.cuda.set_device(0)
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            x = torch.arange(1000 * (k + 1) * 7, device="cuda", dtype=torch.int64)
+            s.synchronize()
+            want = int(x.sum())
+            for _ in range(200):
+                r = C.c_int64(k)
+                abi.call("alpb_vec_reduce_dom", C.byref(r), abi.OP_ADD, 0, abi.OP_MUL, 0, abi.INT64,
+                         x.numel(), dev.ptr(x), abi.INT64, None, None, abi.INT64, None, None, None,
+                         abi.BOOL, 0, dev.stream_ptr(s))
+                if r.value != want + k:
+                    bad.append((k, r.value))
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(6)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
+
+
+@pytest.mark.parametrize("n", [1, 1025, 300001])
+def test_chain_of_eight_slots(cuda, n):
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    rng = np.random.default_rng(n)
+    v = [rng.integers(-1000, 1000, n) for _ in range(8)]
+    t = [torch.from_numpy(a.copy()).cuda() for a in v]
+    S = abi.VecStep
+    steps = [S(kind=abi.VEC_MULADD, op=abi.OP_ADD, mul_op=abi.OP_MUL, z=k, x=k + 1, y=7)
+             for k in range(6)]
+    steps += [S(kind=abi.VEC_FOLDR, op=abi.OP_SUB, z=7, x=0, y=-1),
+              S(kind=abi.VEC_SET, z=6, x=-1, y=-1, descr=abi.DESC_USE_INDEX),
+              S(kind=abi.VEC_REDUCE, op=abi.OP_ADD, mul_op=abi.OP_MUL, z=-1, x=0, y=7)]
+    for k in range(6):
+        v[k] = v[k] + v[k + 1] * v[7]
+    v[7] = v[0] - v[7]
+    v[6] = np.arange(n)
+    res = C.c_int64(5)
+    abi.call("alpb_vec_chain", abi.INT64, n, 8, (C.c_void_p * 8)(*[a.data_ptr() for a in t]),
+             (C.c_int * 8)(*[abi.INT64] * 8), len(steps), (S * len(steps))(*steps), C.byref(res),
+             dev.stream_ptr())
+    for a, b in zip(t, v):
+        assert np.array_equal(a.cpu().numpy(), b)
+    assert res.value == 5 + int((v[0] * v[7]).sum())
