@@ -11,109 +11,101 @@
 // of them.  Each right-hand side keeps its own CG scalars and its own
 // convergence test, exactly as separate runs of the algorithm would.
 //
-// Kernels (all FP64, each row's sum in CRS order):
-//   k_hpcg_rows<NRHS, Op>  one kernel for every row-wise product: the SpMM
-//                          A p, a colour step of the smoother (x_i = (r_i -
-//                          (A x)_i + x_i d) / d on the rows of one colour),
-//                          the restriction (r_c = r_f - A z at injected fine
-//                          rows only) and the prolongation (z_f += z_c)
-//   k_hpcg_dot / k_hpcg_finish  per-right-hand-side dot products in a fixed
-//                          order, and the CG scalar updates on the device
-//   k_hpcg_axpy...         the CG vector updates
+// Kernels (all FP64, every sum in a fixed order):
+//   k_hpcg_cycle<NRHS>   one V-cycle as one persistent cooperative launch: a
+//                        colour step, a restriction or a prolongation between
+//                        two grid barriers
+//   k_hpcg_spmm<NRHS>    A p and the block partials of p . A p
+//   k_hpcg_dot, k_hpcg_axpby, k_hpcg_update   the CG vector steps, with block
+//                        partials of the dot product that follows
+//   k_hpcg_finish        the partials summed, then the CG scalars on the device
 #include "common.cuh"
+#include "persist.cuh"
 
 #include <cmath>
 #include <vector>
 
 namespace alpb {
 
-constexpr int HG_GROUP = 8;     // lanes per matrix row
 constexpr int HG_BLOCK = 256;
+constexpr int HG_ROW = 27;          // entries of a stencil row, at most
+constexpr uint32_t HG_NONE = 0xffffffffu;
 
-// Row-wise product engine: a group of 8 lanes per row; lane q handles the
-// right-hand side q % NRHS and the nonzeroes s, s + S, ... of the row, with
-// s = q / NRHS and S = 8 / NRHS; the S partial sums are combined by an xor
-// tree.  With NRHS = 8 every lane walks its row in CRS order.
-template <int NRHS, class Op>
-__global__ void __launch_bounds__(HG_BLOCK)
-k_hpcg_rows(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ indices,
-	const double *__restrict__ values, const double *__restrict__ x, int64_t count, Op op) {
-	constexpr int S = HG_GROUP / NRHS;
-	constexpr int GPW = 32 / HG_GROUP;  // row groups per warp
-	const int q = threadIdx.x & (HG_GROUP - 1);
-	const int k = q % NRHS, s = q / NRHS;
-	const int g = (threadIdx.x & 31) / HG_GROUP;
-	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
-	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-	// the loop bound is the same for the whole warp, so every lane reaches
-	// every shuffle below
-	for (int64_t wb = warp * GPW; wb < count; wb += nwarps * GPW) {
-		const int64_t idx = wb + g;
-		const bool valid = idx < count;
-		double acc = 0.0;
-		int64_t row = 0;
-		if (valid) {
-			row = op.row(idx);
-			const int64_t b = offsets[row], e = offsets[row + 1];
-			for (int64_t j = b + s; j < e; j += S)
-				acc += values[j] * x[int64_t(indices[j]) * NRHS + k];
+// Loads of the matrix, which no kernel writes, kept where they stand: ahead of
+// the barrier that precedes their use.
+__device__ __forceinline__ void hg_load(uint32_t &v, const uint32_t *p) {
+	asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+}
+__device__ __forceinline__ void hg_load(double &v, const double *p) {
+	asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+}
+__device__ __forceinline__ void hg_load(int64_t &v, const int64_t *p) {
+	asm volatile("ld.global.nc.s64 %0, [%1];" : "=l"(v) : "l"(p));
+}
+
+// One row's product by GL lanes: lane (s, k) of the group takes right-hand
+// side k = lane % NRHS and the entries s, s + S, ... of the row (at most NE,
+// so all of a lane's loads are in flight together: a colour step is one
+// dependent chain offsets -> indices -> x, and the serial walk it replaces
+// paid that chain once per few entries); the S partial sums are combined by
+// an xor tree.
+template <int NRHS>
+struct HgRow {
+	static constexpr int GL = 8 * NRHS < 32 ? 8 * NRHS : 32;
+	static constexpr int RPW = 32 / GL;     // rows per warp
+	static constexpr int S = GL / NRHS;
+	static constexpr int NE = (HG_ROW + S - 1) / S;
+	// where a row's entries are: its offset and length (row < 0: none)
+	struct At {
+		int64_t o;
+		int len;
+	};
+	static __device__ __forceinline__ At at(const int64_t *__restrict__ offsets, int64_t row) {
+		At r{0, 0};
+		if (row >= 0) {
+			int64_t e;
+			hg_load(r.o, offsets + row);
+			hg_load(e, offsets + row + 1);
+			r.len = int(e - r.o);
 		}
+		return r;
+	}
+	uint32_t j[NE];
+	double v[NE];
+	__device__ __forceinline__ void load(const uint32_t *__restrict__ indices,
+		const double *__restrict__ values, const At &r) {
+		const int s = (threadIdx.x & (GL - 1)) / NRHS;
 #pragma unroll
-		for (int o = NRHS; o < HG_GROUP; o <<= 1) {
-			const double w = __shfl_xor_sync(0xffffffffu, acc, o);
-			acc += w;
-		}
-		if (valid && s == 0) op.finish(idx, row, k, acc);
-	}
-}
-
-// ------------------------------------------------------- row operations --
-// y = 0 + A x on every row (set( y, 0 ); mxv( y, A, x ))
-template <int NRHS>
-struct HgSpmm {
-	double *y;
-	__device__ __forceinline__ int64_t row(int64_t i) const { return i; }
-	__device__ __forceinline__ void finish(int64_t, int64_t r, int k, double acc) const {
-		y[r * NRHS + k] = 0.0 + acc;
-	}
-};
-
-// One colour step of the smoother on rows c, c + K, c + 2K, ... (the rows
-// whose index is c modulo K), red_black_gauss_seidel.hpp:63-86:
-//   temp = 0 + A[mask] x;  x[mask] = (r - temp + x d) / d.
-// Fused (temp never stored) when no two neighbours share a colour, so that
-// no row of the colour reads another's new value; otherwise `temp` receives
-// the products and k_hpcg_color_update applies them.
-template <int NRHS>
-struct HgColor {
-	const double *r;
-	double *x;
-	double *temp;  // null: fused
-	double d;
-	int64_t c, K;
-	__device__ __forceinline__ int64_t row(int64_t i) const { return c + i * K; }
-	__device__ __forceinline__ void finish(int64_t, int64_t row, int k, double acc) const {
-		const double t = 0.0 + acc;
-		const int64_t at = row * NRHS + k;
-		if (temp) {
-			temp[at] = t;
-		} else {
-			const double v = r[at] - t + x[at] * d;
-			x[at] = v / d;
+		for (int q = 0; q < NE; ++q) {
+			const int e = s + q * S;
+			j[q] = HG_NONE;
+			v[q] = 0.0;
+			if (e < r.len) {
+				hg_load(j[q], indices + r.o + e);
+				hg_load(v[q], values + r.o + e);
+			}
 		}
 	}
-};
-
-template <int NRHS>
-__global__ void k_hpcg_color_update(const double *r, const double *temp, double *x, double d,
-	int64_t c, int64_t K, int64_t count) {
-	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < count * NRHS;
-		 i += int64_t(gridDim.x) * blockDim.x) {
-		const int64_t at = (c + (i / NRHS) * K) * NRHS + i % NRHS;
-		const double v = r[at] - temp[at] + x[at] * d;
-		x[at] = v / d;
+	// sum_e v_e x[j_e], read through L2 (x changes between the barriers of a
+	// cycle, and a step reads no line of it twice); after_sum runs once the
+	// gathered values are used
+	template <class F>
+	__device__ __forceinline__ double product(const double *x, F &&after_sum) const {
+		const int k = threadIdx.x % NRHS;
+		double g[NE], acc = 0.0;
+#pragma unroll
+		for (int q = 0; q < NE; ++q) g[q] = j[q] != HG_NONE ? __ldcg(x + int64_t(j[q]) * NRHS + k) : 0.0;
+#pragma unroll
+		for (int q = 0; q < NE; ++q)
+			if (j[q] != HG_NONE) acc = fma(v[q], g[q], acc);
+		after_sum();
+#pragma unroll
+		for (int o = NRHS; o < GL; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+		return acc;
 	}
-}
+	static __device__ __forceinline__ int sub() { return (threadIdx.x & 31) / GL; }
+	static __device__ __forceinline__ bool lead() { return (threadIdx.x & (GL - 1)) < NRHS; }
+};
 
 // Fine row of coarse point c under injection: coarse (cx, cy, cz) takes the
 // fine point (2cx, 2cy, 2cz) (coarsener_generator_iterator,
@@ -126,47 +118,200 @@ struct HgInject {
 	}
 };
 
-// Restriction, compute_coarsening (multigrid_v_cycle.hpp:67-86): with
-// Ax = 0 + A z, r_c = 0 + 1 (r_f - Ax) at the injected rows; the product is
-// formed only where the injection reads it.
-template <int NRHS>
-struct HgRestrict {
-	const double *r_f;
-	double *r_c;
-	HgInject inj;
-	__device__ __forceinline__ int64_t row(int64_t c) const { return inj(c); }
-	__device__ __forceinline__ void finish(int64_t c, int64_t f, int k, double acc) const {
-		const double ax = 0.0 + acc;
-		r_c[c * NRHS + k] = 0.0 + 1.0 * (r_f[f * NRHS + k] - ax);
-	}
+// One level as the cycle kernel sees it.
+struct HgLevelArgs {
+	const int64_t *offsets;
+	const uint32_t *indices;
+	const double *values;
+	double *r, *z, *temp;   // temp: null when the smoother is fused
+	int64_t n, nx, ny;
 };
+constexpr int HG_MAX_LEVELS = 16;   // every level halves three dimensions
 
-// Prolongation, compute_prolongation (multigrid_v_cycle.hpp:88-103):
-// z_f += 0 + 1 z_c at the injected rows (the other rows add zero).
-template <int NRHS>
-__global__ void k_hpcg_prolong(double *z_f, const double *z_c, HgInject inj, int64_t count) {
-	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < count * NRHS;
-		 i += int64_t(gridDim.x) * blockDim.x) {
-		const int64_t c = i / NRHS;
-		const int k = int(i % NRHS);
-		const int64_t at = inj(c) * NRHS + k;
-		z_f[at] = z_f[at] + (0.0 + 1.0 * z_c[i]);
+struct HgCycleArgs {
+	HgLevelArgs lv[HG_MAX_LEVELS];
+	int l0, l1;              // this launch's levels [l0, l1)
+	int part;                // HG_DOWN, HG_UP or HG_WHOLE
+	int64_t colors, pre, post;
+	double diag;
+	GridSync *gs;
+	const int32_t *active;   // right-hand sides still iterating: none, no work
+};
+enum { HG_DOWN, HG_UP, HG_WHOLE };
+
+constexpr int HGC_THREADS = 768;
+constexpr int HGC_CLUSTER = 16;     // blocks of a cluster launch
+
+// multi_grid (multigrid_v_cycle.hpp:193-246) on the levels [l0, l1): z = 0;
+// smooth; restrict the residual; recurse; prolong; smooth.  HG_WHOLE ends at
+// the coarsest level, which smooths once; HG_DOWN stops after the restriction
+// to level l1 and HG_UP begins with the prolongation from it.  A smoother
+// (red_black_gauss_seidel.hpp:55-123) is 2 x colors steps, forward then
+// backward, each
+//   temp = 0 + A[mask] x;  x[mask] = (r - temp + x d) / d
+// on the rows c, c + K, ...: in place when no two neighbours share a colour,
+// so that no row of the colour reads another's new value; otherwise the
+// products are stored first and applied after a barrier.
+//
+// What bounds it is the chain of steps: 378 of them per cycle on 64^3 with
+// three coarser levels, each a few thousand rows at most.  As separate
+// launches a step took 17.5 us.  Here it is a barrier, one round of gathers
+// and the update; the entries of a warp's next row are in flight, and the
+// place of the one after is known, before the barrier, so only x is read
+// after it.  CLUSTER: one cluster of blocks with its hardware barrier instead
+// of a block per SM with a barrier through L2 -- coarse levels, where the
+// barrier is most of a step: 1.0 us there, 1.8 us through L2.  Measured us per
+// HPCG iteration, launches -> this: 16^3 with 8 right-hand sides 1451 -> 341,
+// 64^3 with 1 2499 -> 971, 64^3 with 8 4088 -> 1508, 128^3 with 8 10576 -> 8377.
+template <int NRHS, bool CLUSTER>
+__global__ void __launch_bounds__(HGC_THREADS, 1) k_hpcg_cycle(HgCycleArgs a) {
+	using Row = HgRow<NRHS>;
+	using At = typename Row::At;
+	if (*a.active == 0) return;
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	const int k = lane % NRHS;
+	const int G = gridDim.x;
+	// rows and steps in 32 bits: 2^31 stencil rows are more than the memory
+	// rows go round the blocks first, so small steps use every SM
+	const int nrow = G * (HGC_THREADS / 32) * Row::RPW;
+	const int row0 = (w * G + int(blockIdx.x)) * Row::RPW;   // the warp's first
+	const int64_t tid = blockIdx.x * int64_t(HGC_THREADS) + threadIdx.x;
+	const int64_t nthreads = int64_t(G) * HGC_THREADS;
+	const int K = int(a.colors);
+	const auto barrier = [&]() {
+		if constexpr (CLUSTER) {
+			// one fence for the block's writes instead of one per thread
+			__syncthreads();
+			if (threadIdx.x == 0) asm volatile("fence.acq_rel.cluster;" ::: "memory");
+			__syncwarp();
+			asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+			asm volatile("barrier.cluster.wait;" ::: "memory");
+			return true;
+		} else {
+			return grid_sync(a.gs);
+		}
+	};
+
+	// one smoother on level L; false: a barrier gave up
+	const auto smooth = [&](const HgLevelArgs &L) {
+		// rows t, t + 1, ... of a step's colour belong to the warp's lane groups
+		struct Pos {
+			int step, t;
+		};
+		const auto color = [&](int step) { return step < K ? step : 2 * K - 1 - step; };
+		const auto row_of = [&](const Pos &p, int sub) {
+			const int64_t i = color(p.step) + int64_t(p.t + sub) * K;
+			return p.step < 2 * K && i < L.n ? int(i) : -1;
+		};
+		const auto next = [&](Pos p) {   // the warp's next rows: this step's, else the next one's
+			p.t += nrow;
+			if (row_of(p, 0) < 0) p = Pos{p.step + 1, row0};
+			return p;
+		};
+		Pos p0{0, row0}, p1 = next(p0);
+		int i0 = row_of(p0, Row::sub()), i1 = row_of(p1, Row::sub());
+		// One item: the product of p0's rows, entries in `cur`; p1's entries go
+		// to `nxt` from their place `at`, and p2's place to `at_next`: after the
+		// sum, since gathers that share a scoreboard with later loads wait for
+		// those too.  The two sets of registers swap roles from item to item
+		// (copying one to the other would wait for the loads just issued).
+		const auto item = [&](Row &cur, Row &nxt, const At &at, At &at_next) {
+			const Pos p2 = next(p1);
+			const int i2 = row_of(p2, Row::sub());
+			const int64_t o = int64_t(i0) * NRHS + k;
+			const bool mine = i0 >= 0 && Row::lead();
+			const double ri = mine ? __ldcg(L.r + o) : 0.0, xi = mine ? __ldcg(L.z + o) : 0.0;
+			const double p = cur.product(L.z, [&]() {
+				nxt.load(L.indices, L.values, at);
+				at_next = Row::at(L.offsets, i2);
+			});
+			if (mine) {
+				if (L.temp) L.temp[o] = p;
+				else L.z[o] = (ri - p + xi * a.diag) / a.diag;
+			}
+			p0 = p1;
+			p1 = p2;
+			i0 = i1;
+			i1 = i2;
+		};
+		int step = 0;
+		// the barriers between this warp's last item of `step` and its next one
+		const auto end_of_step = [&]() {
+			if (!barrier()) return false;
+			if (L.temp) {
+				const int64_t c = color(step);
+				const int64_t count = c < L.n ? (L.n - 1 - c) / K + 1 : 0;
+				for (int64_t q = tid; q < count * NRHS; q += nthreads) {
+					const int64_t o = (c + (q / NRHS) * K) * NRHS + q % NRHS;
+					L.z[o] = (L.r[o] - L.temp[o] + L.z[o] * a.diag) / a.diag;
+				}
+				if (!barrier()) return false;
+			}
+			++step;
+			return true;
+		};
+		Row even, odd;
+		At at_odd = Row::at(L.offsets, i1), at_even;
+		even.load(L.indices, L.values, Row::at(L.offsets, i0));
+		while (step < 2 * K) {
+			item(even, odd, at_odd, at_even);
+			if (p0.step != step && !end_of_step()) return false;
+			if (step == 2 * K) break;
+			item(odd, even, at_even, at_odd);
+			if (p0.step != step && !end_of_step()) return false;
+		}
+		return true;
+	};
+
+	if (a.part != HG_UP) {
+		if (a.l0 == 0) {
+			for (int64_t q = tid; q < a.lv[0].n * NRHS; q += nthreads) a.lv[0].z[q] = 0.0;
+			if (!barrier()) return;
+		}
+		for (int l = a.l0; l < (a.part == HG_WHOLE ? a.l1 - 1 : a.l1); ++l) {
+			const HgLevelArgs &L = a.lv[l], &C = a.lv[l + 1];
+			for (int64_t q = 0; q < a.pre; ++q)
+				if (!smooth(L)) return;
+			// restriction, compute_coarsening (multigrid_v_cycle.hpp:67-86): r_c =
+			// r_f - A z at the injected rows, formed only there; the coarse z = 0
+			const HgInject inj{C.nx, C.ny, L.nx, L.ny};
+			for (int64_t t0 = row0; t0 < C.n; t0 += nrow) {
+				const int64_t t = t0 + Row::sub();
+				const int64_t f = t < C.n ? inj(t) : -1;
+				Row row;
+				row.load(L.indices, L.values, Row::at(L.offsets, f));
+				const double ax = row.product(L.z, [] {});
+				if (f >= 0 && Row::lead()) {
+					C.r[t * NRHS + k] = L.r[f * NRHS + k] - ax;
+					C.z[t * NRHS + k] = 0.0;
+				}
+			}
+			if (!barrier()) return;
+		}
+		if (a.part == HG_WHOLE && !smooth(a.lv[a.l1 - 1])) return;
+	}
+	if (a.part == HG_DOWN) return;
+	for (int l = a.part == HG_WHOLE ? a.l1 - 2 : a.l1 - 1; l >= a.l0; --l) {
+		const HgLevelArgs &L = a.lv[l], &C = a.lv[l + 1];
+		// prolongation, compute_prolongation (multigrid_v_cycle.hpp:88-103): z_f
+		// += z_c at the injected rows (the other rows add zero)
+		const HgInject inj{C.nx, C.ny, L.nx, L.ny};
+		for (int64_t q = tid; q < C.n * NRHS; q += nthreads) {
+			const int64_t o = inj(q / NRHS) * NRHS + q % NRHS;
+			L.z[o] = L.z[o] + C.z[q];
+		}
+		if (!barrier()) return;
+		for (int64_t q = 0; q < a.post; ++q)
+			if (!smooth(L)) return;
 	}
 }
 
 // ------------------------------------------------------------ CG pieces --
-// Per-right-hand-side dot products x_k . y_k: block partials, then one block
-// sums them in block order (fixed order: deterministic).
+// Per-right-hand-side sums of a block: thread t holds a term of right-hand
+// side t % NRHS (blocks are a multiple of NRHS).  Fixed order: deterministic.
 template <int NRHS>
-__global__ void __launch_bounds__(HG_BLOCK)
-k_hpcg_dot(const double *__restrict__ x, const double *__restrict__ y, int64_t n,
-	double *partials) {
+__device__ __forceinline__ void hg_block_partials(double acc, double *partials) {
 	__shared__ double sm[HG_BLOCK];
-	// thread t handles right-hand side t % NRHS (HG_BLOCK is a multiple of NRHS)
-	double acc = 0.0;
-	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n * NRHS;
-		 i += int64_t(gridDim.x) * blockDim.x)
-		acc += x[i] * y[i];
 	sm[threadIdx.x] = acc;
 	__syncthreads();
 	for (int w = HG_BLOCK / 2; w >= NRHS; w >>= 1) {
@@ -176,14 +321,39 @@ k_hpcg_dot(const double *__restrict__ x, const double *__restrict__ y, int64_t n
 	if (threadIdx.x < NRHS) partials[blockIdx.x * NRHS + threadIdx.x] = sm[threadIdx.x];
 }
 
-// out[k] = 0 + sum over blocks of partials[., k]
+// partials of x_k . y_k
 template <int NRHS>
-__global__ void k_hpcg_dot_finish(const double *partials, int nblocks, double *out) {
-	const int k = threadIdx.x;
-	if (k >= NRHS) return;
-	double v = 0.0;
-	for (int b = 0; b < nblocks; ++b) v += partials[b * NRHS + k];
-	out[k] = 0.0 + v;
+__global__ void __launch_bounds__(HG_BLOCK)
+k_hpcg_dot(const double *__restrict__ x, const double *__restrict__ y, int64_t n,
+	double *partials) {
+	double acc = 0.0;
+	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n * NRHS;
+		 i += int64_t(gridDim.x) * blockDim.x)
+		acc += x[i] * y[i];
+	hg_block_partials<NRHS>(acc, partials);
+}
+
+// y = 0 + A x on every row (set( y, 0 ); mxv( y, A, x )) and the partials of x . y
+template <int NRHS>
+__global__ void __launch_bounds__(HG_BLOCK)
+k_hpcg_spmm(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ indices,
+	const double *__restrict__ values, const double *__restrict__ x, double *__restrict__ y,
+	int64_t n, double *partials) {
+	using Row = HgRow<NRHS>;
+	const int k = threadIdx.x % NRHS;
+	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+	const int64_t step = ((int64_t(gridDim.x) * blockDim.x) >> 5) * Row::RPW;
+	double acc = 0.0;
+	for (int64_t i = warp * Row::RPW + Row::sub(); __any_sync(0xffffffffu, i < n); i += step) {
+		Row row;
+		row.load(indices, values, Row::at(offsets, i < n ? i : -1));
+		const double p = row.product(x, [] {});
+		if (i < n && Row::lead()) {
+			y[i * NRHS + k] = p;
+			acc += p * x[i * NRHS + k];
+		}
+	}
+	hg_block_partials<NRHS>(acc, partials);
 }
 
 // Device-side CG state of one right-hand side.
@@ -207,31 +377,33 @@ __global__ void k_hpcg_axpby(double *out, const double *a, const double *b, cons
 	}
 }
 
-// x += alpha p; r += -alpha Ap (eWiseMul with the ring, hpcg.hpp:206-207)
+// x += alpha p; r += -alpha Ap (eWiseMul with the ring, hpcg.hpp:206-207), and
+// the partials of r . r
 template <int NRHS>
-__global__ void k_hpcg_update(double *x, double *r, const double *p, const double *ap,
-	const HgScalars *sc, int64_t n) {
+__global__ void __launch_bounds__(HG_BLOCK)
+k_hpcg_update(double *x, double *r, const double *p, const double *ap,
+	const HgScalars *sc, int64_t n, double *partials) {
+	double acc = 0.0;
 	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n * NRHS;
 		 i += int64_t(gridDim.x) * blockDim.x) {
 		const int k = int(i % NRHS);
-		if (!sc[k].active) continue;
-		const double al = sc[k].alpha;
-		x[i] = x[i] + al * p[i];
-		r[i] = r[i] + (-al) * ap[i];
+		double ri = r[i];
+		if (sc[k].active) {
+			const double al = sc[k].alpha;
+			x[i] = x[i] + al * p[i];
+			ri = ri + (-al) * ap[i];
+			r[i] = ri;
+		}
+		acc += ri * ri;
 	}
+	hg_block_partials<NRHS>(acc, partials);
 }
 
-// Scalar steps, one thread per right-hand side.  step 0: after r.r of the
-// initial residual; 1: after r.z; 2: after p.Ap; 3: after the new r.r.
-template <int NRHS>
-__global__ void k_hpcg_scalars(HgScalars *sc, const double *dot, int step, int64_t iter,
+__device__ __forceinline__ void hg_scalar_step(HgScalars &s, double dot, int step, int64_t iter,
 	int64_t max_iter, double tol) {
-	const int k = threadIdx.x;
-	if (k >= NRHS) return;
-	HgScalars &s = sc[k];
 	switch (step) {
 	case 0:
-		s.norm0 = sqrt(dot[k]);
+		s.norm0 = sqrt(dot);
 		s.norm = s.norm0;
 		s.iterations = 0;
 		s.active = 1;
@@ -240,21 +412,50 @@ __global__ void k_hpcg_scalars(HgScalars *sc, const double *dot, int step, int64
 	case 1:
 		if (!s.active) return;
 		s.rz_old = s.rz;
-		s.rz = dot[k];
+		s.rz = dot;
 		s.beta = iter == 0 ? 0.0 : s.rz / s.rz_old;
 		break;
 	case 2:
 		if (!s.active) return;
-		s.pap = dot[k];
+		s.pap = dot;
 		s.alpha = s.rz / s.pap;
 		break;
 	case 3:
 		if (!s.active) return;
-		s.norm = sqrt(dot[k]);
+		s.norm = sqrt(dot);
 		s.iterations = iter + 1;
 		// do { ... } while( iter < max && norm / norm0 > tol )  (hpcg.hpp:209)
 		if (!(s.iterations < max_iter && s.norm / s.norm0 > tol)) s.active = 0;
 		break;
+	}
+}
+
+// The block partials summed in a fixed order (thread t: right-hand side
+// t % NRHS, blocks t / NRHS, + HG_BLOCK / NRHS, ..., then a tree), then the
+// scalar step, one thread per right-hand side.  step 0: after r.r of the
+// initial residual; 1: after r.z; 2: after p.Ap; 3: after the new r.r.
+// *active: the right-hand sides still iterating.
+template <int NRHS>
+__global__ void __launch_bounds__(HG_BLOCK)
+k_hpcg_finish(HgScalars *sc, const double *partials, int nblocks, int step, int64_t iter,
+	int64_t max_iter, double tol, int32_t *active) {
+	__shared__ double dot[HG_BLOCK];
+	if (step != 0 && *active == 0) return;   // uniform: only this kernel's end writes it
+	double v = 0.0;
+	for (int b = threadIdx.x / NRHS; b < nblocks; b += HG_BLOCK / NRHS)
+		v += partials[b * NRHS + threadIdx.x % NRHS];
+	dot[threadIdx.x] = v;
+	__syncthreads();
+	for (int w = HG_BLOCK / 2; w >= NRHS; w >>= 1) {
+		if (threadIdx.x < w) dot[threadIdx.x] += dot[threadIdx.x + w];
+		__syncthreads();
+	}
+	const int k = threadIdx.x;
+	if (k < NRHS) {
+		const bool was = step == 0 || sc[k].active;
+		hg_scalar_step(sc[k], dot[k], step, iter, max_iter, tol);
+		if (step == 0) atomicAdd(active, 1);
+		else if (was && !sc[k].active) atomicSub(active, 1);
 	}
 }
 
@@ -352,72 +553,113 @@ struct alpb_hpcg_s {
 	int64_t colors = 27;
 	double diag = 26.0;
 	double *p = nullptr, *ap = nullptr;  // CG vectors of the finest level
-	double *partials = nullptr, *dots = nullptr;
+	double *partials = nullptr;
 	HgScalars *scalars = nullptr;
+	GridSync *gs = nullptr;      // the cycle kernel's barrier
+	int32_t *active = nullptr;   // right-hand sides still iterating
 	int dot_blocks = 0;
 };
 
 namespace alpb {
 
-template <int NRHS, class Op>
-static int hg_rows(const HgLevel &L, const double *x, int64_t count, const Op &op, cudaStream_t s) {
-	if (count <= 0) return ALPB_SUCCESS;
-	k_hpcg_rows<NRHS, Op><<<grid_for(count * HG_GROUP, HG_BLOCK), HG_BLOCK, 0, s>>>(L.offsets,
-		L.indices, L.values, x, count, op);
-	ALPB_LAUNCHED();
-	return ALPB_SUCCESS;
-}
+// Levels of up to this many values (rows times right-hand sides) run in one
+// cluster of blocks.  Measured us per iteration, levels above / below the line
+// in the cluster: 32^3 with 8 right-hand sides 971 / 1334, with 1 652 / 609;
+// 64^3 with 8 1593 / 1988, with 1 1044 / 1002 (a line at 32,768 values takes
+// the better one of each).
+constexpr int64_t HG_CLUSTER_VALUES = 32768;
 
-// red_black_gauss_seidel: colours forward, then backward (:96-117)
-template <int NRHS>
-static int hg_smoother(alpb_hpcg_s *h, HgLevel &L, cudaStream_t s) {
-	const int64_t K = h->colors;
-	for (int pass = 0; pass < 2; ++pass)
-		for (int64_t q = 0; q < K; ++q) {
-			const int64_t c = pass == 0 ? q : K - 1 - q;
-			const int64_t count = c < L.n ? (L.n - 1 - c) / K + 1 : 0;
-			HgColor<NRHS> op{L.r, L.z, L.fused ? nullptr : L.temp, h->diag, c, K};
-			int rc = hg_rows<NRHS>(L, L.z, count, op, s);
-			if (rc != ALPB_SUCCESS) return rc;
-			if (!L.fused && count > 0) {
-				k_hpcg_color_update<NRHS><<<grid_for(count * NRHS, 256), 256, 0, s>>>(L.r, L.temp,
-					L.z, h->diag, c, K, count);
-				ALPB_LAUNCHED();
-			}
+// one launch of the cycle kernel over the levels [l0, l1)
+template <int NRHS, bool CLUSTER>
+static int hg_cycle_part(alpb_hpcg_s *h, HgCycleArgs &a, int l0, int l1, int part,
+	cudaStream_t s) {
+	a.l0 = l0;
+	a.l1 = l1;
+	a.part = part;
+	cudaLaunchConfig_t cfg = {};
+	cfg.blockDim = dim3(HGC_THREADS);
+	cfg.stream = s;
+	cudaLaunchAttribute attr[1];
+	if (CLUSTER) {
+		static std::atomic<bool> ready[64];
+		int dev = 0;
+		ALPB_CUDA(cudaGetDevice(&dev));
+		if (dev >= 64 || !ready[dev].load()) {
+			ALPB_CUDA(cudaFuncSetAttribute(k_hpcg_cycle<NRHS, CLUSTER>,
+				cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+			if (dev < 64) ready[dev].store(true);
 		}
+		cfg.gridDim = dim3(HGC_CLUSTER);
+		attr[0].id = cudaLaunchAttributeClusterDimension;
+		attr[0].val.clusterDim.x = HGC_CLUSTER;
+		attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+	} else {
+		ALPB_CUDA(cudaMemsetAsync(&h->gs->count, 0, sizeof(h->gs->count), s));
+		cfg.gridDim = dim3(sm_count());
+		attr[0].id = cudaLaunchAttributeCooperative;
+		attr[0].val.cooperative = 1;
+	}
+	cfg.attrs = attr;
+	cfg.numAttrs = 1;
+	ALPB_CUDA(cudaLaunchKernelEx(&cfg, k_hpcg_cycle<NRHS, CLUSTER>, a));
+	ALPB_LAUNCHED();
 	return ALPB_SUCCESS;
 }
 
-// multi_grid (multigrid_v_cycle.hpp:193-246): z = 0; smooth; restrict the
-// residual; recurse; prolong; smooth.  The coarsest level smooths once.
+// one V-cycle from the finest r into the finest z
 template <int NRHS>
-static int hg_vcycle(alpb_hpcg_s *h, size_t l, int64_t pre, int64_t post, cudaStream_t s) {
-	HgLevel &L = h->levels[l];
-	ALPB_CUDA(cudaMemsetAsync(L.z, 0, size_t(L.n) * NRHS * 8, s));
+static int hg_vcycle(alpb_hpcg_s *h, int64_t pre, int64_t post, cudaStream_t s) {
+	HgCycleArgs a;
+	const int nl = int(h->levels.size());
+	int coarse = nl;   // first level of the cluster launch
+	for (int l = nl - 1; l >= 0; --l) {
+		const HgLevel &L = h->levels[size_t(l)];
+		a.lv[l] = HgLevelArgs{L.offsets, L.indices, L.values, L.r, L.z, L.fused ? nullptr : L.temp,
+			L.n, L.nx, L.ny};
+		if (L.n * NRHS <= HG_CLUSTER_VALUES) coarse = l;
+	}
+	a.colors = h->colors;
+	a.pre = pre;
+	a.post = post;
+	a.diag = h->diag;
+	a.gs = h->gs;
+	a.active = h->active;
+	if (coarse == nl) return hg_cycle_part<NRHS, false>(h, a, 0, nl, HG_WHOLE, s);
 	int rc = ALPB_SUCCESS;
-	if (l + 1 == h->levels.size()) return hg_smoother<NRHS>(h, L, s);
-	for (int64_t i = 0; i < pre && rc == ALPB_SUCCESS; ++i) rc = hg_smoother<NRHS>(h, L, s);
-	if (rc != ALPB_SUCCESS) return rc;
-	HgLevel &Cl = h->levels[l + 1];
-	const HgInject inj{Cl.nx, Cl.ny, L.nx, L.ny};
-	rc = hg_rows<NRHS>(L, L.z, Cl.n, HgRestrict<NRHS>{L.r, Cl.r, inj}, s);
-	if (rc != ALPB_SUCCESS) return rc;
-	rc = hg_vcycle<NRHS>(h, l + 1, pre, post, s);
-	if (rc != ALPB_SUCCESS) return rc;
-	k_hpcg_prolong<NRHS><<<grid_for(Cl.n * NRHS, 256), 256, 0, s>>>(L.z, Cl.z, inj, Cl.n);
-	ALPB_LAUNCHED();
-	for (int64_t i = 0; i < post && rc == ALPB_SUCCESS; ++i) rc = hg_smoother<NRHS>(h, L, s);
+	if (coarse > 0) rc = hg_cycle_part<NRHS, false>(h, a, 0, coarse, HG_DOWN, s);
+	rc = rc ? rc : hg_cycle_part<NRHS, true>(h, a, coarse, nl, HG_WHOLE, s);
+	if (coarse > 0) rc = rc ? rc : hg_cycle_part<NRHS, false>(h, a, 0, coarse, HG_UP, s);
 	return rc;
 }
 
 template <int NRHS>
-static int hg_dot(alpb_hpcg_s *h, const double *x, const double *y, int64_t n, cudaStream_t s) {
-	k_hpcg_dot<NRHS><<<h->dot_blocks, HG_BLOCK, 0, s>>>(x, y, n, h->partials);
-	ALPB_LAUNCHED();
-	k_hpcg_dot_finish<NRHS><<<1, 32, 0, s>>>(h->partials, h->dot_blocks, h->dots);
+static int hg_finish(alpb_hpcg_s *h, int step, int64_t iter, int64_t max_iter, double tol,
+	cudaStream_t s) {
+	k_hpcg_finish<NRHS><<<1, HG_BLOCK, 0, s>>>(h->scalars, h->partials, h->dot_blocks, step, iter,
+		max_iter, tol, h->active);
 	ALPB_LAUNCHED();
 	return ALPB_SUCCESS;
 }
+
+template <int NRHS>
+static int hg_spmm(alpb_hpcg_s *h, const double *x, cudaStream_t s) {
+	const HgLevel &L = h->levels[0];
+	k_hpcg_spmm<NRHS><<<h->dot_blocks, HG_BLOCK, 0, s>>>(L.offsets, L.indices, L.values, x, h->ap,
+		L.n, h->partials);
+	ALPB_LAUNCHED();
+	return ALPB_SUCCESS;
+}
+
+template <int NRHS>
+static int hg_dot(alpb_hpcg_s *h, const double *x, const double *y, cudaStream_t s) {
+	k_hpcg_dot<NRHS><<<h->dot_blocks, HG_BLOCK, 0, s>>>(x, y, h->levels[0].n, h->partials);
+	ALPB_LAUNCHED();
+	return ALPB_SUCCESS;
+}
+
+// Iterations queued before the host looks whether any right-hand side is left
+// (the kernels of an iteration too many find none and return).
+constexpr int64_t HG_QUEUE = 4;
 
 // algorithms::hpcg (hpcg.hpp:97-223) for NRHS right-hand sides at once
 template <int NRHS>
@@ -427,27 +669,30 @@ static int hg_solve(alpb_hpcg_s *h, const double *b, double *x, bool preconditio
 	HgLevel &L = h->levels[0];
 	const int64_t n = L.n;
 	const unsigned g = grid_for(n * NRHS, 256);
+	ALPB_CUDA(cudaMemsetAsync(h->gs, 0, sizeof(GridSync), s));
+	ALPB_CUDA(cudaMemsetAsync(h->active, 0, 4, s));
 	// Ap = 0; r = 0; p = x; Ap = A x; r = b - Ap; norm = sqrt(r.r)
 	ALPB_CUDA(cudaMemcpyAsync(h->p, x, size_t(n) * NRHS * 8, cudaMemcpyDeviceToDevice, s));
-	int rc = hg_rows<NRHS>(L, x, n, HgSpmm<NRHS>{h->ap}, s);
+	int rc = hg_spmm<NRHS>(h, x, s);
 	if (rc != ALPB_SUCCESS) return rc;
 	k_hpcg_axpby<NRHS><<<g, 256, 0, s>>>(L.r, h->ap, b, h->scalars, 0, n);
 	ALPB_LAUNCHED();
-	hg_dot<NRHS>(h, L.r, L.r, n, s);
-	k_hpcg_scalars<NRHS><<<1, 32, 0, s>>>(h->scalars, h->dots, 0, 0, max_iter, tol);
-	ALPB_LAUNCHED();
+	rc = hg_dot<NRHS>(h, L.r, L.r, s);
+	rc = rc ? rc : hg_finish<NRHS>(h, 0, 0, max_iter, tol, s);
+	if (rc != ALPB_SUCCESS) return rc;
 	HgScalars hs[NRHS];
+	GridSync hgs;
 	for (int64_t iter = 0;; ++iter) {
 		if (precondition) {
-			rc = hg_vcycle<NRHS>(h, 0, pre, post, s);
+			rc = hg_vcycle<NRHS>(h, pre, post, s);
 			if (rc != ALPB_SUCCESS) return rc;
 		} else {
 			ALPB_CUDA(cudaMemcpyAsync(L.z, L.r, size_t(n) * NRHS * 8, cudaMemcpyDeviceToDevice, s));
 		}
 		// r.z, beta; p = z (first iteration) or p = beta p + z
-		hg_dot<NRHS>(h, L.r, L.z, n, s);
-		k_hpcg_scalars<NRHS><<<1, 32, 0, s>>>(h->scalars, h->dots, 1, iter, max_iter, tol);
-		ALPB_LAUNCHED();
+		rc = hg_dot<NRHS>(h, L.r, L.z, s);
+		rc = rc ? rc : hg_finish<NRHS>(h, 1, iter, max_iter, tol, s);
+		if (rc != ALPB_SUCCESS) return rc;
 		if (iter == 0) {
 			ALPB_CUDA(cudaMemcpyAsync(h->p, L.z, size_t(n) * NRHS * 8, cudaMemcpyDeviceToDevice, s));
 		} else {
@@ -459,18 +704,19 @@ static int hg_solve(alpb_hpcg_s *h, const double *b, double *x, bool preconditio
 			h->ap = t;
 		}
 		// Ap = A p; alpha = r.z / p.Ap; x += alpha p; r -= alpha Ap; norm
-		rc = hg_rows<NRHS>(L, h->p, n, HgSpmm<NRHS>{h->ap}, s);
+		rc = hg_spmm<NRHS>(h, h->p, s);
+		rc = rc ? rc : hg_finish<NRHS>(h, 2, iter, max_iter, tol, s);
 		if (rc != ALPB_SUCCESS) return rc;
-		hg_dot<NRHS>(h, h->ap, h->p, n, s);
-		k_hpcg_scalars<NRHS><<<1, 32, 0, s>>>(h->scalars, h->dots, 2, iter, max_iter, tol);
+		k_hpcg_update<NRHS><<<h->dot_blocks, HG_BLOCK, 0, s>>>(x, L.r, h->p, h->ap, h->scalars, n,
+			h->partials);
 		ALPB_LAUNCHED();
-		k_hpcg_update<NRHS><<<g, 256, 0, s>>>(x, L.r, h->p, h->ap, h->scalars, n);
-		ALPB_LAUNCHED();
-		hg_dot<NRHS>(h, L.r, L.r, n, s);
-		k_hpcg_scalars<NRHS><<<1, 32, 0, s>>>(h->scalars, h->dots, 3, iter, max_iter, tol);
-		ALPB_LAUNCHED();
+		rc = hg_finish<NRHS>(h, 3, iter, max_iter, tol, s);
+		if (rc != ALPB_SUCCESS) return rc;
+		if (iter % HG_QUEUE != HG_QUEUE - 1 && iter + 1 < max_iter) continue;
 		ALPB_CUDA(cudaMemcpyAsync(hs, h->scalars, sizeof(hs), cudaMemcpyDeviceToHost, s));
+		ALPB_CUDA(cudaMemcpyAsync(&hgs, h->gs, sizeof(hgs), cudaMemcpyDeviceToHost, s));
 		ALPB_CUDA(cudaStreamSynchronize(s));
+		ALPB_CHECK(hgs.err == 0, ALPB_PANIC, "alpb_hpcg_solve: a grid barrier timed out");
 		bool any = false;
 		for (int k = 0; k < NRHS; ++k) any = any || hs[k].active;
 		if (!any) break;
@@ -499,7 +745,8 @@ int alpb_hpcg_destroy(alpb_hpcg h) {
 	cudaFree(h->p);
 	cudaFree(h->ap);
 	cudaFree(h->partials);
-	cudaFree(h->dots);
+	cudaFree(h->gs);
+	cudaFree(h->active);
 	cudaFree(h->scalars);
 	delete h;
 	return ALPB_SUCCESS;
@@ -600,11 +847,12 @@ int alpb_hpcg_create(alpb_hpcg *out, int64_t nx, int64_t ny, int64_t nz, double 
 	cudaFreeAsync(flag, s);
 	const int64_t n0 = h->levels[0].n;
 	if (rc == ALPB_SUCCESS) {
-		h->dot_blocks = int(grid_for(n0 * nrhs, HG_BLOCK, 2));
+		h->dot_blocks = int(grid_for(n0 * nrhs, HG_BLOCK, 8));
 		if (cudaMalloc(&h->p, size_t(n0) * nrhs * 8) != cudaSuccess ||
 			cudaMalloc(&h->ap, size_t(n0) * nrhs * 8) != cudaSuccess ||
 			cudaMalloc(&h->partials, size_t(h->dot_blocks) * nrhs * 8) != cudaSuccess ||
-			cudaMalloc(&h->dots, size_t(nrhs) * 8) != cudaSuccess ||
+			cudaMalloc(&h->gs, sizeof(GridSync)) != cudaSuccess ||
+			cudaMalloc(&h->active, 4) != cudaSuccess ||
 			cudaMalloc(&h->scalars, size_t(nrhs) * sizeof(HgScalars)) != cudaSuccess) {
 			cudaGetLastError();
 			rc = ALPB_OUTOFMEM;
