@@ -25,6 +25,7 @@ struct PrState {
 	GridSync gs;
 	int64_t iterations;
 	double residual;
+	int zero_values;   // a stored value of the CRS is zero
 };
 
 struct PrArgs {
@@ -81,6 +82,56 @@ struct PrEpi {
 	}
 };
 
+// *zero = 1 where a stored value is zero: without one, a row's out-degree is
+// its length, and the set-up need not walk the rows (a hub row of 1e5 entries
+// on one warp took most of its 320 us on a graph of a million rows; this
+// streaming pass takes about 20)
+__global__ void __launch_bounds__(256) k_pr_zero_values(const double *__restrict__ val,
+	const int64_t *__restrict__ ptr, int64_t n, int *zero) {
+	const int64_t nnz = ptr[n];
+	bool z = false;
+	for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < nnz;
+		 k += int64_t(gridDim.x) * blockDim.x)
+		z |= __ldcs(val + k) == 0.0;
+	if (__any_sync(0xffffffffu, z) && (threadIdx.x & 31) == 0) *zero = 1;
+}
+
+// Row i of the set-up (:224-289 and the initial guess): its scale alpha /
+// count, pr, the pre-scaled first input; returns its dangling mass.
+template <class Args>
+__device__ __forceinline__ double pr_setup_row(const Args &a, int64_t i, double cnt) {
+	const double rsi = cnt > 0.0 ? a.alpha / cnt : 0.0;
+	a.rs[i] = rsi;
+	const double p = a.init_given ? a.pr[i] : 1.0 / double(a.n);
+	a.pr[i] = p;
+	a.next0[i] = rsi == 0.0 ? 0.0 : p * rsi;
+	return rsi == 0.0 ? p : 0.0;
+}
+
+// The set-up's rows of this block; the thread's share of the dangling mass.
+// zero: some stored value is zero, so the out-degrees are counted (one warp
+// per row); otherwise they are the row lengths (one thread per row).
+template <class Args>
+__device__ __forceinline__ double pr_setup_rows(const Args &a, bool zero) {
+	double dang = 0.0;
+	const int64_t tid = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+	const int64_t nt = int64_t(gridDim.x) * blockDim.x;
+	if (!zero) {
+		for (int64_t i = tid; i < a.n; i += nt)
+			dang += pr_setup_row(a, i, double(a.crs_ptr[i + 1] - a.crs_ptr[i]));
+		return dang;
+	}
+	const int lane = threadIdx.x & 31;
+	for (int64_t i = tid >> 5; i < a.n; i += nt >> 5) {
+		const int64_t b = a.crs_ptr[i], e = a.crs_ptr[i + 1];
+		double cnt = 0.0;
+		for (int64_t k = b + lane; k < e; k += 32) cnt += a.crs_val[k] != 0.0 ? 1.0 : 0.0;
+		for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+		if (lane == 0) dang += pr_setup_row(a, i, cnt);
+	}
+	return dang;
+}
+
 struct GatherL2 {
 	const double *x;
 	__device__ __forceinline__ double operator()(uint32_t j) const { return __ldcg(x + j); }
@@ -95,34 +146,14 @@ __global__ void __launch_bounds__(32 * PR_WARPS, 6) k_pagerank(PrArgs a) {
 	PrState *st = a.st;
 	int *err = &st->gs.err;
 	const int64_t G = gridDim.x, n = a.n, nt = a.mt.ntiles;
-	const int lane = threadIdx.x & 31;
 	const int w = threadIdx.x >> 5;
 	const int64_t gw = int64_t(blockIdx.x) * PR_WARPS + w, nw = G * PR_WARPS;
 	// setup: out-degree counts of nonzero-valued entries (the pattern ring of
 	// :224-237), alpha / count (:281-289), initial guess, pre-scaled input
-	double dang = 0.0;
 	for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < nt;
 		 t += G * blockDim.x)
 		a.mt.ready[t] = 0;
-	for (int64_t i = gw; i < n; i += nw) {
-		const int64_t b = a.crs_ptr[i], e = a.crs_ptr[i + 1];
-		double cnt = 0.0;
-		for (int64_t k = b + lane; k < e; k += 32)
-			cnt += (a.crs_val == nullptr || a.crs_val[k] != 0.0) ? 1.0 : 0.0;
-		for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-		if (lane == 0) {
-			const double rsi = cnt > 0.0 ? a.alpha / cnt : 0.0;
-			a.rs[i] = rsi;
-			const double p = a.init_given ? a.pr[i] : 1.0 / double(n);
-			a.pr[i] = p;
-			if (rsi == 0.0) {
-				a.next0[i] = 0.0;
-				dang += p;
-			} else {
-				a.next0[i] = p * rsi;
-			}
-		}
-	}
+	double dang = pr_setup_rows(a, st->zero_values != 0);
 	dang = block_sum(dang, red);
 	if (threadIdx.x == 0) a.blk[blockIdx.x] = dang;
 	if (!grid_sync(&st->gs)) return;
@@ -173,11 +204,11 @@ __global__ void __launch_bounds__(32 * PR_WARPS, 6) k_pagerank(PrArgs a) {
 // ------------------------------------------------ large graphs: per-step --
 // For large graphs one cooperative kernel is the wrong shape: its columns
 // that cross warp tiles wait on each other in tile order, and its grid is
-// capped at what stays co-resident.  There every iteration is instead three
-// ordinary launches -- the product over the CCS with the same row epilogue
-// (k_pr_step; a column that crosses tiles leaves per-tile partials), the
-// crossing columns' epilogue (k_pr_fix), and one block that sums the block
-// partials in a fixed order and decides whether to stop (k_pr_finish).
+// capped at what stays co-resident.  There every iteration is instead
+// two ordinary launches -- the product over the CCS with the same row epilogue
+// (k_pr_step; a column that crosses tiles leaves per-tile partials), and the
+// crossing columns' epilogue (k_pr_fix), whose last block sums the block
+// partials in a fixed order and decides whether to stop.
 // Iterations are queued in chunks; once the stop is decided every queued
 // kernel returns at once, and the host reads the state once per chunk.
 constexpr int PRS_WARPS = 4;
@@ -187,6 +218,8 @@ struct PrStepState {
 	int64_t iterations;
 	double residual, d;
 	int done;
+	int zero_values;          // a stored value of the CRS is zero
+	unsigned int arrived;     // blocks of k_pr_fix that left their partials
 };
 
 struct PrStepArgs {
@@ -206,10 +239,20 @@ struct PrStepArgs {
 	PrStepState *st;
 };
 
-// the row epilogue of both kernels (old pr and the row scale read directly)
+// Shared memory of a warp of k_pr_step: the compact tile, whose y entries hold
+// the rows' old pr, and the scales of the tile's first PRS_RS rows (the others
+// are read where they are needed).  3.2 KB instead of 7.2: what is left of the
+// SM's memory holds the L1 lines of the gathers in flight.
+constexpr int PRS_RS = 64;
+struct PrsWarpSmem {
+	WarpSmemCompact<RF> tile;
+	double rs[PRS_RS];
+};
+
+// the row epilogue (old pr and the row scale fetched with the tile)
 struct PrStepEpi {
 	const PrStepArgs *a;
-	PrWarpSmem *sm;                // null: no per-tile prefetch (the crossing columns)
+	PrsWarpSmem *sm;
 	double *next_out;
 	double d;
 	int64_t base = 0;
@@ -217,17 +260,18 @@ struct PrStepEpi {
 	__device__ __forceinline__ void begin_tile(int64_t i0, int nrows, int lane) {
 		base = i0;
 		for (int k = lane; k < nrows; k += 32) {
-			sm->old_pr[k] = a->pr[i0 + k];
-			sm->rs[k] = __ldg(a->rs + i0 + k);
+			sm->tile.y(k) = a->pr[i0 + k];
+			if (k < PRS_RS) sm->rs[k] = __ldg(a->rs + i0 + k);
 		}
 	}
 	__device__ __forceinline__ void row(int64_t j, double v, bool has) {
 		const double nn = has ? 0.0 + v : 0.0;       // pr_nextnext = 0; += pr_next L
-		const double old = sm ? sm->old_pr[j - base] : a->pr[j];
+		const int q = int(j - base);
+		const double old = sm->tile.y(q);
 		const double nw = nn + d;                    // pr = pr_nextnext + dangling
 		a->pr[j] = nw;
 		acc_res += old > nw ? old - nw : nw - old;
-		const double rsj = sm ? sm->rs[j - base] : a->rs[j];
+		const double rsj = q < PRS_RS ? sm->rs[q] : __ldg(a->rs + j);
 		if (rsj == 0.0) {                            // input of the next iteration
 			next_out[j] = 0.0;
 			acc_dang += nw;
@@ -242,43 +286,21 @@ struct GatherRO {
 	__device__ __forceinline__ double operator()(uint32_t j) const { return __ldg(x + j); }
 };
 
-// set-up (:224-289 and the initial guess): row scales, pr, the pre-scaled
-// first input and the blocks' dangling mass
+// set-up of the per-step solve: the rows, and the blocks' dangling mass
 __global__ void __launch_bounds__(256) k_pr_setup(PrStepArgs a) {
 	__shared__ double red[33];
-	const int lane = threadIdx.x & 31;
-	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
-	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-	double dang = 0.0;
-	for (int64_t i = warp; i < a.n; i += nwarps) {
-		const int64_t b = a.crs_ptr[i], e = a.crs_ptr[i + 1];
-		double cnt = 0.0;
-		for (int64_t k = b + lane; k < e; k += 32)
-			cnt += (a.crs_val == nullptr || a.crs_val[k] != 0.0) ? 1.0 : 0.0;
-		for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-		if (lane == 0) {
-			const double rsi = cnt > 0.0 ? a.alpha / cnt : 0.0;
-			a.rs[i] = rsi;
-			const double p = a.init_given ? a.pr[i] : 1.0 / double(a.n);
-			a.pr[i] = p;
-			if (rsi == 0.0) {
-				a.next0[i] = 0.0;
-				dang += p;
-			} else {
-				a.next0[i] = p * rsi;
-			}
-		}
-	}
-	dang = block_sum(dang, red);
+	const double dang = block_sum(pr_setup_rows(a, a.st->zero_values != 0), red);
 	if (threadIdx.x == 0) {
 		a.blk[blockIdx.x] = 0.0;
 		a.blk[a.grid + blockIdx.x] = dang;
 	}
 }
 
+// Six blocks of four warps per SM: with 5 / 7 / 8 of them 118 / 121 / 139 us per
+// iteration instead of 113 (R-MAT, 1,000,003 vertices; 124 with 7.2 KB a warp).
 __global__ void __launch_bounds__(32 * PRS_WARPS, 6) k_pr_step(PrStepArgs a, int parity) {
 	if (a.st->done) return;
-	__shared__ PrWarpSmem sm[PRS_WARPS];
+	__shared__ PrsWarpSmem sm[PRS_WARPS];
 	__shared__ double red[33];
 	const int w = threadIdx.x >> 5;
 	PrStepEpi epi{&a, &sm[w], parity ? a.next0 : a.next1, a.st->d};
@@ -288,7 +310,7 @@ __global__ void __launch_bounds__(32 * PRS_WARPS, 6) k_pr_step(PrStepArgs a, int
 	WmMeta g = wm_meta(a.mt, t);
 	while (t < a.mt.ntiles) {
 		const WmMeta next = wm_meta(a.mt, t + nw);
-		warp_tile<RF>(t, g, a.mt, a.ccs_ptr, a.ccs_row, a.ccs_val, xl, epi, 0, sm[w].tile);
+		warp_tile<RF, GatherRO, PrStepEpi, WarpSmemCompact<RF>, WM_LOADS_FIRST>(t, g, a.mt, a.ccs_ptr, a.ccs_row, a.ccs_val, xl, epi, 0, sm[w].tile);
 		t += nw;
 		g = next;
 	}
@@ -297,46 +319,6 @@ __global__ void __launch_bounds__(32 * PRS_WARPS, 6) k_pr_step(PrStepArgs a, int
 	if (threadIdx.x == 0) {
 		a.blk[blockIdx.x] = s1;
 		a.blk[a.grid + blockIdx.x] = s2;
-	}
-}
-
-// columns that cross tiles: their partials summed in tile order (tail slots
-// of the first..last-1 tiles, head slot of the last), then the epilogue
-__global__ void __launch_bounds__(256) k_pr_fix(PrStepArgs a, int parity) {
-	if (a.st->done) return;
-	__shared__ double red[33];
-	const MergeTables &mt = a.mt;
-	PrStepEpi epi{&a, nullptr, parity ? a.next0 : a.next1, a.st->d};
-	const int lane = threadIdx.x & 31;
-	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
-	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-	for (int64_t base = warp * 32; base < mt.ntiles; base += nwarps * 32) {
-		const int64_t t = base + lane;
-		const int32_t n = t < mt.ntiles ? mt.span_len[t] : 0;
-		if (n > 0 && n <= 32) {
-			double v = wm_sum_slots<RF>(0.0, mt.tail_val, t, t + n - 1);
-			v += load_bits<double>(mt.head_val + t + n - 1);
-			epi.row(mt.tile_row[t + 1], v, true);
-		}
-		unsigned long_rows = __ballot_sync(0xffffffffu, n > 32);
-		while (long_rows) {
-			const int src = __ffs(long_rows) - 1;
-			long_rows &= long_rows - 1;
-			const int64_t f = base + src;
-			const int32_t nn = __shfl_sync(0xffffffffu, n, src);
-			double v = wm_sum_slots32<RF>(0.0, mt.tail_val, f + lane, f + nn - 1);
-			for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-			if (lane == 0) {
-				v += load_bits<double>(mt.head_val + f + nn - 1);
-				epi.row(mt.tile_row[f + 1], v, true);
-			}
-		}
-	}
-	const double s1 = block_sum(epi.acc_res, red);
-	const double s2 = block_sum(epi.acc_dang, red);
-	if (threadIdx.x == 0) {
-		a.fix[blockIdx.x] = s1;
-		a.fix[a.fix_grid + blockIdx.x] = s2;
 	}
 }
 
@@ -351,13 +333,13 @@ __device__ __forceinline__ void pr_finish_sums(const PrStepArgs &a, int setup,
 	double (*smem)[33], double out[4]) {
 	double v[4] = {0.0, 0.0, 0.0, 0.0};
 	for (int64_t k = threadIdx.x; k < a.grid; k += blockDim.x) {
-		v[0] += a.blk[k];
-		v[1] += a.blk[a.grid + k];
+		v[0] += __ldcg(a.blk + k);
+		v[1] += __ldcg(a.blk + a.grid + k);
 	}
 	if (!setup)
 		for (int64_t k = threadIdx.x; k < a.fix_grid; k += blockDim.x) {
-			v[2] += a.fix[k];
-			v[3] += a.fix[a.fix_grid + k];
+			v[2] += __ldcg(a.fix + k);
+			v[3] += __ldcg(a.fix + a.fix_grid + k);
 		}
 	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
@@ -379,25 +361,90 @@ __device__ __forceinline__ void pr_finish_sums(const PrStepArgs &a, int setup,
 	for (int q = 0; q < 4; ++q) out[q] = smem[q][32];
 }
 
-__global__ void __launch_bounds__(256) k_pr_finish(PrStepArgs a, int setup) {
+// One block: the sums, the next teleport term, and whether to stop.
+__device__ __forceinline__ void pr_finish(const PrStepArgs &a, int setup) {
 	__shared__ double red[4][33];
 	PrStepState *st = a.st;
-	if (st->done) return;
 	double sums[4];
 	pr_finish_sums(a, setup, red, sums);
-	const double r1 = sums[0], d1 = sums[1];
-	const double r2 = setup ? 0.0 : sums[2];
-	const double d2 = setup ? 0.0 : sums[3];
 	if (threadIdx.x == 0) {
-		const double dang = d1 + d2;
+		const double dang = setup ? sums[1] : sums[1] + sums[3];
 		st->d = (a.alpha * dang + 1 - a.alpha) / double(a.n);     // (:390)
 		if (!setup) {
-			st->residual = r1 + r2;
+			st->residual = sums[0] + sums[2];
 			st->iterations += 1;
 			if ((a.conv != 0.0 && st->residual <= a.conv) || st->iterations >= a.max_iter)
 				st->done = 1;
 		}
 	}
+}
+
+__global__ void __launch_bounds__(256) k_pr_first(PrStepArgs a) { pr_finish(a, 1); }
+
+// columns that cross tiles: their partials summed in tile order (tail slots
+// of the first..last-1 tiles, head slot of the last), then the epilogue.  A
+// lane's column, its old value and scale and its slots are loaded side by
+// side: the chain of dependent loads is what bounds this kernel.  The last
+// block to leave its partials closes the iteration (no launch of its own).
+__global__ void __launch_bounds__(256) k_pr_fix(PrStepArgs a, int parity) {
+	if (a.st->done) return;
+	__shared__ double red[33];
+	__shared__ bool last;
+	const MergeTables &mt = a.mt;
+	double *next_out = parity ? a.next0 : a.next1;
+	const double d = a.st->d;
+	double acc_res = 0.0, acc_dang = 0.0;
+	// the row epilogue of k_pr_step on column j with old value and scale loaded
+	const auto finish = [&](int64_t j, double v, double old, double rsj) {
+		const double nw = (0.0 + v) + d;
+		a.pr[j] = nw;
+		acc_res += old > nw ? old - nw : nw - old;
+		next_out[j] = rsj == 0.0 ? 0.0 : nw * rsj;
+		if (rsj == 0.0) acc_dang += nw;
+	};
+	const int lane = threadIdx.x & 31;
+	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+	for (int64_t base = warp * 32; base < mt.ntiles; base += nwarps * 32) {
+		const int64_t t = base + lane;
+		const int32_t n = t < mt.ntiles ? mt.span_len[t] : 0;
+		const int64_t j = t < mt.ntiles ? mt.tile_row[t + 1] : 0;
+		if (n > 0 && n <= 32) {
+			const double old = a.pr[j], rsj = a.rs[j];
+			const double head = load_bits<double>(mt.head_val + t + n - 1);
+			double v = wm_sum_slots<RF>(0.0, mt.tail_val, t, t + n - 1);
+			v += head;
+			finish(j, v, old, rsj);
+		}
+		unsigned long_rows = __ballot_sync(0xffffffffu, n > 32);
+		while (long_rows) {
+			const int src = __ffs(long_rows) - 1;
+			long_rows &= long_rows - 1;
+			const int64_t f = base + src;
+			const int32_t nn = __shfl_sync(0xffffffffu, n, src);
+			const int64_t jj = __shfl_sync(0xffffffffu, j, src);
+			double v = wm_sum_slots32<RF>(0.0, mt.tail_val, f + lane, f + nn - 1);
+			for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+			if (lane == 0) {
+				v += load_bits<double>(mt.head_val + f + nn - 1);
+				finish(jj, v, a.pr[jj], a.rs[jj]);
+			}
+		}
+	}
+	const double s1 = block_sum(acc_res, red);
+	const double s2 = block_sum(acc_dang, red);
+	if (threadIdx.x == 0) {
+		a.fix[blockIdx.x] = s1;
+		a.fix[a.fix_grid + blockIdx.x] = s2;
+		__threadfence();
+		last = atomicAdd(&a.st->arrived, 1u) == gridDim.x - 1;
+		if (last) {
+			a.st->arrived = 0;
+			__threadfence();
+		}
+	}
+	__syncthreads();
+	if (last) pr_finish(a, 0);
 }
 
 static int pagerank_steps(const PrStepArgs &tmpl, alpb_spmv_plan plan, int64_t *iterations,
@@ -421,9 +468,14 @@ static int pagerank_steps(const PrStepArgs &tmpl, alpb_spmv_plan plan, int64_t *
 	a.blk = part;
 	a.fix = part + 2 * a.grid;
 	a.st = st;
+	if (a.crs_val) {
+		k_pr_zero_values<<<grid_for(plan->nnz, 256), 256, 0, s>>>(a.crs_val, a.crs_ptr, a.n,
+			&st->zero_values);
+		ALPB_LAUNCHED();
+	}
 	k_pr_setup<<<a.grid, 256, 0, s>>>(a);
 	ALPB_LAUNCHED();
-	k_pr_finish<<<1, 256, 0, s>>>(a, 1);
+	k_pr_first<<<1, 256, 0, s>>>(a);
 	ALPB_LAUNCHED();
 	PrStepState h{};
 	int64_t queued = 0;
@@ -434,8 +486,6 @@ static int pagerank_steps(const PrStepArgs &tmpl, alpb_spmv_plan plan, int64_t *
 			k_pr_step<<<a.grid, 32 * PRS_WARPS, 0, s>>>(a, parity);
 			ALPB_LAUNCHED();
 			k_pr_fix<<<a.fix_grid, 256, 0, s>>>(a, parity);
-			ALPB_LAUNCHED();
-			k_pr_finish<<<1, 256, 0, s>>>(a, 0);
 			ALPB_LAUNCHED();
 		}
 		queued += chunk;
@@ -456,8 +506,10 @@ static int pagerank_steps(const PrStepArgs &tmpl, alpb_spmv_plan plan, int64_t *
 	return ALPB_SUCCESS;
 }
 
-// Graphs from this many nonzeroes on take the per-step launches.
-constexpr int64_t kPrStepNnz = int64_t(1) << 23;
+// Graphs from this many nonzeroes on take the per-step launches.  Measured us
+// per solve, one kernel against steps, R-MAT: 0.45 M nonzeroes 361 / 438,
+// 0.9 M 557 / 557, 1.5 M 733 / 644, 4.6 M 1260 / 1020, 15 M 4170 / 2840.
+constexpr int64_t kPrStepNnz = int64_t(1) << 20;
 
 // The solve proper.  plan: a WM_TILE plan of the CCS offsets, or null (one is
 // made and destroyed here); work: 3n doubles of scratch, or null.
@@ -538,6 +590,11 @@ static int pagerank_run(int64_t n, const int64_t *crs_row_ptr, const double *crs
 	a.conv = conv;
 	a.init_given = init_given;
 	a.st = st;
+	if (crs_values) {
+		k_pr_zero_values<<<grid_for(plan->nnz, 256), 256, 0, s>>>(crs_values, crs_row_ptr, n,
+			&st->zero_values);
+		ALPB_LAUNCHED();
+	}
 	void *args[] = {&a};
 	ALPB_CUDA(cudaLaunchCooperativeKernel((void *) k_pagerank, dim3(grid), dim3(32 * PR_WARPS), args,
 		0, s));
