@@ -18,6 +18,7 @@
 #include "spmv.cuh"
 #include "merge.cuh"
 #include "wmerge.cuh"
+#include "rowstream.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -829,6 +830,9 @@ int launch_merge(const SpmvArgs &a, const alpb_spmv_plan_s &p, cudaStream_t s) {
 		k_wm_fixup<R><<<grid_for((p.ntiles + 31) / 32 * 32, 256), 256, 0, s>>>(mt,
 			AccumulateY<R>{reinterpret_cast<T *>(a.u)});
 	} else if (p.tile == WM_TILE) {
+		const T *values = reinterpret_cast<const T *>(a.values), *x = reinterpret_cast<const T *>(a.v);
+		T *u = reinterpret_cast<T *>(a.u);
+		const MergeTables mt = merge_tables(p);
 		static int blocks_per_sm = 0;
 		if (!blocks_per_sm) {
 			ALPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm,
@@ -838,10 +842,8 @@ int launch_merge(const SpmvArgs &a, const alpb_spmv_plan_s &p, cudaStream_t s) {
 		int64_t grid = (p.ntiles + WM_WARPS - 1) / WM_WARPS;
 		const int64_t cap = int64_t(sm_count()) * blocks_per_sm;
 		if (grid > cap) grid = cap;
-		const MergeTables mt = merge_tables(p);
 		k_spmv_wmerge<R, PlainX<T>><<<unsigned(grid), 32 * WM_WARPS, 0, s>>>(mt, a.offsets,
-			a.indices, reinterpret_cast<const T *>(a.values),
-			PlainX<T>{reinterpret_cast<const T *>(a.v)}, reinterpret_cast<T *>(a.u), a.left);
+			a.indices, values, PlainX<T>{x}, u, a.left);
 		ALPB_LAUNCHED();
 		// rows crossing tiles: one lane per 32 tiles' worth of first tiles
 		k_wm_fixup<R><<<grid_for((p.ntiles + 31) / 32 * 32, 256), 256, 0, s>>>(mt,
@@ -921,6 +923,44 @@ int launch_vector(const SpmvArgs &a, const alpb_spmv_plan_s *p, int W, bool dens
 	}
 }
 
+// Row-streaming kernel of one chunk shape; the block takes as many warps as
+// its shared memory holds stages for.
+template <class R, int L, int RPL, int U>
+static int launch_rows_as(const SpmvArgs &a, int maxlen, cudaStream_t s) {
+	using T = typename R::T;
+	constexpr int ROWS = 32 / L * RPL;
+	const int cap = rs_cap<R>(ROWS, maxlen);
+	const size_t warp = size_t(RS_STAGES) * size_t(cap) * (sizeof(T) + 4);
+	constexpr size_t room = 220 * 1024;
+	int warps = int(room / warp);
+	if (warps > RS_MAX_WARPS) warps = RS_MAX_WARPS;
+	static std::atomic<bool> ready[64];
+	int dev = 0;
+	ALPB_CUDA(cudaGetDevice(&dev));
+	if (dev >= 64 || !ready[dev].load()) {
+		ALPB_CUDA(cudaFuncSetAttribute(k_spmv_rows<R, L, RPL, U>,
+			cudaFuncAttributeMaxDynamicSharedMemorySize, int(room)));
+		if (dev < 64) ready[dev].store(true);
+	}
+	const int64_t chunks = (a.m_out + ROWS - 1) / ROWS;
+	const int64_t grid = chunks < sm_count() ? chunks : sm_count();
+	const int64_t per = (chunks + grid - 1) / grid;   // chunks of one block
+	if (per < warps) warps = int(per);
+	k_spmv_rows<R, L, RPL, U><<<unsigned(grid), 32 * warps, warp * warps, s>>>(a.offsets,
+		a.indices, reinterpret_cast<const T *>(a.values), reinterpret_cast<const T *>(a.v),
+		reinterpret_cast<T *>(a.u), a.m_out, a.nnz, cap, a.left);
+	ALPB_LAUNCHED();
+	return ALPB_SUCCESS;
+}
+
+// Rows of up to 8 nonzeroes: one lane a row, two rows a lane (a chunk of 64
+// rows); longer ones: two lanes a row.
+template <class R>
+static int launch_rows(const SpmvArgs &a, int maxlen, cudaStream_t s) {
+	if (maxlen <= 8) return launch_rows_as<R, 1, 2, 5>(a, maxlen, s);
+	return launch_rows_as<R, 2, 1, 7>(a, maxlen, s);
+}
+
 static int default_width(double mean) {
 	int w = 1;
 	while (w < 32 && w * 2 <= mean * 0.75 + 1) w *= 2;
@@ -955,6 +995,11 @@ int run_spmv(const SpmvArgs &a, const alpb_spmv_plan_s *p, int force_sched, cuda
 	int W = p ? p->vw : default_width(a.m_out ? double(a.nnz) / double(a.m_out) : 1.0);
 	if (fast && sched == ALPB_SCHED_MERGE_PATH && p && p->tile_row)
 		return launch_merge<R>(a, *p, s);
+	// regular short rows: the row-streaming kernel (16-byte copies of the
+	// storage's ranges, so its arrays have to start on such a boundary)
+	if (fast && p && p->rows && !(reinterpret_cast<uintptr_t>(a.indices) & 15) &&
+		!(reinterpret_cast<uintptr_t>(a.values) & 15))
+		return launch_rows<R>(a, int(p->maxlen), s);
 	return launch_vector<R>(a, p, W, fast, s);
 }
 
@@ -1099,6 +1144,7 @@ int alpb::plan_create_tiles(alpb_spmv_plan_s **plan, int64_t m, int64_t nnz,
 	}
 	if (sched == ALPB_SCHED_AUTO) sched = regular ? ALPB_SCHED_VECTOR : ALPB_SCHED_MERGE_PATH;
 	p->sched = sched;
+	p->rows = regular && vector_width <= 0 && p->maxlen >= 1 && p->maxlen <= RS_MAX_LEN;
 	*plan = p;
 	return ALPB_SUCCESS;
 }
@@ -1276,21 +1322,28 @@ int alpb_spmv_autotune(alpb_spmv_plan p, int ring, int64_t n, const uint32_t *in
 	ALPB_CUDA(cudaEventCreate(&e0));
 	ALPB_CUDA(cudaEventCreate(&e1));
 	// candidates: merge path, and vector widths around the mean row length
-	struct Cand { int sched, w; } cands[8];
+	struct Cand { int sched, w; bool rows; } cands[8];
 	int nc = 0;
-	cands[nc++] = {ALPB_SCHED_MERGE_PATH, p->vw};
-	for (int w = 2; w <= 32; w *= 2) cands[nc++] = {ALPB_SCHED_VECTOR, w};
+	cands[nc++] = {ALPB_SCHED_MERGE_PATH, p->vw, false};
+	if (p->rows) cands[nc++] = {ALPB_SCHED_VECTOR, p->vw, true};
+	for (int w = 2; w <= 32; w *= 2) cands[nc++] = {ALPB_SCHED_VECTOR, w, false};
 	float best = 1e30f;
 	int best_i = 0;
 	const int saved_vw = p->vw;
+	const bool saved_rows = p->rows;
 	a.offsets = p->offsets;
 	for (int c = 0; c < nc; ++c) {
 		p->vw = cands[c].w;
+		p->rows = cands[c].rows;
 		float total = 0;
 		for (int rep = 0; rep < 4; ++rep) {
 			ALPB_CUDA(cudaEventRecord(e0, s));
 			int rc = dispatch_spmv(ring, a, p, cands[c].sched, s);
-			if (rc != ALPB_SUCCESS) { p->vw = saved_vw; return rc; }
+			if (rc != ALPB_SUCCESS) {
+				p->vw = saved_vw;
+				p->rows = saved_rows;
+				return rc;
+			}
 			ALPB_CUDA(cudaEventRecord(e1, s));
 			ALPB_CUDA(cudaEventSynchronize(e1));
 			float ms = 0;
@@ -1301,6 +1354,7 @@ int alpb_spmv_autotune(alpb_spmv_plan p, int ring, int64_t n, const uint32_t *in
 	}
 	p->sched = cands[best_i].sched;
 	p->vw = cands[best_i].sched == ALPB_SCHED_VECTOR ? cands[best_i].w : saved_vw;
+	p->rows = cands[best_i].rows;
 	// skewed rows on the merge path: try the hot-column cache at four sizes,
 	// up to what the shared memory left by the warps' tiles holds
 	hot_release(p);

@@ -9,6 +9,7 @@ struct alpb_spmv_plan_s {
 	const int64_t *offsets = nullptr;  // storage the plan was made for
 	int sched = ALPB_SCHED_VECTOR;
 	int vw = 8;
+	bool rows = false;   // vector schedule: short regular rows, streamed (rowstream.cuh)
 	int device = 0;
 	int64_t ntiles = 0;
 	int64_t tile = 0;               // merge items per tile of the tables below
