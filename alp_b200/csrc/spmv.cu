@@ -175,6 +175,11 @@ struct AccumulateY {
 	__device__ __forceinline__ void row_span(int64_t, int64_t r, typename R::T v, bool has) {
 		row(r, v, has);
 	}
+	// the same in two halves (k_wm_fixup)
+	__device__ __forceinline__ typename R::T load(int64_t r) const { return y[r]; }
+	__device__ __forceinline__ void finish(int64_t r, typename R::T v, typename R::T old) const {
+		y[r] = R::add(old, v);
+	}
 };
 
 template <class R>

@@ -472,11 +472,15 @@ __global__ void __launch_bounds__(256) k_wm_fixup(MergeTables mt, Epi epi) {
 	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
 	for (int64_t base = warp * 32; base < mt.ntiles; base += nwarps * 32) {
 		const int64_t t = base + lane;
+		// the row, its old value and its slots are loaded side by side (the
+		// chain of dependent loads is what bounds this pass)
 		const int32_t n = t < mt.ntiles ? mt.span_len[t] : 0;
+		const int64_t r = t < mt.ntiles ? mt.tile_row[t + 1] : 0;
 		if (n > 0 && n <= 32) {
+			const auto old = epi.load(r);
+			const T head = wm_load_slot<T>(mt.head_val + t + n - 1);
 			T v = wm_sum_slots<R>(R::zero(), mt.tail_val, t, t + n - 1);
-			v = R::add(v, wm_load_slot<T>(mt.head_val + t + n - 1));
-			epi.row(mt.tile_row[t + 1], v, true);
+			epi.finish(r, R::add(v, head), old);
 		}
 		unsigned long_rows = __ballot_sync(WM_FULL, n > 32);
 		while (long_rows) {
@@ -492,7 +496,8 @@ __global__ void __launch_bounds__(256) k_wm_fixup(MergeTables mt, Epi epi) {
 			}
 			if (lane == 0) {
 				v = R::add(v, wm_load_slot<T>(mt.head_val + f + nn - 1));
-				epi.row(mt.tile_row[f + 1], v, true);
+				const int64_t rf = mt.tile_row[f + 1];
+				epi.finish(rf, v, epi.load(rf));
 			}
 		}
 	}
