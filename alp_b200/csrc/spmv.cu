@@ -785,6 +785,43 @@ k_spmv_general_finish(SpmvArgs a, GenChunks g) {
 	gen_count(a, newly);
 }
 
+// Dense product of a small skewed matrix in one launch: a block per long row
+// (more than GEN_LONG nonzeroes), then a lane group per row.  Such a product
+// is launch and latency: the merge path's tile walk is a longer chain than
+// these two loads, and its crossing rows take a second launch.  Nothing is
+// shared between blocks, so a plan may serve several streams at once.
+template <class R, int W>
+__global__ void __launch_bounds__(256) k_spmv_small(SpmvArgs a, const int64_t *__restrict__ crow,
+	const int64_t *__restrict__ first, int64_t nlong) {
+	using T = typename R::T;
+	__shared__ T part[8];
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	T *y = reinterpret_cast<T *>(a.u);
+	T acc = R::zero();
+	bool set = false;
+	if (int64_t(blockIdx.x) < nlong) {
+		const int64_t i = crow[first[blockIdx.x]];
+		gen_gather<R, 256>(a, a.offsets[i], a.offsets[i + 1], threadIdx.x, acc, set);
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o));
+		if (lane == 0) part[w] = acc;
+		__syncthreads();
+		if (threadIdx.x == 0) {
+			for (int k = 1; k < 8; ++k) acc = R::add(acc, part[k]);
+			y[i] = R::add(y[i], acc);
+		}
+		return;
+	}
+	const int64_t i = ((int64_t(blockIdx.x) - nlong) * 256 + threadIdx.x) / W;
+	const int64_t b = i < a.m_out ? a.offsets[i] : 0, e = i < a.m_out ? a.offsets[i + 1] : 0;
+	const bool mine = e > b && e - b <= GEN_LONG;
+	const T old = mine ? y[i] : R::zero();
+	if (mine) gen_gather<R, W>(a, b, e, threadIdx.x & (W - 1), acc, set);
+#pragma unroll
+	for (int o = W / 2; o > 0; o >>= 1) acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o, W));
+	if (mine && (threadIdx.x & (W - 1)) == 0) y[i] = R::add(old, acc);
+}
+
 // Trivial case of blas2.hpp:1001-1037: the output keeps its values; with
 // explicit_zero every unassigned entry becomes the additive identity.
 template <class R>
@@ -905,6 +942,26 @@ int launch_vector_general_w(const SpmvArgs &a, const alpb_spmv_plan_s *p, cudaSt
 	return ALPB_SUCCESS;
 }
 
+// Matrices of up to SMALL_NNZ nonzeroes in rows of up to SMALL_ROW take
+// k_spmv_small where the merge path is the plan's own choice.  Measured us per
+// call (waited for), merge path / this, R-MAT: 4,096 vertices 30.5 / 23.7,
+// 10,000 28.4 / 22.8, 20,000 29.9 / 24.0, 30,000 29.4 / 26.3; 60,000 (0.86 M
+// nonzeroes) 31 either way.
+constexpr int64_t SMALL_NNZ = int64_t(1) << 19;
+constexpr int64_t SMALL_ROW = 8192;
+
+template <class R>
+int launch_small(const SpmvArgs &a, const alpb_spmv_plan_s &p, cudaStream_t s) {
+	const auto go = [&](auto width) {
+		constexpr int W = decltype(width)::value;
+		const int64_t grid = p.gen_rows + (a.m_out * W + 255) / 256;
+		k_spmv_small<R, W><<<unsigned(grid), 256, 0, s>>>(a, p.gen_row, p.gen_first, p.gen_rows);
+		ALPB_LAUNCHED();
+		return ALPB_SUCCESS;
+	};
+	return p.mean < 6 ? go(std::integral_constant<int, 4>{}) : go(std::integral_constant<int, 8>{});
+}
+
 template <class R>
 int launch_vector(const SpmvArgs &a, const alpb_spmv_plan_s *p, int W, bool dense,
 	cudaStream_t s) {
@@ -998,8 +1055,10 @@ int run_spmv(const SpmvArgs &a, const alpb_spmv_plan_s *p, int force_sched, cuda
 	}
 	int sched = force_sched ? force_sched : (p ? p->sched : ALPB_SCHED_VECTOR);
 	int W = p ? p->vw : default_width(a.m_out ? double(a.nnz) / double(a.m_out) : 1.0);
-	if (fast && sched == ALPB_SCHED_MERGE_PATH && p && p->tile_row)
+	if (fast && sched == ALPB_SCHED_MERGE_PATH && p && p->tile_row) {
+		if (p->small && p->lor_n >= 0 && !p->hot_on) return launch_small<R>(a, *p, s);
 		return launch_merge<R>(a, *p, s);
+	}
 	// regular short rows: the row-streaming kernel (16-byte copies of the
 	// storage's ranges, so its arrays have to start on such a boundary)
 	if (fast && p && p->rows && !(reinterpret_cast<uintptr_t>(a.indices) & 15) &&
@@ -1147,6 +1206,7 @@ int alpb::plan_create_tiles(alpb_spmv_plan_s **plan, int64_t m, int64_t nnz,
 	} else {
 		p->vw = regular ? regular_width(p->mean) : default_width(p->mean);
 	}
+	p->small = sched == ALPB_SCHED_AUTO && !regular && nnz <= SMALL_NNZ && p->maxlen <= SMALL_ROW;
 	if (sched == ALPB_SCHED_AUTO) sched = regular ? ALPB_SCHED_VECTOR : ALPB_SCHED_MERGE_PATH;
 	p->sched = sched;
 	p->rows = regular && vector_width <= 0 && p->maxlen >= 1 && p->maxlen <= RS_MAX_LEN;
@@ -1327,19 +1387,21 @@ int alpb_spmv_autotune(alpb_spmv_plan p, int ring, int64_t n, const uint32_t *in
 	ALPB_CUDA(cudaEventCreate(&e0));
 	ALPB_CUDA(cudaEventCreate(&e1));
 	// candidates: merge path, and vector widths around the mean row length
-	struct Cand { int sched, w; bool rows; } cands[8];
+	struct Cand { int sched, w; bool rows, small; } cands[8];
 	int nc = 0;
-	cands[nc++] = {ALPB_SCHED_MERGE_PATH, p->vw, false};
-	if (p->rows) cands[nc++] = {ALPB_SCHED_VECTOR, p->vw, true};
-	for (int w = 2; w <= 32; w *= 2) cands[nc++] = {ALPB_SCHED_VECTOR, w, false};
+	cands[nc++] = {ALPB_SCHED_MERGE_PATH, p->vw, false, false};
+	if (p->small) cands[nc++] = {ALPB_SCHED_MERGE_PATH, p->vw, false, true};
+	if (p->rows) cands[nc++] = {ALPB_SCHED_VECTOR, p->vw, true, false};
+	for (int w = 2; w <= 32; w *= 2) cands[nc++] = {ALPB_SCHED_VECTOR, w, false, false};
 	float best = 1e30f;
 	int best_i = 0;
 	const int saved_vw = p->vw;
-	const bool saved_rows = p->rows;
+	const bool saved_rows = p->rows, saved_small = p->small;
 	a.offsets = p->offsets;
 	for (int c = 0; c < nc; ++c) {
 		p->vw = cands[c].w;
 		p->rows = cands[c].rows;
+		p->small = cands[c].small;
 		float total = 0;
 		for (int rep = 0; rep < 4; ++rep) {
 			ALPB_CUDA(cudaEventRecord(e0, s));
@@ -1347,6 +1409,7 @@ int alpb_spmv_autotune(alpb_spmv_plan p, int ring, int64_t n, const uint32_t *in
 			if (rc != ALPB_SUCCESS) {
 				p->vw = saved_vw;
 				p->rows = saved_rows;
+				p->small = saved_small;
 				return rc;
 			}
 			ALPB_CUDA(cudaEventRecord(e1, s));
@@ -1360,6 +1423,7 @@ int alpb_spmv_autotune(alpb_spmv_plan p, int ring, int64_t n, const uint32_t *in
 	p->sched = cands[best_i].sched;
 	p->vw = cands[best_i].sched == ALPB_SCHED_VECTOR ? cands[best_i].w : saved_vw;
 	p->rows = cands[best_i].rows;
+	p->small = cands[best_i].small;
 	// skewed rows on the merge path: try the hot-column cache at four sizes,
 	// up to what the shared memory left by the warps' tiles holds
 	hot_release(p);

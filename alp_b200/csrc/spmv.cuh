@@ -9,6 +9,7 @@ struct alpb_spmv_plan_s {
 	const int64_t *offsets = nullptr;  // storage the plan was made for
 	int sched = ALPB_SCHED_VECTOR;
 	int vw = 8;
+	bool small = false;  // merge path by the plan's own choice: k_spmv_small instead
 	bool rows = false;   // vector schedule: short regular rows, streamed (rowstream.cuh)
 	int device = 0;
 	int64_t ntiles = 0;
