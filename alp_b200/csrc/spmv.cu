@@ -366,6 +366,8 @@ constexpr int LOR_CHUNK = 256;
 constexpr int GEN_LONG = 64;
 constexpr int GEN_CHUNK = 256;
 constexpr int GEN_BATCH = 4;
+constexpr int64_t GEN_NARROW = int64_t(1) << 20;
+constexpr int GEN_BATCH_BITS = 8;   // where the flags are bits in shared memory
 
 template <bool VALUED>
 __global__ void __launch_bounds__(256)
@@ -431,28 +433,35 @@ k_lor_tail(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ ind
 	}
 }
 
-// Chunk lists of the plan: per row of more than `longer` nonzeroes, its
-// nonzeroes from `head` on in chunks of `chunk`, consecutive in the list.
-// Pass 1 counts (rows == nullptr), pass 2 writes them at positions taken from
-// *count (any order of the rows: no result depends on it); first, when given,
-// lists each row's first chunk at a position from *nrows.
-__global__ void k_row_chunks(const int64_t *__restrict__ offsets, int64_t m, int64_t longer,
-	int64_t head, int64_t chunk, unsigned long long *count, unsigned long long *nrows,
-	int64_t *rows, int64_t *k0s, int64_t *first) {
+// One chunk list of the plan: per row of more than `longer` nonzeroes, its
+// nonzeroes from `head` on in chunks of `chunk`, consecutive in the list at a
+// position taken from *count (any order of the rows: no result depends on
+// it); first, when given, lists each row's first chunk at a position from
+// *nrows.  rows == nullptr: count only.
+struct ChunkList {
+	int64_t longer, head, chunk;
+	unsigned long long *count, *nrows;
+	int64_t *rows, *k0s, *first;
+};
+__device__ __forceinline__ void add_row_chunks(const ChunkList &l, int64_t i, int64_t o, int64_t e) {
+	if (e - o <= l.longer) return;
+	const int64_t b = o + l.head, n = (e - b + l.chunk - 1) / l.chunk;
+	const unsigned long long at = atomicAdd(l.count, (unsigned long long) n);
+	const unsigned long long r = atomicAdd(l.nrows, 1ull);
+	if (!l.rows) return;
+	for (int64_t c = 0; c < n; ++c) {
+		l.rows[at + c] = i;
+		l.k0s[at + c] = b + c * l.chunk;
+	}
+	if (l.first) l.first[r] = int64_t(at);
+}
+__global__ void k_row_chunks(const int64_t *__restrict__ offsets, int64_t m, ChunkList p,
+	ChunkList q) {
 	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m;
 		 i += int64_t(gridDim.x) * blockDim.x) {
-		const int64_t b = offsets[i] + head, e = offsets[i + 1];
-		if (e - offsets[i] <= longer) continue;
-		const int64_t n = (e - b + chunk - 1) / chunk;
-		const unsigned long long at = atomicAdd(count, (unsigned long long) n);
-		const unsigned long long l = atomicAdd(nrows, 1ull);
-		if (rows) {
-			for (int64_t c = 0; c < n; ++c) {
-				rows[at + c] = i;
-				k0s[at + c] = b + c * chunk;
-			}
-			if (first) first[l] = int64_t(at);
-		}
+		const int64_t o = offsets[i], e = offsets[i + 1];
+		add_row_chunks(p, i, o, e);
+		add_row_chunks(q, i, o, e);
 	}
 }
 
@@ -479,11 +488,9 @@ static int lists_build(alpb_spmv_plan_s *p, cudaStream_t s) {
 	unsigned long long *cnt = nullptr, h[4] = {0, 0, 0, 0};  // lor chunks, rows; general chunks, rows
 	ALPB_CUDA(cudaMallocAsync(&cnt, sizeof(h), s));
 	ALPB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(h), s));
-	k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, LOR_HEAD, LOR_HEAD, LOR_CHUNK, cnt,
-		cnt + 1, nullptr, nullptr, nullptr);
-	ALPB_LAUNCHED();
-	k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, GEN_LONG, 0, GEN_CHUNK, cnt + 2, cnt + 3,
-		nullptr, nullptr, nullptr);
+	ChunkList lor{LOR_HEAD, LOR_HEAD, LOR_CHUNK, cnt, cnt + 1, nullptr, nullptr, nullptr};
+	ChunkList gen{GEN_LONG, 0, GEN_CHUNK, cnt + 2, cnt + 3, nullptr, nullptr, nullptr};
+	k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, lor, gen);
 	ALPB_LAUNCHED();
 	ALPB_CUDA(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, s));
 	ALPB_CUDA(cudaStreamSynchronize(s));
@@ -501,14 +508,13 @@ static int lists_build(alpb_spmv_plan_s *p, cudaStream_t s) {
 			return ALPB_OUTOFMEM;
 		}
 		ALPB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(h), s));
-		k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, LOR_HEAD, LOR_HEAD, LOR_CHUNK, cnt,
-			cnt + 1, p->lor_row, p->lor_k0, nullptr);
+		lor.rows = p->lor_row;
+		lor.k0s = p->lor_k0;
+		gen.rows = p->gen_row;
+		gen.k0s = p->gen_k0;
+		gen.first = p->gen_first;
+		k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, lor, gen);
 		ALPB_LAUNCHED();
-		if (h[2] > 0) {
-			k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, GEN_LONG, 0, GEN_CHUNK, cnt + 2,
-				cnt + 3, p->gen_row, p->gen_k0, p->gen_first);
-			ALPB_LAUNCHED();
-		}
 	}
 	ALPB_CUDA(cudaFreeAsync(cnt, s));
 	p->lor_n = int64_t(h[0]);
@@ -586,31 +592,55 @@ k_spmv_vector_dense(const int64_t *__restrict__ offsets, const uint32_t *__restr
 // (the plan's list), one warp each, first in the item order; their partials
 // are summed in chunk order by k_spmv_general_finish (deterministic).
 // Measured, R-MAT: min-plus from a 20% sparse vector, 500,009 vertices,
-// 2289 -> 118 us; lor-land with a 5% frontier and 30% visited, 1,000,003
-// vertices, 474 -> 188 us.
+// 2289 -> 118 us, 78 with the bits and the narrow groups below; lor-land with a
+// 5% frontier and 30% visited, 1,000,003
+// vertices, 474 -> 188, 142 us.
 
-// Rows of the general path: who takes part, and the row's identity term.
+// Rows of the general path: who takes part, and the row's identity term.  Made
+// in two halves: fetch() loads what the row's place says (no load waits for
+// another), decide() reads it, one item later in the row loop.
 template <class R>
 struct GenRow {
-	bool row_ok, id_row, u_has;
-	__device__ __forceinline__ GenRow(const SpmvArgs &a, int64_t i, bool in_range) {
-		row_ok = in_range;
-		if (row_ok && a.masked)
-			row_ok = a.mask_by_structure
-				? (a.u_mask_assigned == nullptr || a.u_mask_assigned[i] != 0)
-				: eval_mask(a.u_mask, a.u_mask_assigned, a.u_mask_type, a.descr, i);
-		id_row = in_range && (a.descr & ALPB_DESC_ADD_IDENTITY) && (a.scatter_sem || row_ok);
-		u_has = in_range && (a.u_assigned == nullptr || a.u_assigned[i] != 0);
+	using T = typename R::T;
+	int64_t i = -1, b = 0, e = 0;
+	uint8_t mask_has, u_flag;
+	T old;
+	bool row_ok = false, id_row = false, u_has = false;
+	__device__ __forceinline__ void fetch(const SpmvArgs &a, int64_t row) {
+		i = row;
+		b = e = 0;
+		mask_has = u_flag = 1;
+		old = R::zero();
+		if (i < 0) return;
+		b = a.offsets[i];
+		e = a.offsets[i + 1];
+		if (a.masked && a.u_mask_assigned) mask_has = a.u_mask_assigned[i];
+		if (a.u_assigned) u_flag = a.u_assigned[i];
+		old = reinterpret_cast<const T *>(a.u)[i];
+	}
+	// longest: rows of more nonzeroes are somebody else's
+	__device__ __forceinline__ void decide(const SpmvArgs &a, int64_t longest) {
+		row_ok = i >= 0 && e - b <= longest;
+		const bool mine = row_ok;
+		if (row_ok && a.masked) {
+			bool t = mask_has != 0;
+			if (!a.mask_by_structure) {   // as eval_mask
+				if (t && !(a.descr & ALPB_DESC_STRUCTURAL) && a.u_mask != nullptr &&
+					a.u_mask_type != ALPB_VOID)
+					t = mask_value_true(a.u_mask, a.u_mask_type, i);
+				if (a.descr & ALPB_DESC_INVERT_MASK) t = !t;
+			}
+			row_ok = t;
+		}
+		id_row = mine && (a.descr & ALPB_DESC_ADD_IDENTITY) && (a.scatter_sem || row_ok);
+		u_has = mine && u_flag != 0;
 		// immutable-nonzero shortcut of the gather (blas2.hpp:351-357)
-		if (R::immutable && !a.scatter_sem && row_ok && u_has &&
-			reinterpret_cast<const typename R::T *>(a.u)[i] != R::zero())
-			row_ok = false;
+		if (R::immutable && !a.scatter_sem && row_ok && u_has && old != R::zero()) row_ok = false;
 	}
 	// the identity's contribution to row i (add_identity), if any
-	__device__ __forceinline__ void identity(const SpmvArgs &a, int64_t i, typename R::T &acc,
-		bool &set) const {
+	__device__ __forceinline__ void identity(const SpmvArgs &a, T &acc, bool &set) const {
 		if (!id_row || i >= a.n_in) return;
-		const typename R::T *x = reinterpret_cast<const typename R::T *>(a.v);
+		const T *x = reinterpret_cast<const T *>(a.v);
 		const bool vm_ok = !a.input_masked ||
 			eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, i);
 		if (vm_ok && ((a.descr & ALPB_DESC_DENSE) || a.v_assigned == nullptr || a.v_assigned[i])) {
@@ -619,13 +649,12 @@ struct GenRow {
 		}
 	}
 	// fold the row's sum into the output; counts a newly assigned entry
-	__device__ __forceinline__ void finish(const SpmvArgs &a, int64_t i, typename R::T acc,
-		bool set, int64_t &newly) const {
+	__device__ __forceinline__ void finish(const SpmvArgs &a, T acc, bool set,
+		int64_t &newly) const {
 		const bool dense_hint = (a.descr & ALPB_DESC_DENSE) != 0;
 		const bool ez = (a.descr & ALPB_DESC_EXPLICIT_ZERO) && !a.scatter_sem && row_ok;
 		if (!(row_ok || id_row) || !(ez || set)) return;
-		typename R::T *y = reinterpret_cast<typename R::T *>(a.u);
-		y[i] = u_has || dense_hint ? R::add(y[i], acc) : acc;
+		reinterpret_cast<T *>(a.u)[i] = u_has || dense_hint ? R::add(old, acc) : acc;
 		if (!u_has && a.u_assigned) {
 			a.u_assigned[i] = 1;
 			++newly;
@@ -633,12 +662,12 @@ struct GenRow {
 	}
 };
 
-// acc (+)= the products of nonzeroes b + lane, b + lane + W, ... < e, in that
-// order; set: any product was there.  With stop_early (immutable rings) a
-// lane ends after a batch that made its sum nonzero.
-template <class R, int W>
+// bits: which inputs take part, one bit each (v_assigned and the input mask
+// are then not read); null without BITS.
+template <class R, int W, bool BITS = false>
 __device__ __forceinline__ void gen_gather(const SpmvArgs &a, int64_t b, int64_t e, int lane,
-	typename R::T &acc, bool &set) {
+	typename R::T &acc, bool &set, const uint32_t *bits = nullptr) {
+	constexpr int GEN_BATCH = BITS ? GEN_BATCH_BITS : ::alpb::GEN_BATCH;
 	using T = typename R::T;
 	const T *__restrict__ values = reinterpret_cast<const T *>(a.values);
 	const T *__restrict__ x = reinterpret_cast<const T *>(a.v);
@@ -653,13 +682,18 @@ __device__ __forceinline__ void gen_gather(const SpmvArgs &a, int64_t b, int64_t
 			on[q] = k0 + q * W < e;
 			j[q] = on[q] ? __ldcs(a.indices + k0 + q * W) : 0u;
 		}
-		if (a.input_masked) {
+		if (BITS) {
+#pragma unroll
+			for (int q = 0; q < GEN_BATCH; ++q)
+				if (on[q]) on[q] = (bits[j[q] >> 5] >> (j[q] & 31)) & 1u;
+		}
+		if (!BITS && a.input_masked) {
 #pragma unroll
 			for (int q = 0; q < GEN_BATCH; ++q)
 				if (on[q])
 					on[q] = eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, j[q]);
 		}
-		if (va) {
+		if (!BITS && va) {
 #pragma unroll
 			for (int q = 0; q < GEN_BATCH; ++q)
 				if (on[q]) on[q] = va[j[q]] != 0;
@@ -701,10 +735,34 @@ __device__ __forceinline__ void gen_count(const SpmvArgs &a, int64_t newly) {
 		atomicAdd((unsigned long long *) a.u_nnz, (unsigned long long) newly);
 }
 
-template <class R, int W>
-__global__ void __launch_bounds__(256)
-k_spmv_vector_general(SpmvArgs a, GenChunks g) {
+// Which inputs take part (assigned, and let through by the input mask), a bit
+// each.
+__global__ void k_pack_present(SpmvArgs a, uint32_t *bits) {
+	const int64_t n32 = (a.n_in + 31) / 32 * 32;
+	for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < n32;
+		 j += int64_t(gridDim.x) * blockDim.x) {
+		const bool on = j < a.n_in && (a.v_assigned == nullptr || a.v_assigned[j] != 0) &&
+			(!a.input_masked || eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, j));
+		const unsigned w = __ballot_sync(0xffffffffu, on);
+		if ((threadIdx.x & 31) == 0) bits[j >> 5] = w;
+	}
+}
+
+// BITS: every block copies the inputs' bits into its shared memory first.  A
+// nonzero then asks shared memory whether its input takes part (a warp's 32
+// random words are about four wavefronts there, and up to 32 in L1), and only
+// those that do gather x.
+template <class R, int W, bool BITS>
+__global__ void __launch_bounds__(BITS ? 1024 : 256)
+k_spmv_vector_general(SpmvArgs a, GenChunks g, const uint32_t *__restrict__ gbits) {
 	using T = typename R::T;
+	extern __shared__ __align__(16) uint32_t gen_bits[];
+	if (BITS) {
+		const int64_t words = (a.n_in + 31) / 32;
+		for (int64_t k = threadIdx.x; k < (words + 3) / 4; k += blockDim.x)
+			reinterpret_cast<uint4 *>(gen_bits)[k] = reinterpret_cast<const uint4 *>(gbits)[k];
+		__syncthreads();
+	}
 	constexpr int RPW = 32 / W;
 	const int wl = threadIdx.x & 31;
 	const int lane = threadIdx.x & (W - 1);
@@ -714,42 +772,47 @@ k_spmv_vector_general(SpmvArgs a, GenChunks g) {
 	const int64_t items = g.nchunks + (a.m_out + RPW - 1) / RPW;
 	const int64_t long_len = g.nchunks > 0 ? GEN_LONG : INT64_MAX;
 	int64_t newly = 0;
-	for (int64_t it = warp; it < items; it += nwarps) {
-		if (it < g.nchunks) {   // one chunk of a long row, the whole warp
-			const int64_t i = g.row[it], k0 = g.k0[it];
-			const GenRow<R> row(a, i, true);
-			T acc = R::zero();
-			bool set = false;
-			if (row.row_ok) {
-				int64_t e = a.offsets[i + 1];
-				if (e > k0 + GEN_CHUNK) e = k0 + GEN_CHUNK;
-				gen_gather<R, 32>(a, k0, e, wl, acc, set);
-			}
-#pragma unroll
-			for (int o = 16; o > 0; o >>= 1)
-				acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o));
-			set = __any_sync(0xffffffffu, set);
-			if (wl == 0) {
-				store_bits<T>(g.val + it, acc);
-				g.has[it] = set ? 1 : 0;
-			}
-			continue;
-		}
-		const int64_t i = (it - g.nchunks) * RPW + sub;
-		const bool in_range = i < a.m_out;
-		const int64_t b = in_range ? a.offsets[i] : 0, e = in_range ? a.offsets[i + 1] : 0;
-		const bool mine = in_range && e - b <= long_len;
-		const GenRow<R> row(a, i, mine);
+	int64_t it = warp;
+	for (; it < g.nchunks; it += nwarps) {   // one chunk of a long row, the whole warp
+		GenRow<R> row;
+		row.fetch(a, g.row[it]);
+		const int64_t k0 = g.k0[it];
+		row.decide(a, INT64_MAX);
 		T acc = R::zero();
 		bool set = false;
-		if (lane == 0) row.identity(a, i, acc, set);
-		if (row.row_ok) gen_gather<R, W>(a, b, e, lane, acc, set);
+		if (row.row_ok)
+			gen_gather<R, 32, BITS>(a, k0, row.e < k0 + GEN_CHUNK ? row.e : k0 + GEN_CHUNK, wl, acc,
+				set, gen_bits);
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o));
+		set = __any_sync(0xffffffffu, set);
+		if (wl == 0) {
+			store_bits<T>(g.val + it, acc);
+			g.has[it] = set ? 1 : 0;
+		}
+	}
+	// groups of rows; what the next group's rows say is fetched before this
+	// one's gathers, which then are all an item waits for
+	const auto row_of = [&](int64_t t) {
+		const int64_t i = (t - g.nchunks) * RPW + sub;
+		return t < items && i < a.m_out ? i : int64_t(-1);
+	};
+	GenRow<R> row, nxt;
+	row.fetch(a, row_of(it));
+	for (; it < items; it += nwarps) {
+		nxt.fetch(a, row_of(it + nwarps));
+		row.decide(a, long_len);
+		T acc = R::zero();
+		bool set = false;
+		if (lane == 0) row.identity(a, acc, set);
+		if (row.row_ok) gen_gather<R, W, BITS>(a, row.b, row.e, lane, acc, set, gen_bits);
 #pragma unroll
 		for (int o = W / 2; o > 0; o >>= 1) {
 			acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o, W));
 			set = set | (__shfl_down_sync(0xffffffffu, int(set), o, W) != 0);
 		}
-		if (lane == 0) row.finish(a, i, acc, set, newly);
+		if (lane == 0) row.finish(a, acc, set, newly);
+		row = nxt;
 	}
 	gen_count(a, newly);
 }
@@ -765,12 +828,14 @@ k_spmv_general_finish(SpmvArgs a, GenChunks g) {
 	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
 	int64_t newly = 0;
 	for (int64_t l = warp; l < g.nlong; l += nwarps) {
-		const int64_t c0 = g.first[l], i = g.row[c0];
-		const int64_t n = (a.offsets[i + 1] - g.k0[c0] + GEN_CHUNK - 1) / GEN_CHUNK;
-		const GenRow<R> row(a, i, true);
+		const int64_t c0 = g.first[l];
+		GenRow<R> row;
+		row.fetch(a, g.row[c0]);
+		const int64_t n = (row.e - row.b + GEN_CHUNK - 1) / GEN_CHUNK;
+		row.decide(a, INT64_MAX);
 		T acc = R::zero();
 		bool set = false;
-		if (lane == 0) row.identity(a, i, acc, set);
+		if (lane == 0) row.identity(a, acc, set);
 		if (row.row_ok)
 			for (int64_t c = c0 + lane; c < c0 + n; c += 32)
 				if (g.has[c]) {
@@ -780,7 +845,7 @@ k_spmv_general_finish(SpmvArgs a, GenChunks g) {
 #pragma unroll
 		for (int o = 16; o > 0; o >>= 1) acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o));
 		set = __any_sync(0xffffffffu, set);
-		if (lane == 0) row.finish(a, i, acc, set, newly);
+		if (lane == 0) row.finish(a, acc, set, newly);
 	}
 	gen_count(a, newly);
 }
@@ -910,29 +975,62 @@ int launch_vector_dense_w(const SpmvArgs &a, cudaStream_t s) {
 	return ALPB_SUCCESS;
 }
 
+// The general path asks the inputs' bits in shared memory from GEN_BITS_NNZ
+// nonzeroes on, for vectors whose bits fit beside an L1 of some size.  R-MAT,
+// us, flags in memory / bits: 500,009 vertices, min-plus, 20% sparse, 118 / 88;
+// 100,000 vertices, lor, 36 / 40, min-plus 25 / 27 (packing costs a launch).
+constexpr int64_t GEN_BITS_NNZ = int64_t(1) << 21;
+constexpr int64_t GEN_BITS_MAX = 200 * 1024 * 8;
+
 template <class R, int W>
 int launch_vector_general_w(const SpmvArgs &a, const alpb_spmv_plan_s *p, cudaStream_t s) {
 	constexpr int RPW = 32 / W;
 	GenChunks g;
 	void *scratch = nullptr;
-	if (p && p->gen_n > 0) {
-		// partials of the long rows' chunks, this call's own (calls on other
-		// streams may use the same plan); without them every row runs in a group
-		if (cudaMallocAsync(&scratch, size_t(p->gen_n) * 9, s) == cudaSuccess) {
-			g.nchunks = p->gen_n;
-			g.nlong = p->gen_rows;
-			g.row = p->gen_row;
-			g.k0 = p->gen_k0;
-			g.first = p->gen_first;
-			g.val = static_cast<uint64_t *>(scratch);
-			g.has = reinterpret_cast<uint8_t *>(g.val + p->gen_n);
+	uint32_t *bits = nullptr;
+	const bool filtered = a.input_masked || (a.v_assigned && !(a.descr & ALPB_DESC_DENSE));
+	const bool want_bits = filtered && a.nnz >= GEN_BITS_NNZ && a.n_in <= GEN_BITS_MAX;
+	const size_t bit_bytes = want_bits ? size_t(a.n_in + 127) / 128 * 16 : 0;
+	const int64_t chunks = p && p->gen_n > 0 ? p->gen_n : 0;
+	if (bit_bytes || chunks) {
+		// bits, then the partials of the long rows' chunks: this call's own
+		// (calls on other streams may use the same plan); without them every
+		// row runs in a group and asks the flags in memory
+		if (cudaMallocAsync(&scratch, bit_bytes + size_t(chunks) * 9, s) == cudaSuccess) {
+			unsigned char *at = static_cast<unsigned char *>(scratch);
+			if (bit_bytes) bits = reinterpret_cast<uint32_t *>(at);
+			if (chunks) {
+				g.nchunks = chunks;
+				g.nlong = p->gen_rows;
+				g.row = p->gen_row;
+				g.k0 = p->gen_k0;
+				g.first = p->gen_first;
+				g.val = reinterpret_cast<uint64_t *>(at + bit_bytes);
+				g.has = reinterpret_cast<uint8_t *>(g.val + chunks);
+			}
 		} else {
 			cudaGetLastError();
 			scratch = nullptr;
 		}
 	}
 	const int64_t items = g.nchunks + (a.m_out + RPW - 1) / RPW;
-	k_spmv_vector_general<R, W><<<grid_for(items * 32, 256, 8), 256, 0, s>>>(a, g);
+	if (bits) {
+		static std::atomic<bool> ready[64];
+		int dev = 0;
+		ALPB_CUDA(cudaGetDevice(&dev));
+		if (dev >= 64 || !ready[dev].load()) {
+			ALPB_CUDA(cudaFuncSetAttribute(k_spmv_vector_general<R, W, true>,
+				cudaFuncAttributeMaxDynamicSharedMemorySize, int(GEN_BITS_MAX / 8)));
+			if (dev < 64) ready[dev].store(true);
+		}
+		k_pack_present<<<grid_for(a.n_in, 256), 256, 0, s>>>(a, bits);
+		ALPB_LAUNCHED();
+		k_spmv_vector_general<R, W, true><<<grid_for(items * 32, 1024, 1), 1024, bit_bytes, s>>>(a,
+			g, bits);
+	} else {
+		k_spmv_vector_general<R, W, false><<<grid_for(items * 32, 256, 8), 256, 0, s>>>(a, g,
+			nullptr);
+	}
 	ALPB_LAUNCHED();
 	if (g.nlong > 0) {
 		k_spmv_general_finish<R><<<grid_for(g.nlong * 32, 256, 8), 256, 0, s>>>(a, g);
@@ -1064,6 +1162,11 @@ int run_spmv(const SpmvArgs &a, const alpb_spmv_plan_s *p, int force_sched, cuda
 	if (fast && p && p->rows && !(reinterpret_cast<uintptr_t>(a.indices) & 15) &&
 		!(reinterpret_cast<uintptr_t>(a.values) & 15))
 		return launch_rows<R>(a, int(p->maxlen), s);
+	// The general path waits for a row's chain of loads, so from GEN_NARROW
+	// nonzeroes on a quarter of the lanes per row, and four times the rows in
+	// flight, is faster (R-MAT, us with 8 / 2 lanes: 1,000,003 vertices, lor,
+	// 185 / 144, 500,009, min-plus, 90 / 70; 20,000: 15.8 / 17.8).
+	if (!fast && a.nnz >= GEN_NARROW && W >= 4) W /= 4;
 	return launch_vector<R>(a, p, W, fast, s);
 }
 

@@ -67,3 +67,47 @@ def test_general_path_long_rows(cuda, oracle, ring, descr, frontier):
         else:
             np.testing.assert_array_equal(got, want)
     plan.close()
+
+
+@pytest.mark.parametrize("n", [65537, 1638400, 1638401])
+@pytest.mark.parametrize("case", ["sparse", "input_mask", "both_inverted"])
+@pytest.mark.parametrize("ring", [0, 1, 2])
+def test_general_path_input_bits(cuda, oracle, ring, case, n):
+    """From 2^21 nonzeroes on the inputs that take part are asked as bits in
+    shared memory, up to 1,638,400 of them (one more: in memory, as below);
+    the last word is ragged for most n.  Rows of up to 2e5 terms: FP64 orders
+    agree to 2 * 2e5 * 2^-53 = 5e-11."""
+    import torch
+    from alp_b200 import device as dev
+    vtype = {0: 3, 1: 1, 2: 2}[ring]
+    npt = {3: np.float64, 2: np.int32, 1: np.uint8}[vtype]
+    rng = np.random.default_rng([ring, n])
+    lens = rng.integers(0, 70, 60000)
+    lens[[5, 77]] = 200000, 300
+    m, nnz = len(lens), int(lens.sum())
+    assert nnz >= 1 << 21
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    col = rng.integers(0, n, nnz).astype(np.uint32)
+    col[-1] = n - 1
+    value = lambda k: (rng.random(k) if vtype == 3 else rng.integers(0, 2 if vtype == 1 else 1000, k)).astype(npt)  # noqa: E731
+    vals, u, v = value(nnz), value(m), value(n)
+    va = (rng.random(n) < 0.1).astype(np.uint8)
+    vm, vma = (rng.random(n) < 0.5).astype(np.uint8), (rng.random(n) < 0.6).astype(np.uint8)
+    kw, gkw, descr = {}, {}, 0
+    T = lambda a: torch.from_numpy(a.copy()).cuda()  # noqa: E731
+    if case != "input_mask":
+        kw["v_assigned"], gkw["v_assigned"] = va, T(va)
+    if case != "sparse":
+        kw.update(v_mask=vm, v_mask_assigned=vma, v_mask_count=int(vma.sum()))
+        gkw.update(v_mask=T(vm), v_mask_assigned=T(vma), v_mask_count=int(vma.sum()))
+        descr = 1 if case == "both_inverted" else 0
+    want = u.copy()
+    assert oracle.mxv(ring, descr, 0, m, n, rp, col, vals, vtype, want, v=v, **kw)[0] == 0
+    A = dev.from_host(m, n, rp, col, vals, vtype)
+    for plan in (dev.Plan(A), None):
+        got = T(u)
+        dev.mxv(ring, A, got, T(v), descr=descr, form=0, plan=plan, **gkw)
+        if vtype == 3:
+            np.testing.assert_allclose(got.cpu().numpy(), want, rtol=5e-11, atol=0)
+        else:
+            np.testing.assert_array_equal(got.cpu().numpy(), want)
