@@ -374,13 +374,14 @@ __device__ __forceinline__ void hp_load_seeds(const HpArgs &a, const HpLanes<G, 
 
 // Chunk descriptor of the chunk loop (warp-uniform).
 struct HpMeta {
-	int64_t b, r;
+	int64_t b;
+	uint32_t r;
 	int len;
 	int32_t slot;
 };
 
 __device__ __forceinline__ HpMeta hp_meta(const HpArgs &a, int64_t c) {
-	HpMeta m{0, 0, 0, -1};
+	HpMeta m{0, 0u, 0, -1};
 	if (c < a.nchunks) {
 		m.b = __ldg(a.beg + c);
 		m.len = int(__ldg(a.beg + c + 1) - m.b);
@@ -428,12 +429,11 @@ __global__ void __launch_bounds__(32 * HP_WARPS, ALPB_HP_MINB) k_hp_chunks(HpArg
 #pragma unroll
 		for (int q = 0; q < SPL; ++q) acc[q] = 0.0;
 		for (int t0 = 0; t0 < m.len; t0 += B * STEP) {
-			double v[B][SPL], wv[B];
+			double v[B][SPL];
 #pragma unroll
 			for (int u = 0; u < B; ++u) {
 				const int t = t0 + u * STEP + L.gsub;
 				const uint32_t i = __shfl_sync(0xffffffffu, myi, t & 31);
-				wv[u] = __shfl_sync(0xffffffffu, myw, t & 31);
 				const double *src = a.in + int64_t(i) * S;
 #pragma unroll
 				for (int q = 0; q < SPL; ++q) {
@@ -443,8 +443,11 @@ __global__ void __launch_bounds__(32 * HP_WARPS, ALPB_HP_MINB) k_hp_chunks(HpArg
 			}
 #pragma unroll
 			for (int u = 0; u < B; ++u) {
+				// the weight is broadcast where it is used: held over the gathers
+				// it would take two registers of each
+				const double wv = __shfl_sync(0xffffffffu, myw, (t0 + u * STEP + L.gsub) & 31);
 #pragma unroll
-				for (int q = 0; q < SPL; ++q) acc[q] = fma(wv[u], v[u][q], acc[q]);
+				for (int q = 0; q < SPL; ++q) acc[q] = fma(wv, v[u][q], acc[q]);
 			}
 		}
 		uint32_t ni = 0;
