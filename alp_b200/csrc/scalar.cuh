@@ -27,10 +27,10 @@ struct ScalarScratch {
 // The calling thread's scratch on the current device (runtime.cu).
 int scalar_scratch(ScalarScratch *out, cudaStream_t s);
 
-// Blocks of a reduction over n entries: eight entries per thread, at most four
-// blocks per SM.
+// Blocks of a reduction over n entries: four entries per thread (one batch of
+// loads) up to the blocks that are resident together.
 inline int scalar_grid(int64_t n) {
-	int64_t g = (n + SCALAR_BLOCK * 8 - 1) / (SCALAR_BLOCK * 8);
+	int64_t g = (n + SCALAR_BLOCK * 4 - 1) / (SCALAR_BLOCK * 4);
 	int64_t cap = int64_t(sm_count()) * 4;
 	if (cap > SCALAR_MAX_BLOCKS) cap = SCALAR_MAX_BLOCKS;
 	if (g > cap) g = cap;
