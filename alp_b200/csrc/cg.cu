@@ -251,7 +251,7 @@ struct CgRowsShape {
 static CgRowsShape cg_rows_shape(int64_t n, int maxlen) {
 	CgRowsShape c;
 	const size_t cap = CGR_SMEM;
-	const int64_t sms = sm_count() < 256 ? sm_count() : 256;   // partials of GridReduce
+	const int64_t sms = sm_count() < GRID_REDUCE_BLOCKS ? sm_count() : GRID_REDUCE_BLOCKS;
 	const int64_t per = (n + sms - 1) / sms;
 	if (per > (1 << 24) || maxlen < 1) return c;
 	while (c.L < 8 && c.L * 2 <= maxlen && (per * c.L + 31) / 32 * 2 <= CGR_WARPS) c.L *= 2;

@@ -16,13 +16,15 @@
 #include "spmv.cuh"
 
 #include <cmath>
+#include <cstddef>
 
 namespace alpb {
 
 using RF = RingPlusTimesF64;
 
 struct PrState {
-	GridSync gs;
+	GridReduce gr;
+	int err;           // a barrier or tile wait gave up
 	int64_t iterations;
 	double residual;
 	int zero_values;   // a stored value of the CRS is zero
@@ -36,15 +38,15 @@ struct PrArgs {
 	const int64_t *crs_ptr;
 	const double *crs_val;
 	double *pr, *rs, *next0, *next1;
-	double *blk;                   // [5][grid]: setup dangling mass; per iteration
-	                               // parity p, residual [1+2p] and dangling [2+2p]
 	int64_t n, max_iter;
 	double alpha, conv;
 	int init_given;
 	PrState *st;
 };
 
-constexpr int PR_WARPS = 4;
+// One block of 16 warps per SM: the iteration of a small graph is its barrier,
+// whose cost grows with the blocks (grid_reduce), and a tile or two per warp.
+constexpr int PR_WARPS = 16;
 
 struct PrWarpSmem {
 	WarpSmem<RF> tile;
@@ -137,27 +139,27 @@ struct GatherL2 {
 	__device__ __forceinline__ double operator()(uint32_t j) const { return __ldcg(x + j); }
 };
 
-// One barrier per iteration; the block partials of iteration k live in the
-// parity-(k & 1) slots, so a block that already writes iteration k+1's never
-// overwrites what a slower block still reads of iteration k.
-__global__ void __launch_bounds__(32 * PR_WARPS, 6) k_pagerank(PrArgs a) {
-	__shared__ PrWarpSmem sm[PR_WARPS];
-	__shared__ double red[33];
+// One barrier per iteration, which carries the iteration's two sums (the L1
+// change and the dangling mass).
+__global__ void __launch_bounds__(32 * PR_WARPS, 1) k_pagerank(PrArgs a) {
+	extern __shared__ __align__(16) unsigned char pr_smem[];
+	PrWarpSmem *sm = reinterpret_cast<PrWarpSmem *>(pr_smem);   // one per warp
+	__shared__ double red[64 * 2];
 	PrState *st = a.st;
-	int *err = &st->gs.err;
+	int *err = &st->err;
 	const int64_t G = gridDim.x, n = a.n, nt = a.mt.ntiles;
 	const int w = threadIdx.x >> 5;
-	const int64_t gw = int64_t(blockIdx.x) * PR_WARPS + w, nw = G * PR_WARPS;
+	// tiles go round the blocks first, so a small graph uses every SM
+	const int64_t gw = int64_t(w) * G + blockIdx.x, nw = G * PR_WARPS;
+	unsigned epoch = 0;
 	// setup: out-degree counts of nonzero-valued entries (the pattern ring of
 	// :224-237), alpha / count (:281-289), initial guess, pre-scaled input
 	for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < nt;
 		 t += G * blockDim.x)
 		a.mt.ready[t] = 0;
-	double dang = pr_setup_rows(a, st->zero_values != 0);
-	dang = block_sum(dang, red);
-	if (threadIdx.x == 0) a.blk[blockIdx.x] = dang;
-	if (!grid_sync(&st->gs)) return;
-	dang = block_sum_array(a.blk, G, red);
+	double dang;
+	if (!grid_reduce(&st->gr, ++epoch, pr_setup_rows(a, st->zero_values != 0), &dang, red, err))
+		return;
 
 	int64_t iter = 0;
 	double residual = 0.0;
@@ -166,28 +168,21 @@ __global__ void __launch_bounds__(32 * PR_WARPS, 6) k_pagerank(PrArgs a) {
 		const double d = (a.alpha * dang + 1 - a.alpha) / double(n);  // (:390)
 		PrEpi epi{&a, &sm[w], nxt, d};
 		GatherL2 xl{cur};
-		const int32_t epoch = int32_t(iter + 1);
 		int64_t t = gw;
 		WmMeta g = wm_meta(a.mt, t);
 		while (t < nt) {
 			const WmMeta next = wm_meta(a.mt, t + nw);
 			if (!warp_tile_ordered<RF>(t, g, a.mt, a.ccs_ptr, a.ccs_row, a.ccs_val, xl, epi, 1,
-					sm[w].tile, epoch, err))
+					sm[w].tile, int32_t(iter + 1), err))
 				break;
 			t += nw;
 			g = next;
 		}
-		double *blk_res = a.blk + (1 + 2 * (iter & 1)) * G;
-		double *blk_dang = a.blk + (2 + 2 * (iter & 1)) * G;
-		const double s1 = block_sum(epi.acc_res, red);
-		const double s2 = block_sum(epi.acc_dang, red);
-		if (threadIdx.x == 0) {
-			blk_res[blockIdx.x] = s1;
-			blk_dang[blockIdx.x] = s2;
-		}
-		if (!grid_sync(&st->gs)) return;
-		residual = block_sum_array(blk_res, G, red);
-		dang = block_sum_array(blk_dang, G, red);
+		const double v[2] = {epi.acc_res, epi.acc_dang};
+		double sum[2];
+		if (!grid_reduce<2>(&st->gr, ++epoch, v, sum, red, err)) return;
+		residual = sum[0];
+		dang = sum[1];
 		++iter;
 		if (a.conv != 0.0 && residual <= a.conv) break;   // (:490)
 		if (iter >= a.max_iter) break;
@@ -507,8 +502,8 @@ static int pagerank_steps(const PrStepArgs &tmpl, alpb_spmv_plan plan, int64_t *
 }
 
 // Graphs from this many nonzeroes on take the per-step launches.  Measured us
-// per solve, one kernel against steps, R-MAT: 0.45 M nonzeroes 361 / 438,
-// 0.9 M 557 / 557, 1.5 M 733 / 644, 4.6 M 1260 / 1020, 15 M 4170 / 2840.
+// per solve, one kernel against steps, R-MAT: 0.86 M nonzeroes 440 / 557, 1.2 M
+// 501 / 496, 2.1 M 750 / 715, 2.9 M 986 / 840, 4.3 M 1358 / 1005.
 constexpr int64_t kPrStepNnz = int64_t(1) << 20;
 
 // The solve proper.  plan: a WM_TILE plan of the CCS offsets, or null (one is
@@ -557,19 +552,33 @@ static int pagerank_run(int64_t n, const int64_t *crs_row_ptr, const double *crs
 		alpb_spmv_plan_destroy(own_plan);
 		return rc;
 	}
-	const int grid = solver_grid(k_pagerank, 32 * PR_WARPS, plan->ntiles, PR_WARPS);
+	const size_t smem = sizeof(PrWarpSmem) * PR_WARPS;
+	static std::atomic<bool> ready[64];
+	int dev = 0;
+	ALPB_CUDA(cudaGetDevice(&dev));
+	if (dev >= 64 || !ready[dev].load()) {
+		const cudaError_t e = cudaFuncSetAttribute(k_pagerank,
+			cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+		if (e != cudaSuccess) {
+			alpb_spmv_plan_destroy(own_plan);
+			set_error("alpb_pagerank: %s", cudaGetErrorString(e));
+			return ALPB_PANIC;
+		}
+		if (dev < 64) ready[dev].store(true);
+	}
+	const int sms = sm_count() < GRID_REDUCE_BLOCKS ? sm_count() : GRID_REDUCE_BLOCKS;
+	const int grid = cooperative_grid(k_pagerank, 32 * PR_WARPS, smem, sms);
 	if (grid <= 0) {
 		alpb_spmv_plan_destroy(own_plan);
 		set_error("alpb_pagerank: no cooperative occupancy");
 		return ALPB_PANIC;
 	}
-	double *vecs = work, *own_vecs = nullptr, *blk = nullptr;
+	double *vecs = work, *own_vecs = nullptr;
 	PrState *st = nullptr;
 	if (!vecs) {
 		ALPB_CUDA(cudaMallocAsync(&own_vecs, size_t(3 * n) * 8, s));
 		vecs = own_vecs;
 	}
-	ALPB_CUDA(cudaMallocAsync(&blk, size_t(5 * int64_t(grid)) * 8, s));
 	ALPB_CUDA(cudaMallocAsync(&st, sizeof(PrState), s));
 	ALPB_CUDA(cudaMemsetAsync(st, 0, sizeof(PrState), s));
 	PrArgs a;
@@ -583,7 +592,6 @@ static int pagerank_run(int64_t n, const int64_t *crs_row_ptr, const double *crs
 	a.rs = vecs;
 	a.next0 = vecs + n;
 	a.next1 = vecs + 2 * n;
-	a.blk = blk;
 	a.n = n;
 	a.max_iter = max_iter;
 	a.alpha = alpha;
@@ -597,16 +605,16 @@ static int pagerank_run(int64_t n, const int64_t *crs_row_ptr, const double *crs
 	}
 	void *args[] = {&a};
 	ALPB_CUDA(cudaLaunchCooperativeKernel((void *) k_pagerank, dim3(grid), dim3(32 * PR_WARPS), args,
-		0, s));
+		smem, s));
 	ALPB_LAUNCHED();
 	PrState h;
-	ALPB_CUDA(cudaMemcpyAsync(&h, st, sizeof(PrState), cudaMemcpyDeviceToHost, s));
-	ALPB_CUDA(cudaFreeAsync(blk, s));
+	ALPB_CUDA(cudaMemcpyAsync(&h.err, &st->err, sizeof(PrState) - offsetof(PrState, err),
+		cudaMemcpyDeviceToHost, s));
 	ALPB_CUDA(cudaFreeAsync(st, s));
 	if (own_vecs) ALPB_CUDA(cudaFreeAsync(own_vecs, s));
 	ALPB_CUDA(cudaStreamSynchronize(s));
 	alpb_spmv_plan_destroy(own_plan);
-	ALPB_CHECK(h.gs.err == 0, ALPB_PANIC, "alpb_pagerank: a grid barrier or tile wait timed out");
+	ALPB_CHECK(h.err == 0, ALPB_PANIC, "alpb_pagerank: a grid barrier or tile wait timed out");
 	*iterations = h.iterations;
 	*residual = h.residual;
 	if (!(h.residual <= conv)) {

@@ -91,31 +91,42 @@ __device__ __forceinline__ double block_sum_array(const double *a, int64_t n, do
 // 2.0 us; value-carrying slots polled by every block took 3.8 us (the polls
 // contend with the stores), pushed to every block's own lines 2.9 us, and
 // gathered and broadcast by one block 3.1 us.
+constexpr int GRID_REDUCE_BLOCKS = 256;
+constexpr int GRID_REDUCE_VALUES = 2;
 struct alignas(128) GridReduce {
 	unsigned long long count;
 	unsigned int pad[30];
-	double part[2][256];     // [epoch parity][block]
+	// [epoch parity][value][block]
+	double part[2][GRID_REDUCE_VALUES][GRID_REDUCE_BLOCKS];
 };
 
-// All threads call, with epoch = 1, 2, ... ; v: this thread's term; *sum: the
-// grid's total in a fixed order (lanes, warps, blocks), the same bits in every
-// thread.  Needs gridDim.x <= min(blockDim.x, 256), *g zeroed before the
-// launch.  Global writes of any block before the call are visible to plain
-// loads of all after it.  false: a wait gave up (*err is set).
-__device__ __forceinline__ bool grid_reduce(GridReduce *g, unsigned epoch, double v,
-	double *sum, double *smem /* >= 64 */, int *err) {
+// All threads call, with epoch = 1, 2, ... ; v: this thread's terms of NV sums;
+// sum: the grid's totals in a fixed order (lanes, warps, blocks), the same bits
+// in every thread.  Needs gridDim.x <= min(blockDim.x, GRID_REDUCE_BLOCKS), *g
+// zeroed before the launch.  Global writes of any block before the call are
+// visible to plain loads of all after it.  false: a wait gave up (*err is set).
+template <int NV>
+__device__ __forceinline__ bool grid_reduce(GridReduce *g, unsigned epoch, const double (&v)[NV],
+	double (&sum)[NV], double *smem /* >= 64 NV */, int *err) {
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 	const int nwarps = blockDim.x >> 5, G = gridDim.x;
-	double *part = g->part[epoch & 1];
-	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-	if (lane == 0) smem[w] = v;
+	double(*part)[GRID_REDUCE_BLOCKS] = g->part[epoch & 1];
+#pragma unroll
+	for (int q = 0; q < NV; ++q) {
+		double t = v[q];
+		for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+		if (lane == 0) smem[64 * q + w] = t;
+	}
 	__syncthreads();
 	int bad = 0;
 	if (w == 0) {
-		double t = lane < nwarps ? smem[lane] : 0.0;
-		for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+#pragma unroll
+		for (int q = 0; q < NV; ++q) {
+			double t = lane < nwarps ? smem[64 * q + lane] : 0.0;
+			for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+			if (lane == 0) part[q][blockIdx.x] = t;
+		}
 		if (lane == 0) {
-			part[blockIdx.x] = t;
 			unsigned long long c;
 			asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;"
 						 : "=l"(c) : "l"(&g->count) : "memory");
@@ -136,15 +147,33 @@ __device__ __forceinline__ bool grid_reduce(GridReduce *g, unsigned epoch, doubl
 	if (__syncthreads_or(bad)) return false;
 	const int gw = (G + 31) >> 5;
 	if (w < gw) {
-		double t = int(threadIdx.x) < G ? __ldcg(part + threadIdx.x) : 0.0;
-		for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-		if (lane == 0) smem[32 + w] = t;
+		double t[NV];
+#pragma unroll
+		for (int q = 0; q < NV; ++q) t[q] = int(threadIdx.x) < G ? __ldcg(part[q] + threadIdx.x) : 0.0;
+#pragma unroll
+		for (int q = 0; q < NV; ++q) {
+			for (int o = 16; o > 0; o >>= 1) t[q] += __shfl_xor_sync(0xffffffffu, t[q], o);
+			if (lane == 0) smem[64 * q + 32 + w] = t[q];
+		}
 	}
 	__syncthreads();
-	double r = 0.0;
-	for (int k = 0; k < gw; ++k) r += smem[32 + k];
-	*sum = r;
+#pragma unroll
+	for (int q = 0; q < NV; ++q) {
+		double r = 0.0;
+		for (int k = 0; k < gw; ++k) r += smem[64 * q + 32 + k];
+		sum[q] = r;
+	}
 	return true;
+}
+
+// One sum.
+__device__ __forceinline__ bool grid_reduce(GridReduce *g, unsigned epoch, double v, double *sum,
+	double *smem, int *err) {
+	const double in[1] = {v};
+	double out[1];
+	const bool ok = grid_reduce<1>(g, epoch, in, out, smem, err);
+	*sum = out[0];
+	return ok;
 }
 
 // Largest grid of `kernel` whose blocks are all co-resident.
