@@ -111,3 +111,38 @@ def test_general_path_input_bits(cuda, oracle, ring, case, n):
             np.testing.assert_allclose(got.cpu().numpy(), want, rtol=5e-11, atol=0)
         else:
             np.testing.assert_array_equal(got.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("path", ["general", "rows", "small", "merge"])
+def test_products_under_capture(cuda, path):
+    """A captured product, replayed on new inputs, gives the direct call's bits
+    (the general path takes its scratch from the stream-ordered pool)."""
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    rng = np.random.default_rng(11)
+    m = n = 40000 if path == "merge" else 5000
+    lens = np.full(m, 5) if path == "rows" else np.minimum(rng.zipf(1.7, m) * 8, 2000)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    col = rng.integers(0, n, int(lens.sum())).astype(np.uint32)
+    A = dev.from_host(m, n, rp, col, rng.random(len(col)))
+    plan = dev.Plan(A, sched=abi.SCHED_MERGE_PATH if path == "merge" else abi.SCHED_AUTO)
+    x, u = (torch.empty(k, dtype=torch.float64, device="cuda") for k in (n, m))
+    xa = torch.from_numpy((rng.random(n) < 0.3).astype(np.uint8)).cuda()
+    kw = {"v_assigned": xa, "v_count": int(xa.sum())} if path == "general" else {}
+    call = lambda: dev.mxv(0, A, u, x, plan=plan, **kw)  # noqa: E731
+    x.fill_(1.0)
+    u.fill_(0.0)
+    call()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        call()
+    for k in range(3):
+        x.copy_(torch.from_numpy(rng.random(n)))
+        u.fill_(float(k))
+        g.replay()
+        got = u.clone()
+        u.fill_(float(k))
+        call()
+        assert torch.equal(got, u)
