@@ -15,6 +15,8 @@
 //   k_hpcg_cycle<NRHS>   one V-cycle as one persistent cooperative launch: a
 //                        colour step, a restriction or a prolongation between
 //                        two grid barriers
+//   k_hpcg_rows<NRHS, Op>  the same steps as launches, on levels far larger
+//                        than L2
 //   k_hpcg_spmm<NRHS>    A p and the block partials of p . A p
 //   k_hpcg_dot, k_hpcg_axpby, k_hpcg_update   the CG vector steps, with block
 //                        partials of the dot product that follows
@@ -142,8 +144,8 @@ enum { HG_DOWN, HG_UP, HG_WHOLE };
 constexpr int HGC_THREADS = 768;
 constexpr int HGC_CLUSTER = 16;     // blocks of a cluster launch
 
-// multi_grid (multigrid_v_cycle.hpp:193-246) on the levels [l0, l1): z = 0;
-// smooth; restrict the residual; recurse; prolong; smooth.  HG_WHOLE ends at
+// multi_grid (multigrid_v_cycle.hpp:193-246) on the levels [l0, l1): z = 0 (the
+// caller's, on l0); smooth; restrict the residual; recurse; prolong; smooth.  HG_WHOLE ends at
 // the coarsest level, which smooths once; HG_DOWN stops after the restriction
 // to level l1 and HG_UP begins with the prolongation from it.  A smoother
 // (red_black_gauss_seidel.hpp:55-123) is 2 x colors steps, forward then
@@ -264,10 +266,6 @@ __global__ void __launch_bounds__(HGC_THREADS, 1) k_hpcg_cycle(HgCycleArgs a) {
 	};
 
 	if (a.part != HG_UP) {
-		if (a.l0 == 0) {
-			for (int64_t q = tid; q < a.lv[0].n * NRHS; q += nthreads) a.lv[0].z[q] = 0.0;
-			if (!barrier()) return;
-		}
 		for (int l = a.l0; l < (a.part == HG_WHOLE ? a.l1 - 1 : a.l1); ++l) {
 			const HgLevelArgs &L = a.lv[l], &C = a.lv[l + 1];
 			for (int64_t q = 0; q < a.pre; ++q)
@@ -303,6 +301,104 @@ __global__ void __launch_bounds__(HGC_THREADS, 1) k_hpcg_cycle(HgCycleArgs a) {
 		if (!barrier()) return;
 		for (int64_t q = 0; q < a.post; ++q)
 			if (!smooth(L)) return;
+	}
+}
+
+// ------------------------------------------------ large levels: launches --
+// Where x is far larger than L2 a colour step is bound by its gathers from
+// memory, and every warp that an SM can hold counts more than the loads each
+// has in flight: such levels run a launch per step, 8 lanes per row, lane
+// (s, k) of the group walking the entries s, s + S, ... of right-hand side k,
+// in 32 registers.  HG_LARGE_VALUES below says which levels these are, and the
+// times of both sides.
+constexpr int HG_GROUP = 8;     // lanes per matrix row
+template <int NRHS, class Op>
+__global__ void __launch_bounds__(HG_BLOCK)
+k_hpcg_rows(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ indices,
+	const double *__restrict__ values, const double *__restrict__ x, int64_t count, Op op) {
+	constexpr int S = HG_GROUP / NRHS;
+	constexpr int GPW = 32 / HG_GROUP;  // row groups per warp
+	const int q = threadIdx.x & (HG_GROUP - 1);
+	const int k = q % NRHS, s = q / NRHS;
+	const int g = (threadIdx.x & 31) / HG_GROUP;
+	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+	// the loop bound is the same for the whole warp, so every lane reaches
+	// every shuffle below
+	for (int64_t wb = warp * GPW; wb < count; wb += nwarps * GPW) {
+		const int64_t idx = wb + g;
+		const bool valid = idx < count;
+		double acc = 0.0;
+		int64_t row = 0;
+		if (valid) {
+			row = op.row(idx);
+			const int64_t b = offsets[row], e = offsets[row + 1];
+			for (int64_t j = b + s; j < e; j += S)
+				acc += values[j] * x[int64_t(indices[j]) * NRHS + k];
+		}
+#pragma unroll
+		for (int o = NRHS; o < HG_GROUP; o <<= 1) {
+			const double w = __shfl_xor_sync(0xffffffffu, acc, o);
+			acc += w;
+		}
+		if (valid && s == 0) op.finish(idx, row, k, acc);
+	}
+}
+
+// One colour step on rows c, c + K, ...: in place, or (temp) the products
+// first and k_hpcg_color_update after, as in the cycle kernel.
+template <int NRHS>
+struct HgColor {
+	const double *r;
+	double *x;
+	double *temp;  // null: fused
+	double d;
+	int64_t c, K;
+	__device__ __forceinline__ int64_t row(int64_t i) const { return c + i * K; }
+	__device__ __forceinline__ void finish(int64_t, int64_t row, int k, double acc) const {
+		const double t = 0.0 + acc;
+		const int64_t at = row * NRHS + k;
+		if (temp) {
+			temp[at] = t;
+		} else {
+			const double v = r[at] - t + x[at] * d;
+			x[at] = v / d;
+		}
+	}
+};
+
+template <int NRHS>
+__global__ void k_hpcg_color_update(const double *r, const double *temp, double *x, double d,
+	int64_t c, int64_t K, int64_t count) {
+	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < count * NRHS;
+		 i += int64_t(gridDim.x) * blockDim.x) {
+		const int64_t at = (c + (i / NRHS) * K) * NRHS + i % NRHS;
+		const double v = r[at] - temp[at] + x[at] * d;
+		x[at] = v / d;
+	}
+}
+
+// Restriction and prolongation, as in the cycle kernel.
+template <int NRHS>
+struct HgRestrict {
+	const double *r_f;
+	double *r_c;
+	HgInject inj;
+	__device__ __forceinline__ int64_t row(int64_t c) const { return inj(c); }
+	__device__ __forceinline__ void finish(int64_t c, int64_t f, int k, double acc) const {
+		const double ax = 0.0 + acc;
+		r_c[c * NRHS + k] = 0.0 + 1.0 * (r_f[f * NRHS + k] - ax);
+	}
+};
+
+template <int NRHS>
+__global__ void k_hpcg_prolong(double *z_f, const double *z_c, HgInject inj, int64_t count) {
+	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < count * NRHS;
+		 i += int64_t(gridDim.x) * blockDim.x) {
+		const int64_t c = i / NRHS;
+		const int k = int(i % NRHS);
+		const int64_t at = inj(c) * NRHS + k;
+		z_f[at] = z_f[at] + (0.0 + 1.0 * z_c[i]);
 	}
 }
 
@@ -557,6 +653,7 @@ struct alpb_hpcg_s {
 	HgScalars *scalars = nullptr;
 	GridSync *gs = nullptr;      // the cycle kernel's barrier
 	int32_t *active = nullptr;   // right-hand sides still iterating
+	int cluster_fits = -1;       // coarse levels in one cluster: -1 not asked yet
 	int dot_blocks = 0;
 };
 
@@ -569,6 +666,34 @@ namespace alpb {
 // the better one of each).
 constexpr int64_t HG_CLUSTER_VALUES = 32768;
 
+static void hg_cluster_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr) {
+	cfg->blockDim = dim3(HGC_THREADS);
+	cfg->gridDim = dim3(HGC_CLUSTER);
+	attr->id = cudaLaunchAttributeClusterDimension;
+	attr->val.clusterDim.x = HGC_CLUSTER;
+	attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+	cfg->attrs = attr;
+	cfg->numAttrs = 1;
+}
+
+// Whether the current device takes the cluster launch (16 blocks of one
+// cluster need as many free SMs in one GPC); asked once per handle.
+template <int NRHS>
+static bool hg_cluster_fits(alpb_hpcg_s *h) {
+	if (h->cluster_fits < 0) {
+		cudaLaunchConfig_t cfg = {};
+		cudaLaunchAttribute attr[1];
+		hg_cluster_config(&cfg, attr);
+		int n = 0;
+		const bool ok = cudaFuncSetAttribute(k_hpcg_cycle<NRHS, true>,
+			cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+			cudaOccupancyMaxActiveClusters(&n, k_hpcg_cycle<NRHS, true>, &cfg) == cudaSuccess;
+		cudaGetLastError();
+		h->cluster_fits = ok && n > 0;
+	}
+	return h->cluster_fits != 0;
+}
+
 // one launch of the cycle kernel over the levels [l0, l1)
 template <int NRHS, bool CLUSTER>
 static int hg_cycle_part(alpb_hpcg_s *h, HgCycleArgs &a, int l0, int l1, int part,
@@ -577,46 +702,87 @@ static int hg_cycle_part(alpb_hpcg_s *h, HgCycleArgs &a, int l0, int l1, int par
 	a.l1 = l1;
 	a.part = part;
 	cudaLaunchConfig_t cfg = {};
-	cfg.blockDim = dim3(HGC_THREADS);
-	cfg.stream = s;
 	cudaLaunchAttribute attr[1];
 	if (CLUSTER) {
-		static std::atomic<bool> ready[64];
-		int dev = 0;
-		ALPB_CUDA(cudaGetDevice(&dev));
-		if (dev >= 64 || !ready[dev].load()) {
-			ALPB_CUDA(cudaFuncSetAttribute(k_hpcg_cycle<NRHS, CLUSTER>,
-				cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-			if (dev < 64) ready[dev].store(true);
-		}
-		cfg.gridDim = dim3(HGC_CLUSTER);
-		attr[0].id = cudaLaunchAttributeClusterDimension;
-		attr[0].val.clusterDim.x = HGC_CLUSTER;
-		attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+		hg_cluster_config(&cfg, attr);
 	} else {
 		ALPB_CUDA(cudaMemsetAsync(&h->gs->count, 0, sizeof(h->gs->count), s));
+		cfg.blockDim = dim3(HGC_THREADS);
 		cfg.gridDim = dim3(sm_count());
 		attr[0].id = cudaLaunchAttributeCooperative;
 		attr[0].val.cooperative = 1;
+		cfg.attrs = attr;
+		cfg.numAttrs = 1;
 	}
-	cfg.attrs = attr;
-	cfg.numAttrs = 1;
+	cfg.stream = s;
 	ALPB_CUDA(cudaLaunchKernelEx(&cfg, k_hpcg_cycle<NRHS, CLUSTER>, a));
 	ALPB_LAUNCHED();
 	return ALPB_SUCCESS;
 }
 
-// one V-cycle from the finest r into the finest z
+// Levels of more values than this (256 MB of x, twice the L2) run a launch per
+// step.  The line lies between 128^3 x 8 = 2^24, where the cycle kernel takes
+// 8.4 ms per iteration and launches 9.3, and 256^3 x 8 = 2^27, where it takes
+// 55.1 and launches 52.1; sizes between were not measured.
+constexpr int64_t HG_LARGE_VALUES = int64_t(1) << 25;
+
+template <int NRHS, class Op>
+static int hg_rows(const HgLevel &L, const double *x, int64_t count, const Op &op, cudaStream_t s) {
+	if (count <= 0) return ALPB_SUCCESS;
+	k_hpcg_rows<NRHS, Op><<<grid_for(count * HG_GROUP, HG_BLOCK), HG_BLOCK, 0, s>>>(L.offsets,
+		L.indices, L.values, x, count, op);
+	ALPB_LAUNCHED();
+	return ALPB_SUCCESS;
+}
+
+// red_black_gauss_seidel: colours forward, then backward (:96-117)
 template <int NRHS>
-static int hg_vcycle(alpb_hpcg_s *h, int64_t pre, int64_t post, cudaStream_t s) {
-	HgCycleArgs a;
+static int hg_smoother(alpb_hpcg_s *h, HgLevel &L, cudaStream_t s) {
+	const int64_t K = h->colors;
+	for (int64_t step = 0; step < 2 * K; ++step) {
+		const int64_t c = step < K ? step : 2 * K - 1 - step;
+		const int64_t count = c < L.n ? (L.n - 1 - c) / K + 1 : 0;
+		HgColor<NRHS> op{L.r, L.z, L.fused ? nullptr : L.temp, h->diag, c, K};
+		const int rc = hg_rows<NRHS>(L, L.z, count, op, s);
+		if (rc != ALPB_SUCCESS) return rc;
+		if (!L.fused && count > 0) {
+			k_hpcg_color_update<NRHS><<<grid_for(count * NRHS, 256), 256, 0, s>>>(L.r, L.temp, L.z,
+				h->diag, c, K, count);
+			ALPB_LAUNCHED();
+		}
+	}
+	return ALPB_SUCCESS;
+}
+
+// multi_grid from level l down and back up again: a large level by launches,
+// the first level that is not large and those below it by the cycle kernel
+template <int NRHS>
+static int hg_vcycle(alpb_hpcg_s *h, int l, int64_t pre, int64_t post, cudaStream_t s) {
 	const int nl = int(h->levels.size());
+	HgLevel &L = h->levels[size_t(l)];
+	ALPB_CUDA(cudaMemsetAsync(L.z, 0, size_t(L.n) * NRHS * 8, s));
+	int rc = ALPB_SUCCESS;
+	if (L.n * NRHS > HG_LARGE_VALUES) {
+		if (l + 1 == nl) return hg_smoother<NRHS>(h, L, s);
+		for (int64_t i = 0; i < pre && rc == ALPB_SUCCESS; ++i) rc = hg_smoother<NRHS>(h, L, s);
+		if (rc != ALPB_SUCCESS) return rc;
+		HgLevel &C = h->levels[size_t(l) + 1];
+		const HgInject inj{C.nx, C.ny, L.nx, L.ny};
+		rc = hg_rows<NRHS>(L, L.z, C.n, HgRestrict<NRHS>{L.r, C.r, inj}, s);
+		rc = rc ? rc : hg_vcycle<NRHS>(h, l + 1, pre, post, s);
+		if (rc != ALPB_SUCCESS) return rc;
+		k_hpcg_prolong<NRHS><<<grid_for(C.n * NRHS, 256), 256, 0, s>>>(L.z, C.z, inj, C.n);
+		ALPB_LAUNCHED();
+		for (int64_t i = 0; i < post && rc == ALPB_SUCCESS; ++i) rc = hg_smoother<NRHS>(h, L, s);
+		return rc;
+	}
+	HgCycleArgs a;
 	int coarse = nl;   // first level of the cluster launch
-	for (int l = nl - 1; l >= 0; --l) {
-		const HgLevel &L = h->levels[size_t(l)];
-		a.lv[l] = HgLevelArgs{L.offsets, L.indices, L.values, L.r, L.z, L.fused ? nullptr : L.temp,
-			L.n, L.nx, L.ny};
-		if (L.n * NRHS <= HG_CLUSTER_VALUES) coarse = l;
+	for (int q = nl - 1; q >= l; --q) {
+		const HgLevel &Q = h->levels[size_t(q)];
+		a.lv[q] = HgLevelArgs{Q.offsets, Q.indices, Q.values, Q.r, Q.z, Q.fused ? nullptr : Q.temp,
+			Q.n, Q.nx, Q.ny};
+		if (Q.n * NRHS <= HG_CLUSTER_VALUES && hg_cluster_fits<NRHS>(h)) coarse = q;
 	}
 	a.colors = h->colors;
 	a.pre = pre;
@@ -624,11 +790,10 @@ static int hg_vcycle(alpb_hpcg_s *h, int64_t pre, int64_t post, cudaStream_t s) 
 	a.diag = h->diag;
 	a.gs = h->gs;
 	a.active = h->active;
-	if (coarse == nl) return hg_cycle_part<NRHS, false>(h, a, 0, nl, HG_WHOLE, s);
-	int rc = ALPB_SUCCESS;
-	if (coarse > 0) rc = hg_cycle_part<NRHS, false>(h, a, 0, coarse, HG_DOWN, s);
+	if (coarse == nl) return hg_cycle_part<NRHS, false>(h, a, l, nl, HG_WHOLE, s);
+	if (coarse > l) rc = hg_cycle_part<NRHS, false>(h, a, l, coarse, HG_DOWN, s);
 	rc = rc ? rc : hg_cycle_part<NRHS, true>(h, a, coarse, nl, HG_WHOLE, s);
-	if (coarse > 0) rc = rc ? rc : hg_cycle_part<NRHS, false>(h, a, 0, coarse, HG_UP, s);
+	if (coarse > l) rc = rc ? rc : hg_cycle_part<NRHS, false>(h, a, l, coarse, HG_UP, s);
 	return rc;
 }
 
@@ -682,9 +847,11 @@ static int hg_solve(alpb_hpcg_s *h, const double *b, double *x, bool preconditio
 	if (rc != ALPB_SUCCESS) return rc;
 	HgScalars hs[NRHS];
 	GridSync hgs;
+	// a large system's iteration is worth far more than a look at the state
+	const int64_t queue = n * NRHS > HG_LARGE_VALUES ? 1 : HG_QUEUE;
 	for (int64_t iter = 0;; ++iter) {
 		if (precondition) {
-			rc = hg_vcycle<NRHS>(h, pre, post, s);
+			rc = hg_vcycle<NRHS>(h, 0, pre, post, s);
 			if (rc != ALPB_SUCCESS) return rc;
 		} else {
 			ALPB_CUDA(cudaMemcpyAsync(L.z, L.r, size_t(n) * NRHS * 8, cudaMemcpyDeviceToDevice, s));
@@ -712,7 +879,7 @@ static int hg_solve(alpb_hpcg_s *h, const double *b, double *x, bool preconditio
 		ALPB_LAUNCHED();
 		rc = hg_finish<NRHS>(h, 3, iter, max_iter, tol, s);
 		if (rc != ALPB_SUCCESS) return rc;
-		if (iter % HG_QUEUE != HG_QUEUE - 1 && iter + 1 < max_iter) continue;
+		if (iter % queue != queue - 1 && iter + 1 < max_iter) continue;
 		ALPB_CUDA(cudaMemcpyAsync(hs, h->scalars, sizeof(hs), cudaMemcpyDeviceToHost, s));
 		ALPB_CUDA(cudaMemcpyAsync(&hgs, h->gs, sizeof(hgs), cudaMemcpyDeviceToHost, s));
 		ALPB_CUDA(cudaStreamSynchronize(s));

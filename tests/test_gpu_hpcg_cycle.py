@@ -92,6 +92,31 @@ def test_cycle_matches_restatement(cuda, dims, levels, colors, pre, post, nrhs):
     assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("colors", [27, 16])
+def test_large_level_by_launches(cuda, colors):
+    """A finest level of more than 2^25 values (a launch per step), its coarse
+    level in the cycle kernel; in place (27 colours), and with neighbours of one
+    colour (16)."""
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    dims, nrhs = (164, 164, 164), 8
+    n = int(np.prod(dims))
+    b = np.random.default_rng(colors).standard_normal((n, nrhs))
+    h = C.c_void_p()
+    abi.call("alpb_hpcg_create", C.byref(h), *dims, 26.0, -1.0, colors, 2, 1, nrhs,
+             dev.stream_ptr())
+    tb = torch.from_numpy(b.reshape(-1).copy()).cuda()
+    x = torch.zeros_like(tb)
+    it, res = (C.c_int64 * nrhs)(), (C.c_double * nrhs)()
+    abi.call("alpb_hpcg_solve", h, dev.ptr(tb), dev.ptr(x), 1, 1, 0, 1, 1e-30, it, res,
+             dev.stream_ptr())
+    abi.lib().alpb_hpcg_destroy(h)
+    want, _ = restated(dims, 1, colors, 1, 0, b, 1)
+    assert list(it) == [1] * nrhs
+    assert np.abs(x.cpu().numpy().reshape(n, nrhs) - want).max() <= 1e-12 * np.abs(want).max()
+
+
 def test_right_hand_sides_stop_on_their_own(cuda):
     """More iterations than are queued at a time; a right-hand side of a
     scaled unit vector and zero-free noise stop at their own steps, and x no
