@@ -9,8 +9,9 @@
 //    list is cut in equal tiles (Merrill & Garland, "Merge-based parallel
 //    sparse matrix-vector multiplication", SC'16), so power-law rows cost the
 //    same as uniform ones; one launch, sums in a fixed order (deterministic).
-//  * vector (general path): W lanes per row, lane-strided loads and a
-//    warp-shuffle tree; carries every ALP semantic of the reference gather:
+//  * vector: regular short rows stream through shared memory (rowstream.cuh),
+//    others take W lanes per row; the general path, W lanes per row with long
+//    rows cut in chunks, carries every ALP semantic of the reference gather:
 //    output/input masks (value or structural, inverted), sparse input and
 //    output vectors with assigned flags, add_identity, use_index,
 //    explicit_zero and the immutable-nonzero shortcut of lor.
