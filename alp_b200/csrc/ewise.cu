@@ -555,9 +555,12 @@ static int vec_chain_run(int domain, int64_t n, int nslots, void *const *values,
 	}
 	c.store = written;
 	const size_t smem = size_t(nslots) * VEC_BATCH * SCALAR_BLOCK * sizeof(T);
-	if (smem > 48 * 1024)   // seven or eight slots of 8 bytes
+	// Without the opt-in a launch has 48 KB, the kernel's own static shared memory
+	// included: six slots of 8 bytes are past it.  Every call asks for the most any
+	// chain takes, so that no thread's call lowers the limit under another's.
+	if (smem > 40 * 1024)
 		ALPB_CUDA(cudaFuncSetAttribute(k_vec_chain<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			int(smem)));
+			int(ALPB_CHAIN_SLOTS * VEC_BATCH * SCALAR_BLOCK * sizeof(T))));
 	if (!c.reduce) {
 		k_vec_chain<T><<<grid_for((n + VEC_BATCH - 1) / VEC_BATCH, SCALAR_BLOCK), SCALAR_BLOCK, smem,
 			s>>>(c, T(0), VecOut{});

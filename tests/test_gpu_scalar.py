@@ -1,6 +1,7 @@
 """Reductions to a host scalar in one launch: sizes at the edges of a thread's
 batch, of a block and of the largest grid, every monoid, an initial value, the
-scratch of several threads and streams at once, and chains of eight slots.
+scratch of several threads and streams at once, and chains of one to eight
+slots.
 
 Integers must be exact (64-bit wrap-around).  FP64 sums of n values in [0, 1)
 in two orders agree to 2 n 2^-53 of the sum."""
@@ -120,3 +121,47 @@ def test_chain_of_eight_slots(cuda, n):
     for a, b in zip(t, v):
         assert np.array_equal(a.cpu().numpy(), b)
     assert res.value == 5 + int((v[0] * v[7]).sum())
+
+
+# one to eight slots of each 8-byte domain, fewest first: a longer chain's
+# shared-memory opt-in stays with the process and would hide a missing one
+CHAINS = """
+import ctypes as C
+import numpy as np, torch
+from alp_b200 import _abi as abi
+abi.call("alpb_init", 0)
+UINT64 = 8
+n, S = 5001, abi.VecStep
+rng = np.random.default_rng(3)
+for slots in range(1, 9):
+    for domain, dt in ((abi.FP64, np.float64), (abi.INT64, np.int64), (UINT64, np.uint64)):
+        for reduce in (False, True):
+            v = [rng.integers(0, 1000, n).astype(dt) for _ in range(slots)]
+            t = [torch.from_numpy(a.view(np.int64).copy()).cuda() for a in v]
+            steps = [S(kind=abi.VEC_FOLDL, op=abi.OP_ADD, z=k, x=(k + 1) % slots, y=-1)
+                     for k in range(slots)]
+            for k in range(slots):
+                v[k] = v[k] + v[(k + 1) % slots]
+            if reduce:
+                steps.append(S(kind=abi.VEC_REDUCE, op=abi.OP_ADD, mul_op=abi.OP_MUL, z=-1, x=0, y=-1))
+            res = np.full(1, 7, dtype=dt)
+            abi.call("alpb_vec_chain", domain, n, slots,
+                     (C.c_void_p * slots)(*[a.data_ptr() for a in t]),
+                     (C.c_int * slots)(*[domain] * slots), len(steps), (S * len(steps))(*steps),
+                     C.c_void_p(res.ctypes.data), None)
+            torch.cuda.synchronize()
+            for a, b in zip(t, v):
+                assert np.array_equal(a.cpu().numpy().view(dt), b), (slots, domain, reduce)
+            # whole numbers below 2^53: FP64 sums are exact
+            assert res[0] == (7 + v[0].sum() if reduce else 7), (slots, domain, reduce)
+print("chains ok")
+"""
+
+
+def test_chains_of_every_length(cuda):
+    import subprocess
+    import sys
+    from pathlib import Path
+    p = subprocess.run([sys.executable, "-c", CHAINS], capture_output=True, text=True, timeout=300,
+                       cwd=Path(__file__).resolve().parent.parent)
+    assert p.returncode == 0 and "chains ok" in p.stdout, p.stdout + p.stderr
