@@ -55,6 +55,12 @@ inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 // number of SMs of the current device (cached per device)
 int sm_count();
 
+// Process-unique id of the calling thread's current CUDA context, 0 where it has
+// none yet.  What is remembered about a device is remembered under this id, not
+// the device's number: after cudaDeviceReset the device has another context, in
+// which no address and no kernel attribute of the old one holds.
+unsigned long long context_id();
+
 inline unsigned grid_for(int64_t work, int block, int max_blocks_per_sm = 8) {
 	int64_t g = (work + block - 1) / block;
 	int64_t cap = int64_t(sm_count()) * max_blocks_per_sm;

@@ -13,8 +13,6 @@
 #include "merge.cuh"
 #include "spmv.cuh"
 
-#include <cuda.h>
-
 #include <mutex>
 
 namespace alpb {
@@ -56,36 +54,6 @@ struct NoallocSlot {
 static std::mutex g_noalloc_mutex;
 static NoallocSlot g_noalloc_slot[kNoallocMaxDevices] = {};
 
-// Id of the calling thread's current context; 0 when there is none yet (or
-// the driver lacks cuCtxGetId).  The two driver calls are looked up through
-// the runtime, so the library does not link the driver library itself.
-typedef CUresult (*CtxGetCurrentFn)(CUcontext *);
-typedef CUresult (*CtxGetIdFn)(CUcontext, unsigned long long *);
-static unsigned long long noalloc_context_id() {
-	static CtxGetCurrentFn get_current = nullptr;
-	static CtxGetIdFn get_id = nullptr;
-	static bool looked_up = false;
-	if (!looked_up) {   // under g_noalloc_mutex
-		void *f = nullptr, *g = nullptr;
-		cudaDriverEntryPointQueryResult q1, q2;
-		if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q1) == cudaSuccess &&
-			q1 == cudaDriverEntryPointSuccess &&
-			cudaGetDriverEntryPoint("cuCtxGetId", &g, cudaEnableDefault, &q2) == cudaSuccess &&
-			q2 == cudaDriverEntryPointSuccess) {
-			get_current = reinterpret_cast<CtxGetCurrentFn>(f);
-			get_id = reinterpret_cast<CtxGetIdFn>(g);
-		}
-		(void) cudaGetLastError();
-		looked_up = true;
-	}
-	if (!get_current || !get_id) return 0;
-	CUcontext ctx = nullptr;
-	unsigned long long id = 0;
-	if (get_current(&ctx) != CUDA_SUCCESS || ctx == nullptr) return 0;
-	if (get_id(ctx, &id) != CUDA_SUCCESS) return 0;
-	return id;
-}
-
 static int noalloc_scratch(unsigned char **out) {
 	int dev = 0;
 	ALPB_CUDA(cudaGetDevice(&dev));
@@ -94,7 +62,7 @@ static int noalloc_scratch(unsigned char **out) {
 		kNoallocMaxDevices);
 	std::lock_guard<std::mutex> lock(g_noalloc_mutex);
 	NoallocSlot &slot = g_noalloc_slot[dev];
-	unsigned long long id = noalloc_context_id();
+	unsigned long long id = context_id();
 	if (id == 0 || slot.ptr == nullptr || slot.ctx_id != id) {
 		void *p = nullptr;
 		// also makes the device's primary context current if nothing had yet
@@ -105,7 +73,7 @@ static int noalloc_scratch(unsigned char **out) {
 			return ALPB_PANIC;
 		}
 		slot.ptr = static_cast<unsigned char *>(p);
-		slot.ctx_id = noalloc_context_id();   // 0 keeps the next call resolving again
+		slot.ctx_id = context_id();   // 0 keeps the next call resolving again
 	}
 	*out = slot.ptr;
 	return ALPB_SUCCESS;

@@ -3,8 +3,11 @@
 #include "common.cuh"
 #include "scalar.cuh"
 
+#include <cuda.h>
+
 #include <cstdarg>
 #include <mutex>
+#include <new>
 
 namespace alpb {
 
@@ -47,52 +50,98 @@ size_t type_size(int type) {
 	return 0;
 }
 
-// A thread's reduction scratch on each device; the destructor runs when the
-// thread ends (at process exit the runtime may already be gone: its errors are
-// of no consequence then).
+// The two driver calls are looked up through the runtime, so the library does
+// not link the driver library itself.
+unsigned long long context_id() {
+	typedef CUresult (*CtxGetCurrentFn)(CUcontext *);
+	typedef CUresult (*CtxGetIdFn)(CUcontext, unsigned long long *);
+	struct Calls {
+		CtxGetCurrentFn current = nullptr;
+		CtxGetIdFn id = nullptr;
+		Calls() {
+			void *f = nullptr, *g = nullptr;
+			cudaDriverEntryPointQueryResult q1, q2;
+			if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q1) == cudaSuccess &&
+				q1 == cudaDriverEntryPointSuccess &&
+				cudaGetDriverEntryPoint("cuCtxGetId", &g, cudaEnableDefault, &q2) == cudaSuccess &&
+				q2 == cudaDriverEntryPointSuccess) {
+				current = reinterpret_cast<CtxGetCurrentFn>(f);
+				id = reinterpret_cast<CtxGetIdFn>(g);
+			}
+			(void) cudaGetLastError();
+		}
+	};
+	static const Calls calls;
+	CUcontext ctx = nullptr;
+	unsigned long long id = 0;
+	if (!calls.id || calls.current(&ctx) != CUDA_SUCCESS || ctx == nullptr) return 0;
+	return calls.id(ctx, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+// Reduction scratch: a thread holds one per context it reduces in.  Addresses of
+// a context that is gone are forgotten, never freed: a later context may have
+// given them to somebody else.
+struct ScalarNode {
+	ScalarScratch sc;
+	ScalarNode *next = nullptr;
+};
 struct ScalarPool {
-	static constexpr int kDevices = 64;
-	ScalarScratch dev[kDevices];
+	ScalarNode *held = nullptr;
 	~ScalarPool() {
-		for (int d = 0; d < kDevices; ++d) {
-			if (dev[d].part) cudaFree(dev[d].part);
-			if (dev[d].host) cudaFreeHost(dev[d].host);
+		const unsigned long long ctx = context_id();
+		while (held) {
+			ScalarNode *n = held;
+			held = n->next;
+			if (ctx != 0 && n->sc.ctx == ctx) {
+				cudaFree(n->sc.part);
+				cudaFreeHost(n->sc.host);
+			}
+			delete n;
 		}
 	}
 };
 static thread_local ScalarPool t_scalar;
 
 int scalar_scratch(ScalarScratch *out, cudaStream_t s) {
-	int d = 0;
-	ALPB_CUDA(cudaGetDevice(&d));
-	ALPB_CHECK(d < ScalarPool::kDevices, ALPB_UNSUPPORTED, "device ordinal %d", d);
-	ScalarScratch &p = t_scalar.dev[d];
-	if (!p.part) {
-		// allocations of a first call must not disturb a capture that another
-		// thread has under way
-		cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-		cudaThreadExchangeStreamCaptureMode(&mode);
-		ScalarScratch n;
-		const size_t bytes = size_t(SCALAR_MAX_BLOCKS) * 8 + 8;
-		cudaError_t e = cudaMalloc(&n.part, bytes);
-		if (e == cudaSuccess) e = cudaMemsetAsync(n.part, 0, bytes, s);
-		if (e == cudaSuccess)
-			e = cudaHostAlloc(reinterpret_cast<void **>(&n.host), 64, cudaHostAllocMapped);
-		if (e == cudaSuccess)
-			e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&n.host_dev), n.host, 0);
-		if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-		cudaThreadExchangeStreamCaptureMode(&mode);
-		if (e != cudaSuccess) {
-			cudaGetLastError();
-			if (n.part) cudaFree(n.part);
-			if (n.host) cudaFreeHost(n.host);
-			set_error("reduction scratch: %s", cudaGetErrorString(e));
-			return e == cudaErrorMemoryAllocation ? ALPB_OUTOFMEM : ALPB_PANIC;
-		}
-		n.arrived = reinterpret_cast<unsigned *>(n.part + SCALAR_MAX_BLOCKS);
-		p = n;
+	unsigned long long ctx = context_id();
+	if (ctx == 0) {
+		ALPB_CUDA(cudaFree(nullptr));   // makes the device's primary context current
+		ctx = context_id();
 	}
-	*out = p;
+	for (const ScalarNode *p = t_scalar.held; p; p = p->next)
+		if (p->sc.ctx == ctx) {
+			*out = p->sc;
+			return ALPB_SUCCESS;
+		}
+	ScalarNode *node = new (std::nothrow) ScalarNode;
+	ALPB_CHECK(node, ALPB_OUTOFMEM, "reduction scratch: out of host memory");
+	ScalarScratch &n = node->sc;
+	n.ctx = ctx;
+	// allocations of a first call must not disturb a capture that another thread
+	// has under way
+	cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+	cudaThreadExchangeStreamCaptureMode(&mode);
+	const size_t bytes = size_t(SCALAR_MAX_BLOCKS) * 8 + 8;
+	cudaError_t e = cudaMalloc(&n.part, bytes);
+	if (e == cudaSuccess) e = cudaMemsetAsync(n.part, 0, bytes, s);
+	if (e == cudaSuccess)
+		e = cudaHostAlloc(reinterpret_cast<void **>(&n.host), 64, cudaHostAllocMapped);
+	if (e == cudaSuccess)
+		e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&n.host_dev), n.host, 0);
+	if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+	cudaThreadExchangeStreamCaptureMode(&mode);
+	if (e != cudaSuccess) {
+		cudaGetLastError();
+		if (n.part) cudaFree(n.part);
+		if (n.host) cudaFreeHost(n.host);
+		delete node;
+		set_error("reduction scratch: %s", cudaGetErrorString(e));
+		return e == cudaErrorMemoryAllocation ? ALPB_OUTOFMEM : ALPB_PANIC;
+	}
+	n.arrived = reinterpret_cast<unsigned *>(n.part + SCALAR_MAX_BLOCKS);
+	node->next = t_scalar.held;
+	t_scalar.held = node;
+	*out = n;
 	return ALPB_SUCCESS;
 }
 

@@ -5,8 +5,8 @@
 // pass over them but what came after it: a second launch whose one thread
 // walked the partials (24 us for 489 of them), an allocation and a release,
 // and two copies.  The entry points wait for the stream before they return,
-// so their scratch is the calling thread's own and is kept: 8 KB on each
-// device the thread uses, released when the thread ends.
+// so their scratch is the calling thread's own and is kept: 8 KB in each
+// context the thread uses, released when the thread ends.
 #pragma once
 #include "common.cuh"
 
@@ -18,13 +18,14 @@ constexpr int SCALAR_BLOCK = 256;
 constexpr int SCALAR_MAX_BLOCKS = 1000;   // partials that fit the scratch
 
 struct ScalarScratch {
+	unsigned long long ctx = 0;     // context_id() of the context it lives in
 	uint64_t *part = nullptr;       // [SCALAR_MAX_BLOCKS] on the device
 	unsigned *arrived = nullptr;    // zero between calls
 	uint64_t *host = nullptr;       // the result, as the host reads it
 	uint64_t *host_dev = nullptr;   // and as the kernel writes it
 };
 
-// The calling thread's scratch on the current device (runtime.cu).
+// The calling thread's scratch in the current context (runtime.cu).
 int scalar_scratch(ScalarScratch *out, cudaStream_t s);
 
 // Blocks of a reduction over n entries: four entries per thread (one batch of
