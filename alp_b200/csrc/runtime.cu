@@ -78,29 +78,51 @@ unsigned long long context_id() {
 	return calls.id(ctx, &id) == CUDA_SUCCESS ? id : 0;
 }
 
-// Reduction scratch: a thread holds one per context it reduces in.  Addresses of
-// a context that is gone are forgotten, never freed: a later context may have
-// given them to somebody else.
+// Reduction scratch: a thread holds one per context it reduces in.  A thread that
+// ends leaves them for the threads after it, without a call to the runtime (a
+// release would invalidate a capture that another thread has under way), so there
+// are never more than the threads that reduced at the same time; alpb_finalize
+// gives back those of its context that no thread holds.  Addresses of a context
+// that is gone are forgotten, never freed: a later context may have given them
+// to somebody else.
 struct ScalarNode {
 	ScalarScratch sc;
 	ScalarNode *next = nullptr;
 };
+static std::mutex g_scalar_mutex;
+static ScalarNode *g_scalar_left = nullptr;   // what ended threads left
 struct ScalarPool {
 	ScalarNode *held = nullptr;
-	~ScalarPool() {
-		const unsigned long long ctx = context_id();
-		while (held) {
-			ScalarNode *n = held;
-			held = n->next;
-			if (ctx != 0 && n->sc.ctx == ctx) {
-				cudaFree(n->sc.part);
-				cudaFreeHost(n->sc.host);
-			}
-			delete n;
-		}
+	~ScalarPool() { leave(); }
+	void leave() {
+		if (!held) return;
+		ScalarNode *last = held;
+		while (last->next) last = last->next;
+		std::lock_guard<std::mutex> lock(g_scalar_mutex);
+		last->next = g_scalar_left;
+		g_scalar_left = held;
+		held = nullptr;
 	}
 };
 static thread_local ScalarPool t_scalar;
+
+// A node of context ctx that an ended thread left, or null.
+static ScalarNode *scalar_left(unsigned long long ctx) {
+	std::lock_guard<std::mutex> lock(g_scalar_mutex);
+	for (ScalarNode **p = &g_scalar_left; *p; p = &(*p)->next)
+		if ((*p)->sc.ctx == ctx) {
+			ScalarNode *n = *p;
+			*p = n->next;
+			return n;
+		}
+	return nullptr;
+}
+
+static void scalar_release(ScalarNode *n) {
+	if (n->sc.part) cudaFree(n->sc.part);
+	if (n->sc.host) cudaFreeHost(n->sc.host);
+	delete n;
+}
 
 int scalar_scratch(ScalarScratch *out, cudaStream_t s) {
 	unsigned long long ctx = context_id();
@@ -113,7 +135,14 @@ int scalar_scratch(ScalarScratch *out, cudaStream_t s) {
 			*out = p->sc;
 			return ALPB_SUCCESS;
 		}
-	ScalarNode *node = new (std::nothrow) ScalarNode;
+	ScalarNode *node = scalar_left(ctx);
+	if (node) {
+		node->next = t_scalar.held;
+		t_scalar.held = node;
+		*out = node->sc;
+		return ALPB_SUCCESS;
+	}
+	node = new (std::nothrow) ScalarNode;
 	ALPB_CHECK(node, ALPB_OUTOFMEM, "reduction scratch: out of host memory");
 	ScalarScratch &n = node->sc;
 	n.ctx = ctx;
@@ -129,12 +158,12 @@ int scalar_scratch(ScalarScratch *out, cudaStream_t s) {
 	if (e == cudaSuccess)
 		e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&n.host_dev), n.host, 0);
 	if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-	cudaThreadExchangeStreamCaptureMode(&mode);
 	if (e != cudaSuccess) {
 		cudaGetLastError();
-		if (n.part) cudaFree(n.part);
-		if (n.host) cudaFreeHost(n.host);
-		delete node;
+		scalar_release(node);
+	}
+	cudaThreadExchangeStreamCaptureMode(&mode);
+	if (e != cudaSuccess) {
 		set_error("reduction scratch: %s", cudaGetErrorString(e));
 		return e == cudaErrorMemoryAllocation ? ALPB_OUTOFMEM : ALPB_PANIC;
 	}
@@ -176,6 +205,8 @@ int alpb_init(int device) {
 
 int alpb_finalize(void) {
 	ALPB_CUDA(cudaDeviceSynchronize());
+	t_scalar.leave();
+	while (ScalarNode *n = scalar_left(context_id())) scalar_release(n);
 	return ALPB_SUCCESS;
 }
 

@@ -6,7 +6,7 @@
 // walked the partials (24 us for 489 of them), an allocation and a release,
 // and two copies.  The entry points wait for the stream before they return,
 // so their scratch is the calling thread's own and is kept: 8 KB in each
-// context the thread uses, released when the thread ends.
+// context the thread uses, left to the next thread when it ends.
 #pragma once
 #include "common.cuh"
 

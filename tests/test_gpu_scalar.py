@@ -96,6 +96,52 @@ def test_threads_and_streams(cuda):
     assert not bad
 
 
+def test_thread_ends_during_a_capture(cuda):
+    """A thread that has reduced ends while another captures: the capture is
+    whole, and the next thread reduces in what the first one left."""
+    import time
+
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    x = torch.arange(5000, device="cuda", dtype=torch.float64)
+    torch.cuda.synchronize()
+    reduced, go, got = threading.Event(), threading.Event(), []
+
+    def work():
+        torch.cuda.set_device(0)
+        d = C.c_double(0.0)
+        abi.call("alpb_reduce_f64", C.byref(d), abi.OP_ADD, x.numel(), dev.ptr(x), None,
+                 C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        got.append(d.value)
+        reduced.set()
+        go.wait(60)
+
+    t = threading.Thread(target=work)
+    t.start()
+    assert reduced.wait(60)
+    y = torch.zeros(5000, device="cuda", dtype=torch.float64)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="global"):
+        abi.call("alpb_foldl_f64", dev.ptr(y), abi.OP_ADD, y.numel(), dev.ptr(x), 0.0,
+                 dev.stream_ptr())
+        go.set()
+        t.join()
+        time.sleep(0.5)     # the thread's own storage goes after join() returns
+        abi.call("alpb_foldl_f64", dev.ptr(y), abi.OP_ADD, y.numel(), dev.ptr(x), 0.0,
+                 dev.stream_ptr())
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, 2 * x)
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert got == [5000 * 4999 / 2] * 2
+    abi.call("alpb_finalize")
+    work()
+    assert got[2] == got[0]
+
+
 @pytest.mark.parametrize("n", [1, 1025, 300001])
 def test_chain_of_eight_slots(cuda, n):
     import torch
