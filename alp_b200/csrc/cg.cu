@@ -274,14 +274,8 @@ static CgRowsShape cg_rows_shape(int64_t n, int maxlen) {
 template <int L>
 static int cg_rows_solve(const CgRowsShape &c, CgRowsArgs a, double *wk, cudaStream_t s,
 	CgState *h) {
-	static std::atomic<bool> ready[64];
-	int dev = 0;
-	ALPB_CUDA(cudaGetDevice(&dev));
-	if (dev >= 64 || !ready[dev].load()) {
-		ALPB_CUDA(cudaFuncSetAttribute(k_cg_rows<L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			CGR_SMEM));
-		if (dev < 64) ready[dev].store(true);
-	}
+	static std::atomic<unsigned long long> allowed_in;
+	ALPB_CUDA(allow_smem(k_cg_rows<L>, CGR_SMEM, allowed_in));
 	const int64_t n = a.n;
 	const size_t ell = size_t(c.grid) * size_t(c.items - c.resident) * size_t(c.steps) * 32;
 	// one allocation: state, partials, the items outside shared memory, r

@@ -61,6 +61,18 @@ int sm_count();
 // which no address and no kernel attribute of the old one holds.
 unsigned long long context_id();
 
+// Lets `kernel` take up to `bytes` of dynamic shared memory (one value per
+// kernel); `in` holds the context in which that was last set.
+template <class K>
+inline cudaError_t allow_smem(K *kernel, size_t bytes, std::atomic<unsigned long long> &in) {
+	const unsigned long long ctx = context_id();
+	if (ctx != 0 && in.load() == ctx) return cudaSuccess;
+	const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		int(bytes));
+	if (e == cudaSuccess) in.store(ctx);
+	return e;
+}
+
 inline unsigned grid_for(int64_t work, int block, int max_blocks_per_sm = 8) {
 	int64_t g = (work + block - 1) / block;
 	int64_t cap = int64_t(sm_count()) * max_blocks_per_sm;

@@ -553,18 +553,12 @@ static int pagerank_run(int64_t n, const int64_t *crs_row_ptr, const double *crs
 		return rc;
 	}
 	const size_t smem = sizeof(PrWarpSmem) * PR_WARPS;
-	static std::atomic<bool> ready[64];
-	int dev = 0;
-	ALPB_CUDA(cudaGetDevice(&dev));
-	if (dev >= 64 || !ready[dev].load()) {
-		const cudaError_t e = cudaFuncSetAttribute(k_pagerank,
-			cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-		if (e != cudaSuccess) {
-			alpb_spmv_plan_destroy(own_plan);
-			set_error("alpb_pagerank: %s", cudaGetErrorString(e));
-			return ALPB_PANIC;
-		}
-		if (dev < 64) ready[dev].store(true);
+	static std::atomic<unsigned long long> allowed_in;
+	const cudaError_t allowed = allow_smem(k_pagerank, smem, allowed_in);
+	if (allowed != cudaSuccess) {
+		alpb_spmv_plan_destroy(own_plan);
+		set_error("alpb_pagerank: %s", cudaGetErrorString(allowed));
+		return ALPB_PANIC;
 	}
 	const int sms = sm_count() < GRID_REDUCE_BLOCKS ? sm_count() : GRID_REDUCE_BLOCKS;
 	const int grid = cooperative_grid(k_pagerank, 32 * PR_WARPS, smem, sms);

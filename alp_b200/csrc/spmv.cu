@@ -1016,14 +1016,8 @@ int launch_vector_general_w(const SpmvArgs &a, const alpb_spmv_plan_s *p, cudaSt
 	}
 	const int64_t items = g.nchunks + (a.m_out + RPW - 1) / RPW;
 	if (bits) {
-		static std::atomic<bool> ready[64];
-		int dev = 0;
-		ALPB_CUDA(cudaGetDevice(&dev));
-		if (dev >= 64 || !ready[dev].load()) {
-			ALPB_CUDA(cudaFuncSetAttribute(k_spmv_vector_general<R, W, true>,
-				cudaFuncAttributeMaxDynamicSharedMemorySize, int(GEN_BITS_MAX / 8)));
-			if (dev < 64) ready[dev].store(true);
-		}
+		static std::atomic<unsigned long long> allowed_in;
+		ALPB_CUDA(allow_smem(k_spmv_vector_general<R, W, true>, GEN_BITS_MAX / 8, allowed_in));
 		k_pack_present<<<grid_for(a.n_in, 256), 256, 0, s>>>(a, bits);
 		ALPB_LAUNCHED();
 		k_spmv_vector_general<R, W, true><<<grid_for(items * 32, 1024, 1), 1024, bit_bytes, s>>>(a,
@@ -1095,14 +1089,8 @@ static int launch_rows_as(const SpmvArgs &a, int maxlen, cudaStream_t s) {
 	constexpr size_t room = 220 * 1024;
 	int warps = int(room / warp);
 	if (warps > RS_MAX_WARPS) warps = RS_MAX_WARPS;
-	static std::atomic<bool> ready[64];
-	int dev = 0;
-	ALPB_CUDA(cudaGetDevice(&dev));
-	if (dev >= 64 || !ready[dev].load()) {
-		ALPB_CUDA(cudaFuncSetAttribute(k_spmv_rows<R, L, RPL, U>,
-			cudaFuncAttributeMaxDynamicSharedMemorySize, int(room)));
-		if (dev < 64) ready[dev].store(true);
-	}
+	static std::atomic<unsigned long long> allowed_in;
+	ALPB_CUDA(allow_smem(k_spmv_rows<R, L, RPL, U>, room, allowed_in));
 	const int64_t chunks = (a.m_out + ROWS - 1) / ROWS;
 	const int64_t grid = chunks < sm_count() ? chunks : sm_count();
 	const int64_t per = (chunks + grid - 1) / grid;   // chunks of one block

@@ -49,6 +49,47 @@ def reductions():
     return [t.value for t in (d, r, v, c)]
 """
 
+SOLVERS = """
+def stencil(sizes):
+    sz, nnz, m = (C.c_int64 * 4)(*sizes), C.c_int64(), int(np.prod(sizes))
+    off = up(np.zeros(m + 1, np.int64))
+    abi.call("alpb_gen_stencil_crs", 3, sz, 26.0, -1.0, 1, off, None, None, C.byref(nnz), None)
+    idx, val = up(np.zeros(nnz.value, np.uint32)), up(np.zeros(nnz.value))
+    abi.call("alpb_gen_stencil_crs", 3, sz, 26.0, -1.0, 1, off, idx, val, C.byref(nnz), None)
+    return m, nnz.value, off, idx, val
+
+def solvers():
+    out = []
+    m, nnz, off, idx, val = stencil((21, 17, 19))
+    for sched in (abi.SCHED_AUTO, abi.SCHED_MERGE_PATH):    # rows streamed; merge path
+        plan = C.c_void_p()
+        abi.call("alpb_spmv_plan_create", C.byref(plan), m, nnz, off, sched, 0, None)
+        y = up(np.zeros(m))
+        abi.call("alpb_mxv", 0, 0, 2, m, m, nnz, off, idx, val, abi.FP64, y, None, None, None, None,
+                 abi.BOOL, -1, up(X[:m].copy()), None, m, None, None, abi.BOOL, -1, plan, None)
+        out.append(down(y, np.zeros(m)))
+    x, it, res = up(np.zeros(m)), C.c_int64(), C.c_double()
+    abi.call("alpb_cg_solve", m, off, idx, val, up(X[:m].copy()), x, 1000, 1e-8, C.byref(it),
+             C.byref(res), None, plan, None)
+    out += [down(x, np.zeros(m)), it.value, res.value]
+    abi.lib().alpb_spmv_plan_destroy(plan)
+    # the stencil is symmetric: its CRS is its CCS
+    p = up(np.zeros(m))
+    abi.call("alpb_pagerank", m, off, idx, None, off, idx, None, p, 0, 0.85, 1e-3, 200, C.byref(it),
+             C.byref(res), None)
+    out += [down(p, np.zeros(m)), it.value, res.value]
+    # a sparse input over more than 2^21 nonzeroes, its flags asked in shared memory
+    m, nnz, off, idx, val = stencil((48, 48, 48))
+    va = (np.arange(m) % 3 == 0).astype(np.uint8)
+    plan, y = C.c_void_p(), up(np.zeros(m))
+    abi.call("alpb_spmv_plan_create", C.byref(plan), m, nnz, off, abi.SCHED_AUTO, 0, None)
+    abi.call("alpb_mxv", 0, 0, 2, m, m, nnz, off, idx, val, abi.FP64, y, None, None, None, None,
+             abi.BOOL, -1, up(np.arange(m) / 7.0), up(va), int(va.sum()), None, None, abi.BOOL, -1,
+             plan, None)
+    abi.lib().alpb_spmv_plan_destroy(plan)
+    return out + [down(y, np.zeros(m))]
+"""
+
 SECOND = """
 abi.call("alpb_init", 0)
 first = work()
@@ -85,3 +126,8 @@ def run(work, program):
 @pytest.mark.parametrize("program", [SECOND, RESET], ids=["second", "reset"])
 def test_reductions(cuda, program):
     run("work = reductions\n", program)
+
+
+@pytest.mark.parametrize("program", [SECOND, RESET], ids=["second", "reset"])
+def test_products_and_solvers(cuda, program):
+    run(SOLVERS + "work = solvers\n", program)
