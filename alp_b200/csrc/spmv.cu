@@ -1127,7 +1127,7 @@ static int regular_width(double mean) {
 }
 
 template <class R>
-int run_spmv(const SpmvArgs &a, const alpb_spmv_plan_s *p, int force_sched, cudaStream_t s) {
+int run_spmv(const SpmvArgs &a, const alpb_spmv_plan_s *plan, int force_sched, cudaStream_t s) {
 	if (a.trivial) {
 		if (a.descr & ALPB_DESC_EXPLICIT_ZERO) {
 			k_spmv_trivial<R><<<grid_for(a.m_out, 256), 256, 0, s>>>(a);
@@ -1137,11 +1137,14 @@ int run_spmv(const SpmvArgs &a, const alpb_spmv_plan_s *p, int force_sched, cuda
 	}
 	const bool fast = a.dense_all && !a.masked && !a.input_masked &&
 		!(a.descr & (ALPB_DESC_ADD_IDENTITY | ALPB_DESC_USE_INDEX));
+	// A plan's tables and lists are those of the offsets it was made from: with
+	// others of the same sizes only its lane width is taken.
+	const alpb_spmv_plan_s *p = plan && plan->offsets == a.offsets ? plan : nullptr;
 	if constexpr (std::is_same<R, RingLorLandBool>::value) {
 		if (fast && !force_sched && p && p->lor_n >= 0) return launch_lor(a, *p, s);
 	}
 	int sched = force_sched ? force_sched : (p ? p->sched : ALPB_SCHED_VECTOR);
-	int W = p ? p->vw : default_width(a.m_out ? double(a.nnz) / double(a.m_out) : 1.0);
+	int W = plan ? plan->vw : default_width(a.m_out ? double(a.nnz) / double(a.m_out) : 1.0);
 	if (fast && sched == ALPB_SCHED_MERGE_PATH && p && p->tile_row) {
 		if (p->small && p->lor_n >= 0 && !p->hot_on) return launch_small<R>(a, *p, s);
 		return launch_merge<R>(a, *p, s);

@@ -252,7 +252,9 @@ ALPB_API int alpb_gen_normal(double *out, int64_t count, uint64_t seed, uint64_t
  * grb::mxv / grb::vxm overloads, blas2.hpp:1532-2230)
  * ====================================================================== */
 /* Analyse a compressed storage (row lengths: mean, max, CV), choose a
- * schedule (sched = ALPB_SCHED_AUTO) and precompute its tile table. */
+ * schedule (sched = ALPB_SCHED_AUTO) and precompute its tile table.  The plan
+ * serves products over this offsets array; alpb_mxv over another one of the
+ * same m and nnz takes its lane width only (vector schedule). */
 ALPB_API int alpb_spmv_plan_create(alpb_spmv_plan *plan, int64_t m, int64_t nnz,
 	const int64_t *offsets, int sched, int vector_width, void *stream);
 ALPB_API int alpb_spmv_plan_destroy(alpb_spmv_plan plan);

@@ -1,0 +1,84 @@
+"""Products with a plan that does not describe their storage, and what a plan
+remembers from one tuning to the next.  Results are compared with the plain
+sums in numpy: rows of up to n positive FP64 terms in two orders agree to
+2 n 2^-53 relative, whole numbers exactly."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def lengths(kind, m, rng):
+    if kind == "regular":
+        return np.full(m, 5)
+    k = np.minimum(rng.zipf(1.6, m), 4000)
+    k[:3] = 4000, 300, 65
+    return k
+
+
+def reshaped(lens, rng):
+    """another structure of the same number of rows and nonzeroes: its rows in
+    another order, then half of each of the first rows moved to one of them"""
+    other = rng.permutation(lens)
+    cut = other[:400] // 2
+    other[:400] -= cut
+    other[401] += cut.sum()
+    return other
+
+
+def storage(lens, n, rng):
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    return rp, rng.integers(0, n, int(rp[-1])).astype(np.uint32)
+
+
+def check(A, rp, col, vals, plan, rng, sparse):
+    import torch
+    from alp_b200 import device as dev
+    m, n = A.m, A.n
+    x, u = rng.random(n), rng.random(m)
+    xa = (rng.random(n) < 0.4).astype(np.uint8)
+    got = torch.from_numpy(u.copy()).cuda()
+    kw = {"v_assigned": torch.from_numpy(xa).cuda()} if sparse else {}
+    dev.mxv(0, A, got, torch.from_numpy(x).cuda(), plan=plan, **kw)
+    terms = vals * x[col] * (xa[col] if sparse else 1)
+    want = u.copy()
+    np.add.at(want, np.repeat(np.arange(m), np.diff(rp)), terms)
+    tol = 2 * np.diff(rp).max() * 2.0 ** -53
+    np.testing.assert_allclose(got.cpu().numpy(), want, rtol=tol, atol=0)
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+@pytest.mark.parametrize("kind,m", [("regular", 4000), ("regular", 500000), ("skewed", 4000),
+                                    ("skewed", 500000)])
+def test_plan_of_another_storage(cuda, kind, m, sparse):
+    from alp_b200 import device as dev
+    rng = np.random.default_rng([m, sparse])
+    n, lens = 70001, lengths(kind, m, rng)
+    rp, col = storage(lens, n, rng)
+    rp2, col2 = storage(reshaped(lens, rng), n, rng)
+    vals = rng.random(len(col))
+    A, B = dev.from_host(m, n, rp, col, vals), dev.from_host(m, n, rp2, col2, vals)
+    assert A.nnz == B.nnz
+    for sched in (0, 1, 2):
+        plan = dev.Plan(A, sched=sched)
+        check(A, rp, col, vals, plan, rng, sparse)
+        check(B, rp2, col2, vals, plan, rng, sparse)
+        check(A, rp, col, vals, plan, rng, sparse)
+
+
+def test_boolean_plan_of_another_storage(cuda):
+    import torch
+    from alp_b200 import device as dev
+    rng = np.random.default_rng(2)
+    m, n, lens = 4000, 70001, lengths("skewed", 4000, rng)
+    rp, col = storage(lens, n, rng)
+    rp2, col2 = storage(reshaped(lens, rng), n, rng)
+    A, B = dev.from_host(m, n, rp, col, None, 0), dev.from_host(m, n, rp2, col2, None, 0)
+    plan = dev.Plan(A)
+    x = (rng.random(n) < 0.01).astype(np.uint8)
+    for M, o, c in ((A, rp, col), (B, rp2, col2)):
+        u = torch.zeros(m, dtype=torch.uint8, device="cuda")
+        dev.mxv(1, M, u, torch.from_numpy(x).cuda(), plan=plan)
+        want = np.zeros(m, np.uint8)
+        np.maximum.at(want, np.repeat(np.arange(m), np.diff(o)), x[c])
+        assert np.array_equal(u.cpu().numpy(), want)
