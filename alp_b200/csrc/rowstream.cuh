@@ -23,6 +23,7 @@ namespace alpb {
 constexpr int RS_STAGES = 2;
 constexpr int RS_MAX_LEN = 64;       // longest row taken
 constexpr int RS_MAX_WARPS = 24;
+constexpr int RS_SLACK = 32;         // see rs_cap
 
 __device__ __forceinline__ void rs_copy16(void *dst, const void *src, int bytes) {
 	const unsigned d = unsigned(__cvta_generic_to_shared(dst));
@@ -84,8 +85,14 @@ k_spmv_rows(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ in
 			t = offsets[(c + 1) * ROWS < m ? (c + 1) * ROWS : m];
 		}
 	};
+	// A chunk of more nonzeroes than a stage holds (offsets that changed after
+	// the plan took their longest row) is not copied, but read where it stands.
+	unsigned direct = 0;   // a bit per stage
 	const auto fetch = [&](int64_t c, int s) {
-		if (c < chunks) {
+		direct &= ~(1u << s);
+		if (c < chunks && t - b > cap - RS_SLACK) {
+			direct |= 1u << s;
+		} else if (c < chunks) {
 			unsigned char *d = mine + s * stage;
 			if (values)
 				rs_fetch(d, values, b * int64_t(sizeof(T)), t * int64_t(sizeof(T)),
@@ -130,6 +137,14 @@ k_spmv_rows(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ in
 #pragma unroll
 		for (int r = 0; r < RPL; ++r) {
 			T acc = R::zero();
+			if (direct >> s & 1u) {
+				for (int q = k; q < len[r]; q += L) {
+					const T a = values ? values[ob[r] + q] : R::one();
+					const T xv = __ldg(x + indices[ob[r] + q]);
+					acc = R::add(acc, left ? R::mull(xv, a) : R::mulr(a, xv));
+				}
+				len[r] = len[r] > 0 ? -1 : 0;   // summed
+			}
 			for (int q0 = k; q0 < len[r]; q0 += U * L) {
 				T xv[U], part = R::zero();
 #pragma unroll
@@ -145,7 +160,7 @@ k_spmv_rows(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ in
 			}
 #pragma unroll
 			for (int d = 1; d < L; d <<= 1) acc = R::add(acc, __shfl_xor_sync(0xffffffffu, acc, d));
-			if (k == 0 && len[r] > 0) y[c * ROWS + r * H + sub] = R::add(yv[r], acc);
+			if (k == 0 && len[r] != 0) y[c * ROWS + r * H + sub] = R::add(yv[r], acc);
 		}
 		s = s + 1 == RS_STAGES ? 0 : s + 1;
 	}
@@ -156,7 +171,7 @@ k_spmv_rows(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ in
 // its first byte down and its last up to 16 (1-byte values: 15 entries each).
 template <class R>
 inline int rs_cap(int rows, int maxlen) {
-	return (rows * maxlen + 32 + 15) / 16 * 16;
+	return (rows * maxlen + RS_SLACK + 15) / 16 * 16;
 }
 
 } // namespace alpb

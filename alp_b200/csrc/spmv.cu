@@ -437,12 +437,16 @@ k_lor_tail(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ ind
 // One chunk list of the plan: per row of more than `longer` nonzeroes, its
 // nonzeroes from `head` on in chunks of `chunk`, consecutive in the list at a
 // position taken from *count (any order of the rows: no result depends on
-// it); first, when given, lists each row's first chunk at a position from
-// *nrows.  rows == nullptr: count only.
+// it); first and number, when given, list each row's first chunk and its chunks
+// at a position from *nrows, listed marks the row.  rows == nullptr: count only.
 struct ChunkList {
 	int64_t longer, head, chunk;
 	unsigned long long *count, *nrows;
-	int64_t *rows, *k0s, *first;
+	int64_t *rows, *k0s;
+	// the general path's list only: chunks are named by their number in the row
+	// (k0s) instead of a place in the storage
+	int64_t *first, *number;
+	uint32_t *listed;
 };
 __device__ __forceinline__ void add_row_chunks(const ChunkList &l, int64_t i, int64_t o, int64_t e) {
 	if (e - o <= l.longer) return;
@@ -452,9 +456,13 @@ __device__ __forceinline__ void add_row_chunks(const ChunkList &l, int64_t i, in
 	if (!l.rows) return;
 	for (int64_t c = 0; c < n; ++c) {
 		l.rows[at + c] = i;
-		l.k0s[at + c] = b + c * l.chunk;
+		l.k0s[at + c] = l.first ? c : b + c * l.chunk;
 	}
-	if (l.first) l.first[r] = int64_t(at);
+	if (l.first) {
+		l.first[r] = int64_t(at);
+		l.number[r] = n;
+		atomicOr(l.listed + (i >> 5), 1u << (i & 31));
+	}
 }
 __global__ void k_row_chunks(const int64_t *__restrict__ offsets, int64_t m, ChunkList p,
 	ChunkList q) {
@@ -470,9 +478,12 @@ static void lists_release(alpb_spmv_plan_s *p) {
 	cudaFree(p->lor_row);
 	cudaFree(p->lor_k0);
 	cudaFree(p->gen_row);
-	cudaFree(p->gen_k0);
+	cudaFree(p->gen_c);
 	cudaFree(p->gen_first);
-	p->lor_row = p->lor_k0 = p->gen_row = p->gen_k0 = p->gen_first = nullptr;
+	cudaFree(p->gen_number);
+	cudaFree(p->gen_listed);
+	p->lor_row = p->lor_k0 = p->gen_row = p->gen_c = p->gen_first = p->gen_number = nullptr;
+	p->gen_listed = nullptr;
 	p->lor_n = -1;
 	p->gen_n = p->gen_rows = 0;
 }
@@ -486,11 +497,12 @@ static int lists_build(alpb_spmv_plan_s *p, cudaStream_t s) {
 		return ALPB_SUCCESS;
 	}
 	const unsigned grid = grid_for(p->m, 256, 4);
+	const size_t listed = size_t(p->m + 31) / 32 * 4;
 	unsigned long long *cnt = nullptr, h[4] = {0, 0, 0, 0};  // lor chunks, rows; general chunks, rows
 	ALPB_CUDA(cudaMallocAsync(&cnt, sizeof(h), s));
 	ALPB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(h), s));
-	ChunkList lor{LOR_HEAD, LOR_HEAD, LOR_CHUNK, cnt, cnt + 1, nullptr, nullptr, nullptr};
-	ChunkList gen{GEN_LONG, 0, GEN_CHUNK, cnt + 2, cnt + 3, nullptr, nullptr, nullptr};
+	ChunkList lor{LOR_HEAD, LOR_HEAD, LOR_CHUNK, cnt, cnt + 1};
+	ChunkList gen{GEN_LONG, 0, GEN_CHUNK, cnt + 2, cnt + 3};
 	k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, lor, gen);
 	ALPB_LAUNCHED();
 	ALPB_CUDA(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -499,8 +511,10 @@ static int lists_build(alpb_spmv_plan_s *p, cudaStream_t s) {
 		if (cudaMalloc(&p->lor_row, size_t(h[0]) * 8) != cudaSuccess ||
 			cudaMalloc(&p->lor_k0, size_t(h[0]) * 8) != cudaSuccess ||
 			(h[2] > 0 && (cudaMalloc(&p->gen_row, size_t(h[2]) * 8) != cudaSuccess ||
-				cudaMalloc(&p->gen_k0, size_t(h[2]) * 8) != cudaSuccess ||
-				cudaMalloc(&p->gen_first, size_t(h[3]) * 8) != cudaSuccess))) {
+				cudaMalloc(&p->gen_c, size_t(h[2]) * 8) != cudaSuccess ||
+				cudaMalloc(&p->gen_first, size_t(h[3]) * 8) != cudaSuccess ||
+				cudaMalloc(&p->gen_number, size_t(h[3]) * 8) != cudaSuccess ||
+				cudaMalloc(&p->gen_listed, listed) != cudaSuccess))) {
 			cudaGetLastError();
 			cudaFreeAsync(cnt, s);
 			cudaStreamSynchronize(s);
@@ -512,8 +526,11 @@ static int lists_build(alpb_spmv_plan_s *p, cudaStream_t s) {
 		lor.rows = p->lor_row;
 		lor.k0s = p->lor_k0;
 		gen.rows = p->gen_row;
-		gen.k0s = p->gen_k0;
+		gen.k0s = p->gen_c;
 		gen.first = p->gen_first;
+		gen.number = p->gen_number;
+		gen.listed = p->gen_listed;
+		if (h[2] > 0) ALPB_CUDA(cudaMemsetAsync(p->gen_listed, 0, listed, s));
 		k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, lor, gen);
 		ALPB_LAUNCHED();
 	}
@@ -604,24 +621,28 @@ template <class R>
 struct GenRow {
 	using T = typename R::T;
 	int64_t i = -1, b = 0, e = 0;
+	uint32_t listed;
 	uint8_t mask_has, u_flag;
 	T old;
 	bool row_ok = false, id_row = false, u_has = false;
-	__device__ __forceinline__ void fetch(const SpmvArgs &a, int64_t row) {
+	__device__ __forceinline__ void fetch(const SpmvArgs &a, int64_t row,
+		const uint32_t *in_list = nullptr) {
 		i = row;
 		b = e = 0;
+		listed = 0;
 		mask_has = u_flag = 1;
 		old = R::zero();
 		if (i < 0) return;
 		b = a.offsets[i];
 		e = a.offsets[i + 1];
+		if (in_list) listed = in_list[i >> 5] >> (i & 31) & 1u;
 		if (a.masked && a.u_mask_assigned) mask_has = a.u_mask_assigned[i];
 		if (a.u_assigned) u_flag = a.u_assigned[i];
 		old = reinterpret_cast<const T *>(a.u)[i];
 	}
-	// longest: rows of more nonzeroes are somebody else's
-	__device__ __forceinline__ void decide(const SpmvArgs &a, int64_t longest) {
-		row_ok = i >= 0 && e - b <= longest;
+	// listed rows are somebody else's
+	__device__ __forceinline__ void decide(const SpmvArgs &a) {
+		row_ok = i >= 0 && listed == 0;
 		const bool mine = row_ok;
 		if (row_ok && a.masked) {
 			bool t = mask_has != 0;
@@ -718,15 +739,31 @@ __device__ __forceinline__ void gen_gather(const SpmvArgs &a, int64_t b, int64_t
 	}
 }
 
-// Chunks of the long rows (rows of more than GEN_LONG nonzeroes) and where
-// their partials go; nchunks = 0: every row runs in a row group.
+// The listed long rows: their chunks, and where the chunks' partials go;
+// nchunks = 0: every row runs in a row group.  A row's last chunk runs to the row's end and which rows are
+// listed is read from the list, so offsets that changed under the plan cost
+// time, not right sums.
 struct GenChunks {
 	int64_t nchunks = 0, nlong = 0;
-	const int64_t *row = nullptr, *k0 = nullptr;    // [nchunks]
-	const int64_t *first = nullptr;                 // [nlong] first chunk of a long row
-	uint64_t *val = nullptr;                        // [nchunks] partial sums
-	uint8_t *has = nullptr;                         // [nchunks]
+	const int64_t *row = nullptr, *c = nullptr;             // [chunks] row, number in the row
+	const int64_t *first = nullptr, *number = nullptr;      // [nlong] first chunk, chunks
+	const uint32_t *listed = nullptr;                       // a bit per row
+	uint64_t *val = nullptr;                                // [nchunks] partial sums
+	uint8_t *has = nullptr;                                 // [nchunks]
 };
+
+// Chunk c of n of a listed row, by one warp: the partial in lane 0, set in all.
+template <class R, bool BITS>
+__device__ __forceinline__ void gen_chunk(const SpmvArgs &a, const GenRow<R> &row, int64_t c,
+	bool last, int wl, typename R::T &acc, bool &set, const uint32_t *bits = nullptr) {
+	const int64_t k0 = row.b + c * GEN_CHUNK;
+	if (row.row_ok)
+		gen_gather<R, 32, BITS>(a, k0, last || row.e < k0 + GEN_CHUNK ? row.e : k0 + GEN_CHUNK, wl,
+			acc, set, bits);
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o));
+	set = __any_sync(0xffffffffu, set);
+}
 
 // warp-aggregated count of newly assigned entries
 __device__ __forceinline__ void gen_count(const SpmvArgs &a, int64_t newly) {
@@ -768,25 +805,19 @@ k_spmv_vector_general(SpmvArgs a, GenChunks g, const uint32_t *__restrict__ gbit
 	const int wl = threadIdx.x & 31;
 	const int lane = threadIdx.x & (W - 1);
 	const int sub = wl / W;
+	int64_t newly = 0;
 	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
 	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
 	const int64_t items = g.nchunks + (a.m_out + RPW - 1) / RPW;
-	const int64_t long_len = g.nchunks > 0 ? GEN_LONG : INT64_MAX;
-	int64_t newly = 0;
 	int64_t it = warp;
 	for (; it < g.nchunks; it += nwarps) {   // one chunk of a long row, the whole warp
 		GenRow<R> row;
 		row.fetch(a, g.row[it]);
-		const int64_t k0 = g.k0[it];
-		row.decide(a, INT64_MAX);
+		const int64_t c = g.c[it];
+		row.decide(a);
 		T acc = R::zero();
 		bool set = false;
-		if (row.row_ok)
-			gen_gather<R, 32, BITS>(a, k0, row.e < k0 + GEN_CHUNK ? row.e : k0 + GEN_CHUNK, wl, acc,
-				set, gen_bits);
-#pragma unroll
-		for (int o = 16; o > 0; o >>= 1) acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o));
-		set = __any_sync(0xffffffffu, set);
+		gen_chunk<R, BITS>(a, row, c, it + 1 == g.nchunks || g.c[it + 1] == 0, wl, acc, set, gen_bits);
 		if (wl == 0) {
 			store_bits<T>(g.val + it, acc);
 			g.has[it] = set ? 1 : 0;
@@ -799,10 +830,10 @@ k_spmv_vector_general(SpmvArgs a, GenChunks g, const uint32_t *__restrict__ gbit
 		return t < items && i < a.m_out ? i : int64_t(-1);
 	};
 	GenRow<R> row, nxt;
-	row.fetch(a, row_of(it));
+	row.fetch(a, row_of(it), g.listed);
 	for (; it < items; it += nwarps) {
-		nxt.fetch(a, row_of(it + nwarps));
-		row.decide(a, long_len);
+		nxt.fetch(a, row_of(it + nwarps), g.listed);
+		row.decide(a);
 		T acc = R::zero();
 		bool set = false;
 		if (lane == 0) row.identity(a, acc, set);
@@ -832,8 +863,8 @@ k_spmv_general_finish(SpmvArgs a, GenChunks g) {
 		const int64_t c0 = g.first[l];
 		GenRow<R> row;
 		row.fetch(a, g.row[c0]);
-		const int64_t n = (row.e - row.b + GEN_CHUNK - 1) / GEN_CHUNK;
-		row.decide(a, INT64_MAX);
+		const int64_t n = g.number[l];
+		row.decide(a);
 		T acc = R::zero();
 		bool set = false;
 		if (lane == 0) row.identity(a, acc, set);
@@ -1004,8 +1035,10 @@ int launch_vector_general_w(const SpmvArgs &a, const alpb_spmv_plan_s *p, cudaSt
 				g.nchunks = chunks;
 				g.nlong = p->gen_rows;
 				g.row = p->gen_row;
-				g.k0 = p->gen_k0;
+				g.c = p->gen_c;
 				g.first = p->gen_first;
+				g.number = p->gen_number;
+				g.listed = p->gen_listed;
 				g.val = reinterpret_cast<uint64_t *>(at + bit_bytes);
 				g.has = reinterpret_cast<uint8_t *>(g.val + chunks);
 			}

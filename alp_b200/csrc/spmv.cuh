@@ -51,11 +51,13 @@ struct alpb_spmv_plan_s {
 	int64_t *lor_row = nullptr;
 	int64_t *lor_k0 = nullptr;
 	// General path: the rows of more than GEN_LONG nonzeroes in chunks of
-	// GEN_CHUNK, a row's chunks consecutive; gen_first: each row's first chunk.
+	// GEN_CHUNK, a row's chunks consecutive.
 	int64_t gen_n = 0, gen_rows = 0;
-	int64_t *gen_row = nullptr;
-	int64_t *gen_k0 = nullptr;
-	int64_t *gen_first = nullptr;
+	int64_t *gen_row = nullptr;      // [gen_n] the chunk's row
+	int64_t *gen_c = nullptr;        // [gen_n] its number in the row
+	int64_t *gen_first = nullptr;    // [gen_rows] a row's first chunk
+	int64_t *gen_number = nullptr;   // [gen_rows] its chunks
+	uint32_t *gen_listed = nullptr;  // a bit per row: in the list
 };
 
 namespace alpb {

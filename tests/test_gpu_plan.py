@@ -82,3 +82,30 @@ def test_boolean_plan_of_another_storage(cuda):
         want = np.zeros(m, np.uint8)
         np.maximum.at(want, np.repeat(np.arange(m), np.diff(o)), x[c])
         assert np.array_equal(u.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+@pytest.mark.parametrize("kind,m", [("regular", 4000), ("regular", 500000), ("skewed", 500000)])
+def test_structure_changed_in_place(cuda, kind, m, sparse):
+    """The offsets a plan was made from get another structure of as many
+    nonzeroes.  Products that ran on the plan's lane width alone (the vector
+    schedule, the general path) stay right: no row is lost to a list of long
+    rows, and no row outgrows its stage in shared memory."""
+    from alp_b200 import device as dev
+    if kind == "skewed" and not sparse:
+        pytest.skip("a merge-path plan's tile table is the structure")
+    rng = np.random.default_rng([m, sparse, 7])
+    n, lens = 70001, lengths(kind, m, rng)
+    rp, col = storage(lens, n, rng)
+    rp2, col2 = storage(reshaped(lens, rng), n, rng)
+    vals = rng.random(len(col))
+    A, B = dev.from_host(m, n, rp, col, vals), dev.from_host(m, n, rp2, col2, vals)
+    for sched in (0, 2):
+        plan = dev.Plan(A, sched=sched)
+        check(A, rp, col, vals, plan, rng, sparse)
+        old = A.offsets.clone(), A.indices.clone()
+        A.offsets.copy_(B.offsets)
+        A.indices.copy_(B.indices)
+        check(A, rp2, col2, vals, plan, rng, sparse)
+        A.offsets.copy_(old[0])
+        A.indices.copy_(old[1])
