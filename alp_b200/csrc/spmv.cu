@@ -367,7 +367,7 @@ constexpr int LOR_CHUNK = 256;
 constexpr int GEN_LONG = 64;
 constexpr int GEN_CHUNK = 256;
 constexpr int GEN_BATCH = 4;
-constexpr int64_t GEN_NARROW = int64_t(1) << 20;
+constexpr int64_t GEN_NARROW = int64_t(1) << 20;   // see launch_general
 constexpr int GEN_BATCH_BITS = 8;   // where the flags are bits in shared memory
 
 template <bool VALUED>
@@ -439,12 +439,13 @@ k_lor_tail(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ ind
 // position taken from *count (any order of the rows: no result depends on
 // it); first and number, when given, list each row's first chunk and its chunks
 // at a position from *nrows, listed marks the row.  rows == nullptr: count only.
+constexpr int64_t LIST_LAST = int64_t(1) << 62;
 struct ChunkList {
 	int64_t longer, head, chunk;
 	unsigned long long *count, *nrows;
 	int64_t *rows, *k0s;
 	// the general path's list only: chunks are named by their number in the row
-	// (k0s) instead of a place in the storage
+	// (k0s; LIST_LAST marks the last) instead of a place in the storage
 	int64_t *first, *number;
 	uint32_t *listed;
 };
@@ -456,7 +457,7 @@ __device__ __forceinline__ void add_row_chunks(const ChunkList &l, int64_t i, in
 	if (!l.rows) return;
 	for (int64_t c = 0; c < n; ++c) {
 		l.rows[at + c] = i;
-		l.k0s[at + c] = l.first ? c : b + c * l.chunk;
+		l.k0s[at + c] = l.first ? c | (c + 1 == n ? LIST_LAST : 0) : b + c * l.chunk;
 	}
 	if (l.first) {
 		l.first[r] = int64_t(at);
@@ -477,11 +478,7 @@ __global__ void k_row_chunks(const int64_t *__restrict__ offsets, int64_t m, Chu
 static void lists_release(alpb_spmv_plan_s *p) {
 	cudaFree(p->lor_row);
 	cudaFree(p->lor_k0);
-	cudaFree(p->gen_row);
-	cudaFree(p->gen_c);
-	cudaFree(p->gen_first);
-	cudaFree(p->gen_number);
-	cudaFree(p->gen_listed);
+	cudaFree(p->gen_row);   // the general path's five lists
 	p->lor_row = p->lor_k0 = p->gen_row = p->gen_c = p->gen_first = p->gen_number = nullptr;
 	p->gen_listed = nullptr;
 	p->lor_n = -1;
@@ -510,11 +507,7 @@ static int lists_build(alpb_spmv_plan_s *p, cudaStream_t s) {
 	if (h[0] > 0) {
 		if (cudaMalloc(&p->lor_row, size_t(h[0]) * 8) != cudaSuccess ||
 			cudaMalloc(&p->lor_k0, size_t(h[0]) * 8) != cudaSuccess ||
-			(h[2] > 0 && (cudaMalloc(&p->gen_row, size_t(h[2]) * 8) != cudaSuccess ||
-				cudaMalloc(&p->gen_c, size_t(h[2]) * 8) != cudaSuccess ||
-				cudaMalloc(&p->gen_first, size_t(h[3]) * 8) != cudaSuccess ||
-				cudaMalloc(&p->gen_number, size_t(h[3]) * 8) != cudaSuccess ||
-				cudaMalloc(&p->gen_listed, listed) != cudaSuccess))) {
+			(h[2] > 0 && cudaMalloc(&p->gen_row, size_t(h[2] + h[3]) * 16 + listed) != cudaSuccess)) {
 			cudaGetLastError();
 			cudaFreeAsync(cnt, s);
 			cudaStreamSynchronize(s);
@@ -525,12 +518,18 @@ static int lists_build(alpb_spmv_plan_s *p, cudaStream_t s) {
 		ALPB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(h), s));
 		lor.rows = p->lor_row;
 		lor.k0s = p->lor_k0;
+		if (h[2] > 0) {   // one allocation
+			p->gen_c = p->gen_row + h[2];
+			p->gen_first = p->gen_c + h[2];
+			p->gen_number = p->gen_first + h[3];
+			p->gen_listed = reinterpret_cast<uint32_t *>(p->gen_number + h[3]);
+			ALPB_CUDA(cudaMemsetAsync(p->gen_listed, 0, listed, s));
+		}
 		gen.rows = p->gen_row;
 		gen.k0s = p->gen_c;
 		gen.first = p->gen_first;
 		gen.number = p->gen_number;
 		gen.listed = p->gen_listed;
-		if (h[2] > 0) ALPB_CUDA(cudaMemsetAsync(p->gen_listed, 0, listed, s));
 		k_row_chunks<<<grid, 256, 0, s>>>(p->offsets, p->m, lor, gen);
 		ALPB_LAUNCHED();
 	}
@@ -599,20 +598,110 @@ k_spmv_vector_dense(const int64_t *__restrict__ offsets, const uint32_t *__restr
 	}
 }
 
-// General path, all ALP semantics; see the file comment.  Two kinds of work
-// items share one launch: chunks of long rows, then groups of 32/W rows.
+// warp-aggregated count of newly assigned entries
+__device__ __forceinline__ void gen_count(const SpmvArgs &a, int64_t newly) {
+	if (!a.u_nnz) return;
+	for (int o = 16; o > 0; o >>= 1) newly += __shfl_down_sync(0xffffffffu, newly, o);
+	if ((threadIdx.x & 31) == 0 && newly)
+		atomicAdd((unsigned long long *) a.u_nnz, (unsigned long long) newly);
+}
+
+// General path, all ALP semantics; see the file comment.  Two kernels.
 //
-// What bounds it is the dependent chain index -> flag -> value and x of each
-// nonzero, so a lane issues GEN_BATCH of each before it uses any, and the row
+// k_spmv_vector_plain: W lanes walk a row, one nonzero of each lane after the
+// other, in few registers: many warps hide the chain index -> flag -> value and
+// x of each nonzero.  No list, no scratch.  It is the faster one where row
+// lengths hardly differ (stencils: neighbouring rows share lines of flags and x,
+// and a row is only a few steps; us, this / the other with as many lanes, 27-point
+// 130^3 under a mask 181 / 231, from a 50% sparse vector 201 / 280) and it
+// serves calls without a plan.
+//
+// k_spmv_vector_general, for rows of differing lengths: two kinds of work items,
+// chunks of long rows, then groups of 32/W rows.  What bounds it is that same
+// chain, so a lane issues GEN_BATCH of each load before it uses any, and the row
 // lengths: with W lanes on every row, a hub row of 1e5 nonzeroes ran as 1e4
-// dependent steps of one lane group while the rest of the chip idled.  Rows
-// of more than GEN_LONG nonzeroes are therefore cut in chunks of GEN_CHUNK
-// (the plan's list), one warp each, first in the item order; their partials
-// are summed in chunk order by k_spmv_general_finish (deterministic).
+// dependent steps of one lane group while the rest of the chip idled.  Rows of
+// more than GEN_LONG nonzeroes are therefore cut in chunks of GEN_CHUNK (the
+// plan's list), one warp each, first in the item order; their partials are
+// summed in chunk order by k_spmv_general_finish (deterministic).
 // Measured, R-MAT: min-plus from a 20% sparse vector, 500,009 vertices,
 // 2289 -> 118 us, 78 with the bits and the narrow groups below; lor-land with a
-// 5% frontier and 30% visited, 1,000,003
-// vertices, 474 -> 188, 142 us.
+// 5% frontier and 30% visited, 1,000,003 vertices, 474 -> 188, 142 us.
+template <class R, int W>
+__global__ void __launch_bounds__(256)
+k_spmv_vector_plain(SpmvArgs a) {
+	using T = typename R::T;
+	constexpr int RPW = 32 / W;
+	const T *__restrict__ values = reinterpret_cast<const T *>(a.values);
+	const T *__restrict__ x = reinterpret_cast<const T *>(a.v);
+	T *__restrict__ y = reinterpret_cast<T *>(a.u);
+	const bool dense_hint = (a.descr & ALPB_DESC_DENSE) != 0;
+	const bool add_identity = (a.descr & ALPB_DESC_ADD_IDENTITY) != 0;
+	const bool use_index = (a.descr & ALPB_DESC_USE_INDEX) != 0;
+	const bool explicit_zero = (a.descr & ALPB_DESC_EXPLICIT_ZERO) != 0;
+	const int lane = threadIdx.x & (W - 1);
+	const int sub = (threadIdx.x & 31) / W;
+	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+	int64_t newly = 0;
+	for (int64_t base = warp * RPW; base < a.m_out; base += nwarps * RPW) {
+		const int64_t i = base + sub;
+		const bool in_range = i < a.m_out;
+		bool row_ok = in_range;
+		if (row_ok && a.masked)
+			row_ok = a.mask_by_structure
+				? (a.u_mask_assigned == nullptr || a.u_mask_assigned[i] != 0)
+				: eval_mask(a.u_mask, a.u_mask_assigned, a.u_mask_type, a.descr, i);
+		const bool id_row = in_range && add_identity && (a.scatter_sem || row_ok);
+		const bool u_has = in_range && (a.u_assigned == nullptr || a.u_assigned[i] != 0);
+		// immutable-nonzero shortcut of the gather (blas2.hpp:351-357)
+		if (R::immutable && !a.scatter_sem && row_ok && u_has && y[i] != R::zero()) row_ok = false;
+		const bool active = row_ok || id_row;
+		T acc = R::zero();
+		bool set = false;
+		if (active) {
+			if (id_row && lane == 0 && i < a.n_in) {
+				const bool vm_ok = !a.input_masked ||
+					eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, i);
+				if (vm_ok && (dense_hint || a.v_assigned == nullptr || a.v_assigned[i])) {
+					acc = a.left ? R::mull(x[i], R::one()) : R::mulr(R::one(), x[i]);
+					set = true;
+				}
+			}
+			const int64_t b = row_ok ? a.offsets[i] : 0, e = row_ok ? a.offsets[i + 1] : 0;
+			for (int64_t k = b + lane; k < e; k += W) {
+				const uint32_t j = a.indices[k];
+				if (a.input_masked &&
+					!eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, j))
+					continue;
+				if (!dense_hint && a.v_assigned != nullptr && !a.v_assigned[j]) continue;
+				const T av = values ? values[k] : R::one();
+				const T xv = use_index ? T(j) : x[j];
+				acc = R::add(a.left ? R::mull(xv, av) : R::mulr(av, xv), acc);
+				set = true;
+				if (R::immutable && acc != R::zero()) break;
+			}
+		}
+#pragma unroll
+		for (int o = W / 2; o > 0; o >>= 1) {
+			acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o, W));
+			set = set | (__shfl_down_sync(0xffffffffu, int(set), o, W) != 0);
+		}
+		const bool ez = explicit_zero && !a.scatter_sem && row_ok;
+		if (active && lane == 0 && (ez || set)) {
+			if (u_has || dense_hint) {
+				y[i] = R::add(y[i], acc);
+			} else {
+				y[i] = acc;
+			}
+			if (!u_has && a.u_assigned) {
+				a.u_assigned[i] = 1;
+				++newly;
+			}
+		}
+	}
+	gen_count(a, newly);
+}
 
 // Rows of the general path: who takes part, and the row's identity term.  Made
 // in two halves: fetch() loads what the row's place says (no load waits for
@@ -739,8 +828,9 @@ __device__ __forceinline__ void gen_gather(const SpmvArgs &a, int64_t b, int64_t
 	}
 }
 
-// The listed long rows: their chunks, and where the chunks' partials go;
-// nchunks = 0: every row runs in a row group.  A row's last chunk runs to the row's end and which rows are
+// The listed long rows: their chunks, and where the chunks' partials go.
+// nchunks = 0: the first nlong blocks take a listed row each, without partials
+// in memory.  A row's last chunk runs to the row's end and which rows are
 // listed is read from the list, so offsets that changed under the plan cost
 // time, not right sums.
 struct GenChunks {
@@ -765,12 +855,43 @@ __device__ __forceinline__ void gen_chunk(const SpmvArgs &a, const GenRow<R> &ro
 	set = __any_sync(0xffffffffu, set);
 }
 
-// warp-aggregated count of newly assigned entries
-__device__ __forceinline__ void gen_count(const SpmvArgs &a, int64_t newly) {
-	if (!a.u_nnz) return;
-	for (int o = 16; o > 0; o >>= 1) newly += __shfl_down_sync(0xffffffffu, newly, o);
-	if ((threadIdx.x & 31) == 0 && newly)
-		atomicAdd((unsigned long long *) a.u_nnz, (unsigned long long) newly);
+// One listed row by a block of 8 warps, the adds in the order of chunks and
+// finish pass: lane c % 32 of the first warp takes the partial of chunk c.
+template <class R>
+__device__ __forceinline__ void gen_long_row(const SpmvArgs &a, const GenChunks &g, int64_t l,
+	int64_t &newly) {
+	using T = typename R::T;
+	__shared__ T part[8];
+	__shared__ uint8_t has[8];
+	const int wl = threadIdx.x & 31, w = threadIdx.x >> 5;
+	GenRow<R> row;
+	row.fetch(a, g.row[g.first[l]]);
+	const int64_t n = g.number[l];
+	row.decide(a);
+	T acc = R::zero();
+	bool set = false;
+	if (threadIdx.x == 0) row.identity(a, acc, set);
+	for (int64_t c0 = 0; c0 < n; c0 += 8) {
+		T p = R::zero();
+		bool ps = false;
+		if (c0 + w < n) gen_chunk<R, false>(a, row, c0 + w, c0 + w == n - 1, wl, p, ps);
+		if (wl == 0) {
+			part[w] = p;
+			has[w] = ps ? 1 : 0;
+		}
+		__syncthreads();
+		const int q = wl - int(c0 & 31);
+		if (w == 0 && q >= 0 && q < 8 && has[q]) {
+			acc = R::add(acc, part[q]);
+			set = true;
+		}
+		if (__syncthreads_or(R::immutable && acc != R::zero())) break;
+	}
+	if (w != 0) return;
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o));
+	set = __any_sync(0xffffffffu, set);
+	if (wl == 0) row.finish(a, acc, set, newly);
 }
 
 // Which inputs take part (assigned, and let through by the input mask), a bit
@@ -786,14 +907,18 @@ __global__ void k_pack_present(SpmvArgs a, uint32_t *bits) {
 	}
 }
 
-// BITS: every block copies the inputs' bits into its shared memory first.  A
-// nonzero then asks shared memory whether its input takes part (a warp's 32
+// How the general kernel runs.  GEN_CHUNKS: flags asked in memory, long rows in
+// chunks (or none listed).  GEN_BLOCKS: the same, but the first blocks take a listed
+// row each.  GEN_BITS: as GEN_CHUNKS, and every block copies the inputs' bits into its
+// shared memory first.  A nonzero then asks shared memory whether its input takes part (a warp's 32
 // random words are about four wavefronts there, and up to 32 in L1), and only
 // those that do gather x.
-template <class R, int W, bool BITS>
-__global__ void __launch_bounds__(BITS ? 1024 : 256)
+enum { GEN_CHUNKS, GEN_BLOCKS, GEN_BITS };
+template <class R, int W, int MODE>
+__global__ void __launch_bounds__(MODE == GEN_BITS ? 1024 : 256)
 k_spmv_vector_general(SpmvArgs a, GenChunks g, const uint32_t *__restrict__ gbits) {
 	using T = typename R::T;
+	constexpr bool BITS = MODE == GEN_BITS;
 	extern __shared__ __align__(16) uint32_t gen_bits[];
 	if (BITS) {
 		const int64_t words = (a.n_in + 31) / 32;
@@ -806,18 +931,28 @@ k_spmv_vector_general(SpmvArgs a, GenChunks g, const uint32_t *__restrict__ gbit
 	const int lane = threadIdx.x & (W - 1);
 	const int sub = wl / W;
 	int64_t newly = 0;
-	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
-	const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+	int64_t block = blockIdx.x, nblocks = gridDim.x;
+	if constexpr (MODE == GEN_BLOCKS) {
+		if (block < g.nlong) {
+			gen_long_row<R>(a, g, block, newly);
+			gen_count(a, newly);
+			return;
+		}
+		block -= g.nlong;
+		nblocks -= g.nlong;
+	}
+	const int64_t warp = (block * int64_t(blockDim.x) + threadIdx.x) >> 5;
+	const int64_t nwarps = (nblocks * int64_t(blockDim.x)) >> 5;
 	const int64_t items = g.nchunks + (a.m_out + RPW - 1) / RPW;
 	int64_t it = warp;
-	for (; it < g.nchunks; it += nwarps) {   // one chunk of a long row, the whole warp
+	for (; MODE != GEN_BLOCKS && it < g.nchunks; it += nwarps) {   // one chunk of a long row, the whole warp
 		GenRow<R> row;
 		row.fetch(a, g.row[it]);
 		const int64_t c = g.c[it];
 		row.decide(a);
 		T acc = R::zero();
 		bool set = false;
-		gen_chunk<R, BITS>(a, row, c, it + 1 == g.nchunks || g.c[it + 1] == 0, wl, acc, set, gen_bits);
+		gen_chunk<R, BITS>(a, row, c & ~LIST_LAST, (c & LIST_LAST) != 0, wl, acc, set, gen_bits);
 		if (wl == 0) {
 			store_bits<T>(g.val + it, acc);
 			g.has[it] = set ? 1 : 0;
@@ -1014,31 +1149,54 @@ int launch_vector_dense_w(const SpmvArgs &a, cudaStream_t s) {
 constexpr int64_t GEN_BITS_NNZ = int64_t(1) << 21;
 constexpr int64_t GEN_BITS_MAX = 200 * 1024 * 8;
 
+// Below this many nonzeroes the listed rows run a block each in the one launch:
+// the partials' memory and the finish pass cost a small product more than the
+// chip they fill (R-MAT, min-plus from a 20% sparse vector, us, blocks / chunks:
+// 20,000 vertices, 0.23 M nonzeroes, 16 / 23; 100,000, 1.4 M, 34 / 28).
+constexpr int64_t GEN_SCRATCH_NNZ = int64_t(1) << 20;
+static_assert(GEN_SCRATCH_NNZ <= GEN_BITS_NNZ, "the kernel with the bits takes chunks");
+
+// A call under stream capture takes no scratch: its graph would hold allocation
+// nodes, and could not be a child graph or run twice at once.
+static bool capturing(cudaStream_t s) {
+	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+	if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+	cudaGetLastError();   // the legacy stream during another stream's capture
+	return true;
+}
+
+// Some inputs may not take part.
+static bool gen_filtered(const SpmvArgs &a) {
+	return a.input_masked || (a.v_assigned && !(a.descr & ALPB_DESC_DENSE));
+}
+
+// lists: p's lists are used.
 template <class R, int W>
-int launch_vector_general_w(const SpmvArgs &a, const alpb_spmv_plan_s *p, cudaStream_t s) {
+int launch_general_w(const SpmvArgs &a, const alpb_spmv_plan_s *p, bool lists, cudaStream_t s) {
 	constexpr int RPW = 32 / W;
 	GenChunks g;
+	if (lists) {
+		g.nlong = p->gen_rows;
+		g.row = p->gen_row;
+		g.c = p->gen_c;
+		g.first = p->gen_first;
+		g.number = p->gen_number;
+		g.listed = p->gen_listed;
+	}
 	void *scratch = nullptr;
 	uint32_t *bits = nullptr;
-	const bool filtered = a.input_masked || (a.v_assigned && !(a.descr & ALPB_DESC_DENSE));
-	const bool want_bits = filtered && a.nnz >= GEN_BITS_NNZ && a.n_in <= GEN_BITS_MAX;
+	const bool want_bits = gen_filtered(a) && a.nnz >= GEN_BITS_NNZ && a.n_in <= GEN_BITS_MAX;
 	const size_t bit_bytes = want_bits ? size_t(a.n_in + 127) / 128 * 16 : 0;
-	const int64_t chunks = p && p->gen_n > 0 ? p->gen_n : 0;
-	if (bit_bytes || chunks) {
+	const int64_t chunks = lists && a.nnz >= GEN_SCRATCH_NNZ ? p->gen_n : 0;
+	if ((bit_bytes || chunks) && !capturing(s)) {
 		// bits, then the partials of the long rows' chunks: this call's own
-		// (calls on other streams may use the same plan); without them every
-		// row runs in a group and asks the flags in memory
+		// (calls on other streams may use the same plan); without them the
+		// listed rows run a block each and the flags are asked in memory
 		if (cudaMallocAsync(&scratch, bit_bytes + size_t(chunks) * 9, s) == cudaSuccess) {
 			unsigned char *at = static_cast<unsigned char *>(scratch);
 			if (bit_bytes) bits = reinterpret_cast<uint32_t *>(at);
 			if (chunks) {
 				g.nchunks = chunks;
-				g.nlong = p->gen_rows;
-				g.row = p->gen_row;
-				g.c = p->gen_c;
-				g.first = p->gen_first;
-				g.number = p->gen_number;
-				g.listed = p->gen_listed;
 				g.val = reinterpret_cast<uint64_t *>(at + bit_bytes);
 				g.has = reinterpret_cast<uint8_t *>(g.val + chunks);
 			}
@@ -1050,21 +1208,31 @@ int launch_vector_general_w(const SpmvArgs &a, const alpb_spmv_plan_s *p, cudaSt
 	const int64_t items = g.nchunks + (a.m_out + RPW - 1) / RPW;
 	if (bits) {
 		static std::atomic<unsigned long long> allowed_in;
-		ALPB_CUDA(allow_smem(k_spmv_vector_general<R, W, true>, GEN_BITS_MAX / 8, allowed_in));
+		ALPB_CUDA(allow_smem(k_spmv_vector_general<R, W, GEN_BITS>, GEN_BITS_MAX / 8, allowed_in));
 		k_pack_present<<<grid_for(a.n_in, 256), 256, 0, s>>>(a, bits);
 		ALPB_LAUNCHED();
-		k_spmv_vector_general<R, W, true><<<grid_for(items * 32, 1024, 1), 1024, bit_bytes, s>>>(a,
-			g, bits);
+		k_spmv_vector_general<R, W, GEN_BITS><<<grid_for(items * 32, 1024, 1), 1024, bit_bytes,
+			s>>>(a, g, bits);
+	} else if (g.nlong > 0 && g.nchunks == 0) {
+		k_spmv_vector_general<R, W, GEN_BLOCKS><<<unsigned(g.nlong + grid_for(items * 32, 256, 8)),
+			256, 0, s>>>(a, g, nullptr);
 	} else {
-		k_spmv_vector_general<R, W, false><<<grid_for(items * 32, 256, 8), 256, 0, s>>>(a, g,
+		k_spmv_vector_general<R, W, GEN_CHUNKS><<<grid_for(items * 32, 256, 8), 256, 0, s>>>(a, g,
 			nullptr);
 	}
 	ALPB_LAUNCHED();
-	if (g.nlong > 0) {
+	if (g.nchunks > 0) {
 		k_spmv_general_finish<R><<<grid_for(g.nlong * 32, 256, 8), 256, 0, s>>>(a, g);
 		ALPB_LAUNCHED();
 	}
 	if (scratch) ALPB_CUDA(cudaFreeAsync(scratch, s));
+	return ALPB_SUCCESS;
+}
+
+template <class R, int W>
+int launch_plain_w(const SpmvArgs &a, cudaStream_t s) {
+	k_spmv_vector_plain<R, W><<<grid_for(a.m_out * W, 256, 8), 256, 0, s>>>(a);
+	ALPB_LAUNCHED();
 	return ALPB_SUCCESS;
 }
 
@@ -1088,27 +1256,48 @@ int launch_small(const SpmvArgs &a, const alpb_spmv_plan_s &p, cudaStream_t s) {
 	return p.mean < 6 ? go(std::integral_constant<int, 4>{}) : go(std::integral_constant<int, 8>{});
 }
 
-template <class R>
-int launch_vector(const SpmvArgs &a, const alpb_spmv_plan_s *p, int W, bool dense,
-	cudaStream_t s) {
-	if (dense) {
-		switch (W) {
-		case 1: return launch_vector_dense_w<R, 1>(a, s);
-		case 2: return launch_vector_dense_w<R, 2>(a, s);
-		case 4: return launch_vector_dense_w<R, 4>(a, s);
-		case 8: return launch_vector_dense_w<R, 8>(a, s);
-		case 16: return launch_vector_dense_w<R, 16>(a, s);
-		default: return launch_vector_dense_w<R, 32>(a, s);
-		}
-	}
+// f(integral_constant of W)
+template <class F>
+static int with_width(int W, const F &f) {
 	switch (W) {
-	case 1: return launch_vector_general_w<R, 1>(a, p, s);
-	case 2: return launch_vector_general_w<R, 2>(a, p, s);
-	case 4: return launch_vector_general_w<R, 4>(a, p, s);
-	case 8: return launch_vector_general_w<R, 8>(a, p, s);
-	case 16: return launch_vector_general_w<R, 16>(a, p, s);
-	default: return launch_vector_general_w<R, 32>(a, p, s);
+	case 1: return f(std::integral_constant<int, 1>{});
+	case 2: return f(std::integral_constant<int, 2>{});
+	case 4: return f(std::integral_constant<int, 4>{});
+	case 8: return f(std::integral_constant<int, 8>{});
+	case 16: return f(std::integral_constant<int, 16>{});
+	default: return f(std::integral_constant<int, 32>{});
 	}
+}
+
+// The general path.  Which kernel: k_spmv_vector_plain without a plan, for rows
+// of nearly one length, and for matrices without hub rows whose width the caller
+// gave or that are small; measured us, plain / the other, min-plus from a 20%
+// sparse vector unless said:
+//   hub rows, R-MAT 100,000 vertices 373 / 28, lognormal rows 300,000 118 / 50
+//   (under a mask, FP64, 2,000,000: 265 / 288); lists for rows that are merely
+//   longer than GEN_LONG cost more than they give (rows of 200: 82 / 93,
+//   of 0 to 100: 122 / 124, 74 without the lists);
+//   random rows, no hubs, from GEN_NARROW nonzeroes on: mean 16 and 1,000,000 rows
+//   110 / 70, mean 30 and 300,000 rows 74 / 45; where the inputs' flags do not fit as
+//   bits, mean 16 and 3,000,000 rows (2 lanes) 314 / 382 (478 / 344 in FP64), mean 30
+//   and 2,000,000 rows 462 / 528: from 8 lanes on the plain one;
+//   one length: 27-point 117^3 116 / 274, 5-point 1200^2 37 / 57, rows of 200 as above.
+// A lane waits for its row's chain of loads, so from GEN_NARROW nonzeroes on a
+// quarter of the lanes per row, and four times the rows in flight, is faster
+// (R-MAT with lists, us with 8 / 2 lanes: 1,000,003 vertices, lor, 185 / 144,
+// 500,009, min-plus, 90 / 70; 20,000: 15.8 / 17.8); without lists a hub row would
+// run on those few.  A width that the caller gave is kept.
+static bool gen_no_bits(const SpmvArgs &a) { return gen_filtered(a) && a.n_in > GEN_BITS_MAX; }
+template <class R>
+int launch_general(const SpmvArgs &a, const alpb_spmv_plan_s *p, int W, cudaStream_t s) {
+	const bool lists = p && p->hubs && p->gen_n > 0;
+	if (!p || p->steady ||
+		(!lists && (p->given_width || a.nnz < GEN_NARROW || (W >= 8 && gen_no_bits(a)))))
+		return with_width(W, [&](auto w) { return launch_plain_w<R, decltype(w)::value>(a, s); });
+	if (!p->given_width && a.nnz >= GEN_NARROW && W >= 4) W /= 4;
+	return with_width(W, [&](auto w) {
+		return launch_general_w<R, decltype(w)::value>(a, p, lists, s);
+	});
 }
 
 // Row-streaming kernel of one chunk shape; the block takes as many warps as
@@ -1187,12 +1376,8 @@ int run_spmv(const SpmvArgs &a, const alpb_spmv_plan_s *plan, int force_sched, c
 	if (fast && p && p->rows && !(reinterpret_cast<uintptr_t>(a.indices) & 15) &&
 		!(reinterpret_cast<uintptr_t>(a.values) & 15))
 		return launch_rows<R>(a, int(p->maxlen), s);
-	// The general path waits for a row's chain of loads, so from GEN_NARROW
-	// nonzeroes on a quarter of the lanes per row, and four times the rows in
-	// flight, is faster (R-MAT, us with 8 / 2 lanes: 1,000,003 vertices, lor,
-	// 185 / 144, 500,009, min-plus, 90 / 70; 20,000: 15.8 / 17.8).
-	if (!fast && a.nnz >= GEN_NARROW && W >= 4) W /= 4;
-	return launch_vector<R>(a, p, W, fast, s);
+	if (!fast) return launch_general<R>(a, p, W, s);
+	return with_width(W, [&](auto w) { return launch_vector_dense_w<R, decltype(w)::value>(a, s); });
 }
 
 int dispatch_spmv(int ring, const SpmvArgs &a, const alpb_spmv_plan_s *p, int force_sched,
@@ -1334,6 +1519,11 @@ int alpb::plan_create_tiles(alpb_spmv_plan_s **plan, int64_t m, int64_t nnz,
 	} else {
 		p->vw = regular ? regular_width(p->mean) : default_width(p->mean);
 	}
+	p->given_width = vector_width > 0;
+	// rows of nearly one length (stencils with their boundaries), and rows so long
+	// that no lane group should walk one: launch_general has the figures
+	p->steady = p->cv < 0.15;
+	p->hubs = !p->steady && p->maxlen > 256 && p->maxlen >= 8 * p->mean;
 	p->small = sched == ALPB_SCHED_AUTO && !regular && nnz <= SMALL_NNZ && p->maxlen <= SMALL_ROW;
 	if (sched == ALPB_SCHED_AUTO) sched = regular ? ALPB_SCHED_VECTOR : ALPB_SCHED_MERGE_PATH;
 	p->sched = sched;

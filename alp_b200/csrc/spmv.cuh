@@ -11,6 +11,9 @@ struct alpb_spmv_plan_s {
 	int vw = 8;
 	bool small = false;  // merge path by the plan's own choice: k_spmv_small instead
 	bool rows = false;   // vector schedule: short regular rows, streamed (rowstream.cuh)
+	bool steady = false;       // rows of nearly one length
+	bool hubs = false;         // some rows far longer than the others
+	bool given_width = false;  // vw is the caller's
 	int device = 0;
 	int64_t ntiles = 0;
 	int64_t tile = 0;               // merge items per tile of the tables below
@@ -54,7 +57,7 @@ struct alpb_spmv_plan_s {
 	// GEN_CHUNK, a row's chunks consecutive.
 	int64_t gen_n = 0, gen_rows = 0;
 	int64_t *gen_row = nullptr;      // [gen_n] the chunk's row
-	int64_t *gen_c = nullptr;        // [gen_n] its number in the row
+	int64_t *gen_c = nullptr;        // [gen_n] its number in the row, the last one marked
 	int64_t *gen_first = nullptr;    // [gen_rows] a row's first chunk
 	int64_t *gen_number = nullptr;   // [gen_rows] its chunks
 	uint32_t *gen_listed = nullptr;  // a bit per row: in the list

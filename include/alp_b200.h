@@ -313,7 +313,10 @@ ALPB_API int alpb_spmv_plan_info(alpb_spmv_plan plan, int *sched, int *vector_wi
  * the host) drive the trivial cases (blas2.hpp:1001-1037) and the dense
  * checks (blas2.hpp:950-971): v_count = nnz(v); u_mask_count = nnz(u_mask)
  * or -1 for "no output mask"; v_mask_count likewise for the input mask.
- * `plan` may be NULL (vector schedule, no scratch).
+ * `plan` may be NULL (vector schedule, no scratch).  With a plan, a product
+ * with masks, sparse vectors or a descriptor may take scratch from the device's
+ * stream-ordered pool for the call; under stream capture it takes none, and
+ * the captured graph holds kernels only.
  */
 ALPB_API int alpb_mxv(int ring, uint32_t descr, int form,
 	int64_t m_out, int64_t n_in, int64_t nnz,

@@ -146,3 +146,105 @@ def test_products_under_capture(cuda, path):
         u.fill_(float(k))
         call()
         assert torch.equal(got, u)
+
+
+def lane_sums(rp, x, W):
+    """Row sums of x as W lanes take them: lane l the entries l, l + W, ... in
+    order, then the lanes by halves."""
+    lens = np.diff(rp)
+    acc = np.zeros((len(lens), W))
+    for k in range(0, int(lens.max(initial=0)), W):
+        for lane in range(W):
+            on = lens > k + lane
+            acc[on, lane] = x[rp[:-1][on] + k + lane] + acc[on, lane]
+    while acc.shape[1] > 1:
+        h = acc.shape[1] // 2
+        acc = acc[:, :h] + acc[:, h:]
+    return acc[:, 0]
+
+
+@pytest.mark.parametrize("case", ["no_plan", "steady", "given", "given_hubs", "narrow"])
+def test_general_path_lane_width(cuda, case):
+    """Which lanes sum a row, in the bits of an FP64 product by a pattern matrix
+    of more than 2^20 nonzeroes: the default width without a plan, the plan's on
+    rows of one length, the caller's where one was given, a quarter of the
+    plan's own where lengths differ.  Rows in the plan's list of long rows (more
+    than 64 nonzeroes, beside hub rows) are left out."""
+    import torch
+    from alp_b200 import device as dev
+    rng = np.random.default_rng(17)
+    m, n = 60000, 30011
+    if case == "steady":
+        lens, kw, W = np.full(m, 27), {}, 4
+    elif case == "no_plan":
+        lens, kw, W = rng.integers(10, 45, m), None, 16
+    else:
+        lens = rng.integers(0, 61, m)
+        kw, W = ({}, 4) if case == "narrow" else ({"vector_width": 8}, 8)
+        if case == "given_hubs":
+            lens[[3, 40000]] = 5000, 90
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    nnz = int(rp[-1])
+    assert nnz > 1 << 20
+    col = rng.integers(0, n, nnz).astype(np.uint32)
+    A = dev.from_host(m, n, rp, col, None, 0)
+    plan = None if kw is None else dev.Plan(A, **kw)
+    x, u = rng.random(n), rng.random(m)
+    xa = np.ones(n, np.uint8)
+    got = torch.from_numpy(u.copy()).cuda()
+    dev.mxv(0, A, got, torch.from_numpy(x).cuda(), plan=plan, v_assigned=torch.from_numpy(xa).cuda())
+    want = np.where(lens > 0, u + lane_sums(rp, x[col], W), u)
+    ok = got.cpu().numpy() == want
+    if case == "given_hubs":
+        ok |= lens > 64
+    assert ok.all(), np.flatnonzero(~ok)[:5]
+
+
+@pytest.mark.parametrize("vertices", [3000, 200000])
+def test_captured_general_product_holds_no_allocation(cuda, vertices):
+    """Under capture the general path takes no scratch: the graph has only
+    kernels, so it can be a child of another graph; hub rows, with and without
+    the size that asks input bits in shared memory, give the direct bits."""
+    import ctypes as C
+
+    import torch
+    from alp_b200 import device as dev
+    cu = C.CDLL("libcuda.so.1")
+    rng = np.random.default_rng(vertices)
+    m = n = vertices
+    lens = np.minimum(rng.zipf(1.7, m) * 8, 3000)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    A = dev.from_host(m, n, rp, rng.integers(0, n, int(rp[-1])).astype(np.uint32), rng.random(int(rp[-1])))
+    assert vertices < 10000 or A.nnz > 1 << 21
+    plan = dev.Plan(A)
+    x = torch.from_numpy(rng.random(n)).cuda()
+    xa = torch.from_numpy((rng.random(n) < 0.3).astype(np.uint8)).cuda()
+    u, count = torch.zeros(m, dtype=torch.float64, device="cuda"), int(xa.sum())
+
+    def call():
+        dev.mxv(0, A, u, x, plan=plan, v_assigned=xa, v_count=count)
+
+    call()
+    want = u.clone()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        call()
+    raw, k = C.c_void_p(g.raw_cuda_graph()), C.c_size_t()
+    assert cu.cuGraphGetNodes(raw, None, C.byref(k)) == 0 and k.value >= 1
+    nodes = (C.c_void_p * k.value)()
+    assert cu.cuGraphGetNodes(raw, nodes, C.byref(k)) == 0
+    for node in nodes:
+        kind = C.c_int()
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        assert kind.value == 0      # CU_GRAPH_NODE_TYPE_KERNEL
+    parent, child, run = C.c_void_p(), C.c_void_p(), C.c_void_p()
+    assert cu.cuGraphCreate(C.byref(parent), 0) == 0
+    assert cu.cuGraphAddChildGraphNode(C.byref(child), parent, None, C.c_size_t(0), raw) == 0
+    assert cu.cuGraphInstantiateWithFlags(C.byref(run), parent, C.c_ulonglong(0)) == 0
+    for _ in range(2):
+        u.zero_()
+        torch.cuda.synchronize()
+        assert cu.cuGraphLaunch(run, C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(u, want)
+    assert cu.cuGraphExecDestroy(run) == 0 and cu.cuGraphDestroy(parent) == 0
