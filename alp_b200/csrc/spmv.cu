@@ -775,10 +775,10 @@ struct GenRow {
 
 // bits: which inputs take part, one bit each (v_assigned and the input mask
 // are then not read); null without BITS.
-template <class R, int W, bool BITS = false>
+template <class R, int W, bool BITS = false, int BATCH = BITS ? GEN_BATCH_BITS : GEN_BATCH>
 __device__ __forceinline__ void gen_gather(const SpmvArgs &a, int64_t b, int64_t e, int lane,
 	typename R::T &acc, bool &set, const uint32_t *bits = nullptr) {
-	constexpr int GEN_BATCH = BITS ? GEN_BATCH_BITS : ::alpb::GEN_BATCH;
+	constexpr int GEN_BATCH = BATCH;
 	using T = typename R::T;
 	const T *__restrict__ values = reinterpret_cast<const T *>(a.values);
 	const T *__restrict__ x = reinterpret_cast<const T *>(a.v);
@@ -846,10 +846,15 @@ struct GenChunks {
 template <class R, bool BITS>
 __device__ __forceinline__ void gen_chunk(const SpmvArgs &a, const GenRow<R> &row, int64_t c,
 	bool last, int wl, typename R::T &acc, bool &set, const uint32_t *bits = nullptr) {
-	const int64_t k0 = row.b + c * GEN_CHUNK;
-	if (row.row_ok)
-		gen_gather<R, 32, BITS>(a, k0, last || row.e < k0 + GEN_CHUNK ? row.e : k0 + GEN_CHUNK, wl,
-			acc, set, bits);
+	int64_t k0 = row.b + c * GEN_CHUNK;
+	const int64_t end = last || row.e < k0 + GEN_CHUNK ? row.e : k0 + GEN_CHUNK;
+	bool go = row.row_ok;
+	if (R::immutable && a.probe && go) {   // one nonzero a lane, then the rest
+		gen_gather<R, 32, BITS, 1>(a, k0, k0 + 32 < end ? k0 + 32 : end, wl, acc, set, bits);
+		go = !__any_sync(0xffffffffu, acc != R::zero());
+		k0 += 32;
+	}
+	if (go) gen_gather<R, 32, BITS>(a, k0, end, wl, acc, set, bits);
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o));
 	set = __any_sync(0xffffffffu, set);
@@ -972,7 +977,16 @@ k_spmv_vector_general(SpmvArgs a, GenChunks g, const uint32_t *__restrict__ gbit
 		T acc = R::zero();
 		bool set = false;
 		if (lane == 0) row.identity(a, acc, set);
-		if (row.row_ok) gen_gather<R, W, BITS>(a, row.b, row.e, lane, acc, set, gen_bits);
+		if (row.row_ok) {
+			int64_t k0 = row.b;
+			if (R::immutable && a.probe) {   // one nonzero a lane, then the rest
+				gen_gather<R, W, BITS, 1>(a, k0, k0 + W < row.e ? k0 + W : row.e, lane, acc, set,
+					gen_bits);
+				k0 += W;
+			}
+			if (!R::immutable || acc == R::zero())
+				gen_gather<R, W, BITS>(a, k0, row.e, lane, acc, set, gen_bits);
+		}
 #pragma unroll
 		for (int o = W / 2; o > 0; o >>= 1) {
 			acc = R::add(acc, __shfl_down_sync(0xffffffffu, acc, o, W));
@@ -1888,6 +1902,8 @@ int alpb_mxv(int ring, uint32_t descr, int form, int64_t m_out, int64_t n_in, in
 		}
 		if (a.scatter_sem) a.dense_all = false;
 	}
+	// many inputs take part: a row of lor is likely decided by its first nonzeroes
+	a.probe = (input_masked && !invert ? std::min(v_mask_count, v_count) : v_count) >= n_in / 4;
 	if (m_out == 0) return ALPB_SUCCESS;
 	return dispatch_spmv(ring, a, plan, 0, as_stream(stream));
 }

@@ -89,6 +89,7 @@ struct SpmvArgs {
 	// the scatter path applies add_identity outside the output mask and
 	// ignores explicit_zero.
 	bool mask_by_structure, scatter_sem;
+	bool probe;  // general path: look at a row's first nonzeroes alone
 };
 
 // Run one SpMV with the plan's schedule (force_sched != 0 overrides it).

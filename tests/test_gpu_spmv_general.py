@@ -248,3 +248,38 @@ def test_captured_general_product_holds_no_allocation(cuda, vertices):
         torch.cuda.synchronize()
         assert torch.equal(u, want)
     assert cu.cuGraphExecDestroy(run) == 0 and cu.cuGraphDestroy(parent) == 0
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("density", [0.3, 1.0])
+@pytest.mark.parametrize("true", [0.0, 0.02, 1.0])
+def test_boolean_rows_of_many_inputs(cuda, oracle, true, density, masked):
+    """From a quarter of the inputs on a boolean row is looked at by its first
+    nonzeroes alone before the rest: whichever nonzero decides it, and whether it
+    is assigned at all when none does."""
+    import torch
+    from alp_b200 import device as dev
+    rng = np.random.default_rng([int(100 * true), int(10 * density), masked])
+    n = 9001
+    lens = np.array(LENGTHS * 3)
+    lens = np.concatenate([lens, rng.integers(0, 60, 40000 if masked else 400)])
+    m = len(lens)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    col = rng.integers(0, n, int(rp[-1])).astype(np.uint32)
+    v = (rng.random(n) < true).astype(np.uint8)
+    va = (rng.random(n) < density).astype(np.uint8)
+    u, ua = (rng.random(m) < 0.1).astype(np.uint8), (rng.random(m) < 0.5).astype(np.uint8)
+    mask = (rng.random(m) < 0.6).astype(np.uint8)
+    T = lambda a: torch.from_numpy(a.copy()).cuda()  # noqa: E731
+    kw = dict(u_mask=mask, u_mask_assigned=mask, u_mask_count=int(mask.sum())) if masked else {}
+    wu, wa = u.copy(), ua.copy()
+    rc, wn = oracle.mxv(1, 0, 0, m, n, rp, col, None, 0, wu, wa, v=v, v_assigned=va, **kw)
+    assert rc == 0
+    A = dev.from_host(m, n, rp, col, None, 0)
+    for plan in (dev.Plan(A), dev.Plan(A, vector_width=8), None):
+        gu, ga = T(u), T(ua)
+        gn = torch.tensor([int(ua.sum())], dtype=torch.int64, device="cuda")
+        dev.mxv(1, A, gu, T(v), form=0, u_assigned=ga, u_nnz=gn, v_assigned=T(va), plan=plan,
+                **{k: T(a) if isinstance(a, np.ndarray) else a for k, a in kw.items()})
+        assert np.array_equal(ga.cpu().numpy() != 0, wa != 0) and int(gn) == wn
+        assert np.array_equal(gu.cpu().numpy()[wa != 0], wu[wa != 0])
