@@ -903,9 +903,10 @@ __device__ __forceinline__ void gen_long_row(const SpmvArgs &a, const GenChunks 
 // each.
 __global__ void k_pack_present(SpmvArgs a, uint32_t *bits) {
 	const int64_t n32 = (a.n_in + 31) / 32 * 32;
+	const uint8_t *va = (a.descr & ALPB_DESC_DENSE) ? nullptr : a.v_assigned;
 	for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < n32;
 		 j += int64_t(gridDim.x) * blockDim.x) {
-		const bool on = j < a.n_in && (a.v_assigned == nullptr || a.v_assigned[j] != 0) &&
+		const bool on = j < a.n_in && (va == nullptr || va[j] != 0) &&
 			(!a.input_masked || eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, j));
 		const unsigned w = __ballot_sync(0xffffffffu, on);
 		if ((threadIdx.x & 31) == 0) bits[j >> 5] = w;

@@ -283,3 +283,37 @@ def test_boolean_rows_of_many_inputs(cuda, oracle, true, density, masked):
                 **{k: T(a) if isinstance(a, np.ndarray) else a for k, a in kw.items()})
         assert np.array_equal(ga.cpu().numpy() != 0, wa != 0) and int(gn) == wn
         assert np.array_equal(gu.cpu().numpy()[wa != 0], wu[wa != 0])
+
+
+@pytest.mark.parametrize("ring", [0, 1, 2])
+def test_dense_descriptor_ignores_flags_at_every_size(cuda, oracle, ring):
+    """Under the dense descriptor the input's flags are not read, also where an
+    input mask is asked as bits (more than 2^21 nonzeroes).  Sums of up to 100
+    positive terms: FP64 orders agree to 2 * 100 * 2^-53."""
+    import torch
+    from alp_b200 import device as dev
+    vtype = {0: 3, 1: 1, 2: 2}[ring]
+    npt = {3: np.float64, 2: np.int32, 1: np.uint8}[vtype]
+    rng = np.random.default_rng(ring)
+    m, n = 60000, 20000
+    lens = rng.integers(0, 100, m)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    nnz = int(rp[-1])
+    assert nnz >= 1 << 21
+    col = rng.integers(0, n, nnz).astype(np.uint32)
+    value = lambda k: (rng.random(k) if vtype == 3 else rng.integers(0, 2 if vtype == 1 else 1000, k)).astype(npt)  # noqa: E731
+    vals, u, v = value(nnz), value(m), value(n)
+    vm = (rng.random(n) < 0.5).astype(np.uint8)
+    stale, full = np.zeros(n, np.uint8), np.ones(n, np.uint8)
+    A = dev.from_host(m, n, rp, col, vals, vtype)
+    T = lambda a: torch.from_numpy(a.copy()).cuda()  # noqa: E731
+    want = u.copy()
+    assert oracle.mxv(ring, 16, 0, m, n, rp, col, vals, vtype, want, v=v, v_assigned=full, v_mask=vm,
+                      v_mask_assigned=full, v_mask_count=n)[0] == 0
+    got = T(u)
+    dev.mxv(ring, A, got, T(v), descr=16, form=0, plan=dev.Plan(A), v_assigned=T(stale), v_count=n,
+            v_mask=T(vm), v_mask_assigned=T(full), v_mask_count=n)
+    if vtype == 3:
+        np.testing.assert_allclose(got.cpu().numpy(), want, rtol=3e-14, atol=0)
+    else:
+        np.testing.assert_array_equal(got.cpu().numpy(), want)
