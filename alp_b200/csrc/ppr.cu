@@ -36,6 +36,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 namespace alpb {
@@ -372,16 +373,18 @@ __device__ __forceinline__ void hp_load_seeds(const HpArgs &a, const HpLanes<G, 
 	}
 }
 
-// Chunk descriptor of the chunk loop (warp-uniform).
+// Chunk descriptor of the chunk loop (warp-uniform).  Row: see hp_late.
+template <class Row>
 struct HpMeta {
 	int64_t b;
-	uint32_t r;
+	Row r;
 	int len;
 	int32_t slot;
 };
 
-__device__ __forceinline__ HpMeta hp_meta(const HpArgs &a, int64_t c) {
-	HpMeta m{0, 0u, 0, -1};
+template <class Row>
+__device__ __forceinline__ HpMeta<Row> hp_meta(const HpArgs &a, int64_t c) {
+	HpMeta<Row> m{0, 0, 0, -1};
 	if (c < a.nchunks) {
 		m.b = __ldg(a.beg + c);
 		m.len = int(__ldg(a.beg + c + 1) - m.b);
@@ -389,6 +392,20 @@ __device__ __forceinline__ HpMeta hp_meta(const HpArgs &a, int64_t c) {
 		m.slot = __ldg(a.cslot + c);
 	}
 	return m;
+}
+
+// Late: a nonzero's weight is broadcast where it is used instead of with the
+// gathers, over which it would take two registers of each nonzero in flight,
+// and rows are numbered in 32 bits.  Which of the two the compiler turns into
+// the faster kernel differs (64 registers, with or without a few spills);
+// measured ms per iteration, weights with the gathers / late:
+//   seeds                    8      16      32      64     128
+//   forward  s22, s24     10.70   12.27   17.96   32.2    16.2 (s22)
+//                         10.47   12.80   16.76   30.1    18.3
+//   adjoint               11.04   12.55   17.46   31.5    15.8
+//                          9.35   11.49   16.47   32.0    18.1
+constexpr bool hp_late(int mode, int G, int SPL) {
+	return SPL == 1 ? !(mode == HP_FWD && G == 16) : SPL == 2 && mode != HP_ADJ;
 }
 
 // Main gather: one warp per chunk, chunks strided over the grid's warps.
@@ -401,6 +418,8 @@ template <int MODE, int G, int SPL>
 __global__ void __launch_bounds__(32 * HP_WARPS, ALPB_HP_MINB) k_hp_chunks(HpArgs a) {
 	constexpr int STEP = 32 / G;
 	constexpr int B = SPL >= 4 ? ALPB_HP_BATCH / 2 : ALPB_HP_BATCH;
+	constexpr bool LATE = hp_late(MODE, G, SPL);
+	using Row = std::conditional_t<LATE, uint32_t, int64_t>;
 	__shared__ double red[HP_WARPS * 2 * HP_MAX_SEEDS];
 	if (MODE != HP_MU && *a.sd.n_active == 0) return;
 	const HpLanes<G, SPL> L;
@@ -414,7 +433,7 @@ __global__ void __launch_bounds__(32 * HP_WARPS, ALPB_HP_MINB) k_hp_chunks(HpArg
 	for (int q = 0; q < SPL; ++q) res[q] = dng[q] = 0.0;
 	const int64_t nw = int64_t(gridDim.x) * HP_WARPS;
 	int64_t c = int64_t(blockIdx.x) * HP_WARPS + (threadIdx.x >> 5);
-	HpMeta m = hp_meta(a, c);
+	HpMeta<Row> m = hp_meta<Row>(a, c);
 	uint32_t myi = 0;
 	double myw = 0.0;
 	if (L.lane < m.len) {
@@ -422,18 +441,19 @@ __global__ void __launch_bounds__(32 * HP_WARPS, ALPB_HP_MINB) k_hp_chunks(HpArg
 		myw = __ldg(a.val + m.b + L.lane);
 	}
 	for (; c < a.nchunks; c += nw) {
-		const HpMeta mn = hp_meta(a, c + nw);
+		const HpMeta<Row> mn = hp_meta<Row>(a, c + nw);
 		HpEpiIn<SPL> e;
 		if (m.slot < 0) hp_epi_load<MODE>(a, L, m.r, e);
 		double acc[SPL];
 #pragma unroll
 		for (int q = 0; q < SPL; ++q) acc[q] = 0.0;
 		for (int t0 = 0; t0 < m.len; t0 += B * STEP) {
-			double v[B][SPL];
+			double v[B][SPL], wv[LATE ? 1 : B];
 #pragma unroll
 			for (int u = 0; u < B; ++u) {
 				const int t = t0 + u * STEP + L.gsub;
 				const uint32_t i = __shfl_sync(0xffffffffu, myi, t & 31);
+				if (!LATE) wv[u] = __shfl_sync(0xffffffffu, myw, t & 31);
 				const double *src = a.in + int64_t(i) * S;
 #pragma unroll
 				for (int q = 0; q < SPL; ++q) {
@@ -443,11 +463,9 @@ __global__ void __launch_bounds__(32 * HP_WARPS, ALPB_HP_MINB) k_hp_chunks(HpArg
 			}
 #pragma unroll
 			for (int u = 0; u < B; ++u) {
-				// the weight is broadcast where it is used: held over the gathers
-				// it would take two registers of each
-				const double wv = __shfl_sync(0xffffffffu, myw, (t0 + u * STEP + L.gsub) & 31);
+				if (LATE) wv[0] = __shfl_sync(0xffffffffu, myw, (t0 + u * STEP + L.gsub) & 31);
 #pragma unroll
-				for (int q = 0; q < SPL; ++q) acc[q] = fma(wv, v[u][q], acc[q]);
+				for (int q = 0; q < SPL; ++q) acc[q] = fma(wv[LATE ? 0 : u], v[u][q], acc[q]);
 			}
 		}
 		uint32_t ni = 0;
