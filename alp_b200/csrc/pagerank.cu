@@ -504,7 +504,12 @@ static int pagerank_steps(const PrStepArgs &tmpl, alpb_spmv_plan plan, int64_t *
 // Graphs from this many nonzeroes on take the per-step launches.  Measured us
 // per solve, one kernel against steps, R-MAT: 0.86 M nonzeroes 440 / 557, 1.2 M
 // 501 / 496, 2.1 M 750 / 715, 2.9 M 986 / 840, 4.3 M 1358 / 1005.
+// On stencils (the CCS plan's tiles hold whole columns) nothing crosses tiles and
+// the one kernel has no wait but its barrier: 27-point 1.6 M 608 / 932, 4.6 M
+// 1217 / 1426, 8.2 M 1921 / 2001, 13.5 M 3107 / 2992 (40 iterations), 5-point 4 M
+// 1400 / 1609, 7.2 M 2270 / 2348, 9.8 M 3003 / 2997.
 constexpr int64_t kPrStepNnz = int64_t(1) << 20;
+constexpr int64_t kPrStepNnzWhole = int64_t(1) << 23;
 
 // The solve proper.  plan: a WM_TILE plan of the CCS offsets, or null (one is
 // made and destroyed here); work: 3n doubles of scratch, or null.
@@ -522,7 +527,7 @@ static int pagerank_run(int64_t n, const int64_t *crs_row_ptr, const double *crs
 		if (rc != ALPB_SUCCESS) return rc;
 		plan = own_plan;
 	}
-	if (plan->nnz >= kPrStepNnz) {
+	if (plan->nnz >= (plan->tile_d ? kPrStepNnzWhole : kPrStepNnz)) {
 		double *vecs = work, *own_vecs = nullptr;
 		if (!vecs) {
 			ALPB_CUDA(cudaMallocAsync(&own_vecs, size_t(3 * n) * 8, s));
