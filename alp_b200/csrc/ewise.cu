@@ -389,16 +389,15 @@ struct ChainArgs {
 	T rident;
 };
 
-// op applied to VEC_BATCH pairs: one decision per step, not one per entry
-template <class T, class F>
-__device__ __forceinline__ void chain_each(T (&z)[VEC_BATCH], const T (&a)[VEC_BATCH],
-	const T (&b)[VEC_BATCH], const F &f) {
+// op applied to B pairs: one decision per step, not one per entry
+template <class T, int B, class F>
+__device__ __forceinline__ void chain_each(T (&z)[B], const T (&a)[B], const T (&b)[B],
+	const F &f) {
 #pragma unroll
-	for (int q = 0; q < VEC_BATCH; ++q) z[q] = f(a[q], b[q]);
+	for (int q = 0; q < B; ++q) z[q] = f(a[q], b[q]);
 }
-template <class T>
-__device__ __forceinline__ void chain_op(int op, T (&z)[VEC_BATCH], const T (&a)[VEC_BATCH],
-	const T (&b)[VEC_BATCH]) {
+template <class T, int B>
+__device__ __forceinline__ void chain_op(int op, T (&z)[B], const T (&a)[B], const T (&b)[B]) {
 	switch (op) {
 	case ALPB_OP_ADD: chain_each(z, a, b, [](T u, T v) { return opv(ALPB_OP_ADD, u, v); }); break;
 	case ALPB_OP_SUB: chain_each(z, a, b, [](T u, T v) { return opv(ALPB_OP_SUB, u, v); }); break;
@@ -407,55 +406,56 @@ __device__ __forceinline__ void chain_op(int op, T (&z)[VEC_BATCH], const T (&a)
 	}
 }
 
-// The entries i, i + S, ... of a thread, VEC_BATCH at a time.  The slots'
+// The entries i, i + S, ... of a thread, B at a time: VEC_BATCH of them, or one
+// while the vectors are so short that threads are left over (launch rule below).  The slots'
 // values wait in shared memory, [slot][batch][thread]: the steps name their
 // slots by number, and an array indexed so in registers went to local memory.
 // Two updates with a dot, a dot and two folds on 16e6 entries (1.3 GB): 791 us
 // then, 438 with one slot's loads waited for before the next, 391 now.
-template <class T>
+template <class T, int B>
 __global__ void __launch_bounds__(SCALAR_BLOCK, 4) k_vec_chain(ChainArgs<T> c, T init, VecOut out) {
 	extern __shared__ __align__(16) unsigned char chain_smem[];
 	T *v = reinterpret_cast<T *>(chain_smem) + threadIdx.x;
 	const auto at = [&](int slot, int q) -> T & {
-		return v[(slot * VEC_BATCH + q) * SCALAR_BLOCK];
+		return v[(slot * B + q) * SCALAR_BLOCK];
 	};
 	T acc = c.rident;
 	const int64_t S = int64_t(gridDim.x) * blockDim.x;
 	for (int64_t i0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i0 < c.n;
-		 i0 += VEC_BATCH * S) {
+		 i0 += B * S) {
 		// four slots' loads before the first of them is put down (every type is
 		// the domain's own)
 #pragma unroll
 		for (int h = 0; h < ALPB_CHAIN_SLOTS; h += 4) {
-			T t[4][VEC_BATCH];
+			T t[4][B];
 #pragma unroll
 			for (int s = 0; s < 4; ++s)
 				if (h + s < c.nslots && ((c.load >> (h + s)) & 1)) {
 					const T *p = static_cast<const T *>(c.val[h + s]);
 #pragma unroll
-					for (int q = 0; q < VEC_BATCH; ++q)
+					for (int q = 0; q < B; ++q)
 						t[s][q] = i0 + q * S < c.n ? p[i0 + q * S] : T(0);
 				}
 #pragma unroll
 			for (int s = 0; s < 4; ++s)
 				if (h + s < c.nslots && ((c.load >> (h + s)) & 1)) {
 #pragma unroll
-					for (int q = 0; q < VEC_BATCH; ++q) at(h + s, q) = t[s][q];
+					for (int q = 0; q < B; ++q) at(h + s, q) = t[s][q];
 				}
 		}
-		const auto get = [&](int slot, T scalar, T (&t)[VEC_BATCH]) {
+		const auto get = [&](int slot, T scalar, T (&t)[B]) {
 #pragma unroll
-			for (int q = 0; q < VEC_BATCH; ++q) t[q] = slot >= 0 ? at(slot, q) : scalar;
+			for (int q = 0; q < B; ++q) t[q] = slot >= 0 ? at(slot, q) : scalar;
 		};
 		for (int k = 0; k < c.nsteps; ++k) {
 			const ChainStep<T> &o = c.step[k];
-			T x[VEC_BATCH], y[VEC_BATCH], z[VEC_BATCH];
+			T x[B], y[B], z[B];
 			get(o.x, o.alpha, x);
 			if (o.kind != ALPB_VEC_SET) get(o.z, T(0), z);
 			switch (o.kind) {
 			case ALPB_VEC_SET:
 #pragma unroll
-				for (int q = 0; q < VEC_BATCH; ++q) z[q] = o.use_index ? T(i0 + q * S) : x[q];
+				for (int q = 0; q < B; ++q) z[q] = o.use_index ? T(i0 + q * S) : x[q];
 				break;
 			case ALPB_VEC_FOLDL: chain_op(o.op, z, z, x); break;
 			case ALPB_VEC_FOLDR: chain_op(o.op, z, x, z); break;
@@ -466,21 +466,21 @@ __global__ void __launch_bounds__(SCALAR_BLOCK, 4) k_vec_chain(ChainArgs<T> c, T
 				break;
 			}
 #pragma unroll
-			for (int q = 0; q < VEC_BATCH; ++q) at(o.z, q) = z[q];
+			for (int q = 0; q < B; ++q) at(o.z, q) = z[q];
 		}
 		if (c.reduce) {   // as k_vec_dot on dense operands
-			T x[VEC_BATCH], y[VEC_BATCH];
+			T x[B], y[B];
 			get(c.rx, T(0), x);
 			get(c.ry, T(0), y);
 			if (c.ry >= 0) chain_op(c.rmul, x, x, y);
 #pragma unroll
-			for (int q = 0; q < VEC_BATCH; ++q)
+			for (int q = 0; q < B; ++q)
 				if (i0 + q * S < c.n) acc = opv(c.radd, acc, x[q]);
 		}
 		for (int s = 0; s < c.nslots; ++s)
 			if ((c.store >> s) & 1) {
 #pragma unroll
-				for (int q = 0; q < VEC_BATCH; ++q)
+				for (int q = 0; q < B; ++q)
 					if (i0 + q * S < c.n) static_cast<T *>(c.val[s])[i0 + q * S] = at(s, q);
 			}
 	}
@@ -493,6 +493,11 @@ static bool domain_type(int domain, int type) {
 	return type == domain || (domain == ALPB_UINT64 && type == ALPB_INT64) ||
 		(domain == ALPB_INT64 && type == ALPB_UINT64);
 }
+
+// Chains without a reduction on up to this many entries run an entry per thread.
+// us, before four were taken at a time / four / one, eight updates: 1,000 entries 6.5 / 8.4
+// / 3.9, 100,000 7.4 / 8.7 / 5.1, 300,000 14.1 / 9.8 / 10.5.
+constexpr int64_t CHAIN_ONE = int64_t(1) << 17;
 
 template <class T>
 static int vec_chain_run(int domain, int64_t n, int nslots, void *const *values,
@@ -555,15 +560,21 @@ static int vec_chain_run(int domain, int64_t n, int nslots, void *const *values,
 	}
 	c.store = written;
 	const size_t smem = size_t(nslots) * VEC_BATCH * SCALAR_BLOCK * sizeof(T);
+	if (!c.reduce && n <= CHAIN_ONE) {
+		k_vec_chain<T, 1><<<grid_for(n, SCALAR_BLOCK), SCALAR_BLOCK, smem / VEC_BATCH, s>>>(c, T(0),
+			VecOut{});
+		ALPB_LAUNCHED();
+		return ALPB_SUCCESS;
+	}
 	// Without the opt-in a launch has 48 KB, the kernel's own static shared memory
 	// included: six slots of 8 bytes are past it.  Every call asks for the most any
 	// chain takes, so that no thread's call lowers the limit under another's.
 	if (smem > 40 * 1024)
-		ALPB_CUDA(cudaFuncSetAttribute(k_vec_chain<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			int(ALPB_CHAIN_SLOTS * VEC_BATCH * SCALAR_BLOCK * sizeof(T))));
+		ALPB_CUDA(cudaFuncSetAttribute(k_vec_chain<T, VEC_BATCH>,
+			cudaFuncAttributeMaxDynamicSharedMemorySize, int(ALPB_CHAIN_SLOTS * VEC_BATCH * SCALAR_BLOCK * sizeof(T))));
 	if (!c.reduce) {
-		k_vec_chain<T><<<grid_for((n + VEC_BATCH - 1) / VEC_BATCH, SCALAR_BLOCK), SCALAR_BLOCK, smem,
-			s>>>(c, T(0), VecOut{});
+		k_vec_chain<T, VEC_BATCH><<<grid_for((n + VEC_BATCH - 1) / VEC_BATCH, SCALAR_BLOCK),
+			SCALAR_BLOCK, smem, s>>>(c, T(0), VecOut{});
 		ALPB_LAUNCHED();
 		return ALPB_SUCCESS;
 	}
@@ -573,7 +584,7 @@ static int vec_chain_run(int domain, int64_t n, int nslots, void *const *values,
 	if (rc != ALPB_SUCCESS) return rc;
 	T init;
 	memcpy(&init, result, sizeof(T));
-	k_vec_chain<T><<<scalar_grid(n), SCALAR_BLOCK, smem, s>>>(c, init,
+	k_vec_chain<T, VEC_BATCH><<<scalar_grid(n), SCALAR_BLOCK, smem, s>>>(c, init,
 		VecOut{sc.part, sc.arrived, sc.host_dev});
 	ALPB_LAUNCHED();
 	ALPB_CUDA(cudaStreamSynchronize(s));

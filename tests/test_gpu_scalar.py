@@ -211,3 +211,26 @@ def test_chains_of_every_length(cuda):
     p = subprocess.run([sys.executable, "-c", CHAINS], capture_output=True, text=True, timeout=300,
                        cwd=Path(__file__).resolve().parent.parent)
     assert p.returncode == 0 and "chains ok" in p.stdout, p.stdout + p.stderr
+
+
+@pytest.mark.parametrize("n", [131071, 131072, 131073, 131072 + 1024])
+def test_chains_around_one_entry_per_thread(cuda, n):
+    """Chains without a reduction take one entry a thread up to 131,072 entries,
+    four beyond."""
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    rng = np.random.default_rng(n)
+    v = [rng.integers(-1000, 1000, n) for _ in range(3)]
+    t = [torch.from_numpy(a.copy()).cuda() for a in v]
+    S = abi.VecStep
+    steps = [S(kind=abi.VEC_SET, z=2, x=-1, y=-1, descr=abi.DESC_USE_INDEX),
+             S(kind=abi.VEC_MULADD, op=abi.OP_ADD, mul_op=abi.OP_MUL, z=0, x=1, y=2),
+             S(kind=abi.VEC_FOLDR, op=abi.OP_SUB, z=1, x=0, y=-1)]
+    abi.call("alpb_vec_chain", abi.INT64, n, 3, (C.c_void_p * 3)(*[a.data_ptr() for a in t]),
+             (C.c_int * 3)(*[abi.INT64] * 3), 3, (S * 3)(*steps), None, dev.stream_ptr())
+    v[2] = np.arange(n)
+    v[0] = v[0] + v[1] * v[2]
+    v[1] = v[0] - v[1]
+    for a, b in zip(t, v):
+        assert np.array_equal(a.cpu().numpy(), b)
