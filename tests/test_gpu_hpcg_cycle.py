@@ -94,8 +94,8 @@ def test_cycle_matches_restatement(cuda, dims, levels, colors, pre, post, nrhs):
 
 @pytest.mark.parametrize("colors", [27, 16])
 def test_large_level_by_launches(cuda, colors):
-    """A finest level of more than 2^25 values (a launch per step), its coarse
-    level in the cycle kernel; in place (27 colours), and with neighbours of one
+    """A finest level of more than 100,000 warps' worth of rows per colour step (a
+    launch per step), its coarse level in the cycle kernel; in place (27 colours), and with neighbours of one
     colour (16)."""
     import torch
     from alp_b200 import _abi as abi
@@ -142,3 +142,36 @@ def test_right_hand_sides_stop_on_their_own(cuda):
     (mixed, xm), (first, xf), (second, xs) = out
     assert mixed == [first[0], second[1]] and max(mixed) > 4
     assert np.array_equal(xm[:, 0], xf[:, 0]) and np.array_equal(xm[:, 1], xs[:, 1])
+
+
+@pytest.mark.parametrize("nrhs,dims", [(8, (48, 48, 48)), (8, (51, 51, 53)), (4, (80, 80, 81)),
+                                       (4, (81, 81, 81)), (2, (20, 21, 22)), (1, (20, 21, 22))])
+def test_plain_iterations(cuda, nrhs, dims):
+    """Without the preconditioner, on both sides of the size from which A p is a
+    walk over the rows with a pass for the dot product (rows times right-hand
+    sides squared above 2^23).  Six iterations of a contraction, sums of 27 terms
+    and of n products: 1e-12 of x as above."""
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    n = int(np.prod(dims))
+    b = np.random.default_rng([n, nrhs]).standard_normal((n, nrhs))
+    h = C.c_void_p()
+    abi.call("alpb_hpcg_create", C.byref(h), *dims, 26.0, -1.0, 27, 4, 0, nrhs, dev.stream_ptr())
+    tb = torch.from_numpy(b.reshape(-1).copy()).cuda()
+    x = torch.zeros_like(tb)
+    it, res = (C.c_int64 * nrhs)(), (C.c_double * nrhs)()
+    abi.call("alpb_hpcg_solve", h, dev.ptr(tb), dev.ptr(x), 0, 1, 1, 6, 1e-30, it, res,
+             dev.stream_ptr())
+    abi.lib().alpb_hpcg_destroy(h)
+    A, want, r = stencil(*dims), np.zeros_like(b), b.copy()
+    p, rr = r.copy(), (r * r).sum(0)
+    for _ in range(6):
+        ap = A @ p
+        alpha = rr / (p * ap).sum(0)
+        want += alpha * p
+        r -= alpha * ap
+        new = (r * r).sum(0)
+        p, rr = r + new / rr * p, new
+    assert list(it) == [6] * nrhs
+    assert np.abs(x.cpu().numpy().reshape(n, nrhs) - want).max() <= 1e-12 * np.abs(want).max()
