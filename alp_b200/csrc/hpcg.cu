@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(HGC_THREADS, 1) k_hpcg_cycle(HgCycleArgs a) {
 // memory, and every warp that an SM can hold counts more than the loads each
 // has in flight: such levels run a launch per step, 8 lanes per row, lane
 // (s, k) of the group walking the entries s, s + S, ... of right-hand side k,
-// in 32 registers.  HG_LARGE_VALUES below says which levels these are, and the
+// in 32 registers.  hg_by_launches below says which levels these are, and the
 // times of both sides.
 constexpr int HG_GROUP = 8;     // lanes per matrix row
 template <int NRHS, class Op>
@@ -672,6 +672,7 @@ struct alpb_hpcg_s {
 	GridSync *gs = nullptr;      // the cycle kernel's barrier
 	int32_t *active = nullptr;   // right-hand sides still iterating
 	int cluster_fits = -1;       // coarse levels in one cluster: -1 not asked yet
+	int cycle_fits = -1;         // the cycle kernel's blocks all resident: the same
 	int dot_blocks = 0;
 };
 
@@ -738,11 +739,32 @@ static int hg_cycle_part(alpb_hpcg_s *h, HgCycleArgs &a, int l0, int l1, int par
 	return ALPB_SUCCESS;
 }
 
-// Levels of more values than this (256 MB of x, twice the L2) run a launch per
-// step.  The line lies between 128^3 x 8 = 2^24, where the cycle kernel takes
-// 8.4 ms per iteration and launches 9.3, and 256^3 x 8 = 2^27, where it takes
-// 55.1 and launches 52.1; sizes between were not measured.
-constexpr int64_t HG_LARGE_VALUES = int64_t(1) << 25;
+// Levels whose colour steps hold more than this many warps' worth of rows run a
+// launch per step: what the cycle kernel saves is the launch and a step's latency,
+// and beyond this the warps that an SM can hold count more.  Measured us per
+// iteration, cycle kernel / launches (items per step of the finest level):
+//   8 right-hand sides: 128^3 (78 K) 8434 / 9536, 160 x 144^2 (123 K) 12987 / 12875,
+//     160^3 (152 K) 15020 / 14338, 192^3 (262 K) 26408 / 24727
+//   4: 128^3 (78 K) 6694 / 7069, 144^3 (111 K) 9907 / 9384, 160^3 (152 K) 12205 / 10293
+//   2: 160^3 (76 K) 7617 / 7524, 192^3 (131 K) 11983 / 10650; 8 colours 128^3 (131 K)
+//     3899 / 3317
+// With one right-hand side a warp takes four rows in both, and the cycle kernel
+// stays ahead: 256^3 (155 K) 17359 / 19387, 384^3 (524 K) 59445 / 63526; but not where
+// a step is two passes: one colour, 96^3 (221 K) 710 / 684.
+constexpr int64_t HG_STEP_ITEMS = 100000;
+
+// Whether level L runs by launches (also where the cycle kernel's one block per
+// SM cannot be resident; asked once per handle).
+template <int NRHS>
+static bool hg_by_launches(alpb_hpcg_s *h, const HgLevel &L) {
+	if (h->cycle_fits < 0) {
+		h->cycle_fits = cooperative_grid(k_hpcg_cycle<NRHS, false>, HGC_THREADS, 0, 0) >= sm_count();
+		cudaGetLastError();
+	}
+	if (!h->cycle_fits) return true;
+	const int64_t rows = (L.n + h->colors - 1) / h->colors;
+	return (NRHS > 1 || !L.fused) && rows / HgRow<NRHS>::RPW > HG_STEP_ITEMS;
+}
 
 template <int NRHS, class Op>
 static int hg_rows(const HgLevel &L, const double *x, int64_t count, const Op &op, cudaStream_t s) {
@@ -780,7 +802,7 @@ static int hg_vcycle(alpb_hpcg_s *h, int l, int64_t pre, int64_t post, cudaStrea
 	HgLevel &L = h->levels[size_t(l)];
 	ALPB_CUDA(cudaMemsetAsync(L.z, 0, size_t(L.n) * NRHS * 8, s));
 	int rc = ALPB_SUCCESS;
-	if (L.n * NRHS > HG_LARGE_VALUES) {
+	if (hg_by_launches<NRHS>(h, L)) {
 		if (l + 1 == nl) return hg_smoother<NRHS>(h, L, s);
 		for (int64_t i = 0; i < pre && rc == ALPB_SUCCESS; ++i) rc = hg_smoother<NRHS>(h, L, s);
 		if (rc != ALPB_SUCCESS) return rc;
@@ -877,7 +899,7 @@ static int hg_solve(alpb_hpcg_s *h, const double *b, double *x, bool preconditio
 	HgScalars hs[NRHS];
 	GridSync hgs;
 	// a large system's iteration is worth far more than a look at the state
-	const int64_t queue = n * NRHS > HG_LARGE_VALUES ? 1 : HG_QUEUE;
+	const int64_t queue = precondition && hg_by_launches<NRHS>(h, L) ? 1 : HG_QUEUE;
 	for (int64_t iter = 0;; ++iter) {
 		if (precondition) {
 			rc = hg_vcycle<NRHS>(h, 0, pre, post, s);
