@@ -315,7 +315,9 @@ constexpr int HG_GROUP = 8;     // lanes per matrix row
 template <int NRHS, class Op>
 __global__ void __launch_bounds__(HG_BLOCK, 8)
 k_hpcg_rows(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ indices,
-	const double *__restrict__ values, const double *__restrict__ x, int64_t count, Op op) {
+	const double *__restrict__ values, const double *__restrict__ x, int64_t count, Op op,
+	const int32_t *active) {
+	if (active && *active == 0) return;   // no right-hand side still iterates
 	constexpr int S = HG_GROUP / NRHS;
 	constexpr int PARTS = NRHS < 4 ? 1 : NRHS / 2;   // of a lane's sum: 27 terms in one round more
 	constexpr int GPW = 32 / HG_GROUP;  // row groups per warp
@@ -435,11 +437,13 @@ __device__ __forceinline__ void hg_block_partials(double acc, double *partials) 
 	if (threadIdx.x < NRHS) partials[blockIdx.x * NRHS + threadIdx.x] = sm[threadIdx.x];
 }
 
-// partials of x_k . y_k
+// partials of x_k . y_k (the vector steps return at once where `active` is given
+// and no right-hand side still iterates: the host looks every few iterations)
 template <int NRHS>
 __global__ void __launch_bounds__(HG_BLOCK)
 k_hpcg_dot(const double *__restrict__ x, const double *__restrict__ y, int64_t n,
-	double *partials) {
+	double *partials, const int32_t *active) {
+	if (active && *active == 0) return;
 	double acc = 0.0;
 	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n * NRHS;
 		 i += int64_t(gridDim.x) * blockDim.x)
@@ -452,7 +456,8 @@ template <int NRHS>
 __global__ void __launch_bounds__(HG_BLOCK)
 k_hpcg_spmm(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ indices,
 	const double *__restrict__ values, const double *__restrict__ x, double *__restrict__ y,
-	int64_t n, double *partials) {
+	int64_t n, double *partials, const int32_t *active) {
+	if (active && *active == 0) return;
 	using Row = HgRow<NRHS>;
 	const int k = threadIdx.x % NRHS;
 	const int64_t warp = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
@@ -480,7 +485,8 @@ struct HgScalars {
 
 template <int NRHS>
 __global__ void k_hpcg_axpby(double *out, const double *a, const double *b, const HgScalars *sc,
-	int which, int64_t n) {
+	int which, int64_t n, const int32_t *active) {
+	if (active && *active == 0) return;
 	// which 0: out = b - a   (r = b - Ap, eWiseApply with minus)
 	//       1: out = beta a + b  (Ap = beta p + z, eWiseMulAdd into a cleared vector)
 	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n * NRHS;
@@ -496,7 +502,8 @@ __global__ void k_hpcg_axpby(double *out, const double *a, const double *b, cons
 template <int NRHS>
 __global__ void __launch_bounds__(HG_BLOCK)
 k_hpcg_update(double *x, double *r, const double *p, const double *ap,
-	const HgScalars *sc, int64_t n, double *partials) {
+	const HgScalars *sc, int64_t n, double *partials, const int32_t *active) {
+	if (*active == 0) return;
 	double acc = 0.0;
 	for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n * NRHS;
 		 i += int64_t(gridDim.x) * blockDim.x) {
@@ -767,10 +774,11 @@ static bool hg_by_launches(alpb_hpcg_s *h, const HgLevel &L) {
 }
 
 template <int NRHS, class Op>
-static int hg_rows(const HgLevel &L, const double *x, int64_t count, const Op &op, cudaStream_t s) {
+static int hg_rows(const HgLevel &L, const double *x, int64_t count, const Op &op, cudaStream_t s,
+	const int32_t *active = nullptr) {
 	if (count <= 0) return ALPB_SUCCESS;
 	k_hpcg_rows<NRHS, Op><<<grid_for(count * HG_GROUP, HG_BLOCK), HG_BLOCK, 0, s>>>(L.offsets,
-		L.indices, L.values, x, count, op);
+		L.indices, L.values, x, count, op, active);
 	ALPB_LAUNCHED();
 	return ALPB_SUCCESS;
 }
@@ -847,8 +855,9 @@ static int hg_finish(alpb_hpcg_s *h, int step, int64_t iter, int64_t max_iter, d
 }
 
 template <int NRHS>
-static int hg_dot(alpb_hpcg_s *h, const double *x, const double *y, cudaStream_t s) {
-	k_hpcg_dot<NRHS><<<h->dot_blocks, HG_BLOCK, 0, s>>>(x, y, h->levels[0].n, h->partials);
+static int hg_dot(alpb_hpcg_s *h, const double *x, const double *y, cudaStream_t s,
+	const int32_t *active) {
+	k_hpcg_dot<NRHS><<<h->dot_blocks, HG_BLOCK, 0, s>>>(x, y, h->levels[0].n, h->partials, active);
 	ALPB_LAUNCHED();
 	return ALPB_SUCCESS;
 }
@@ -861,20 +870,21 @@ static int hg_dot(alpb_hpcg_s *h, const double *x, const double *y, cudaStream_t
 // 596 / 635; 1: 160^3 479 / 362, 256^3 2078 / 1497.
 constexpr int64_t HG_WALK = int64_t(1) << 23;   // rows * nrhs^2
 template <int NRHS>
-static int hg_spmm(alpb_hpcg_s *h, const double *x, cudaStream_t s) {
+static int hg_spmm(alpb_hpcg_s *h, const double *x, cudaStream_t s, const int32_t *active) {
 	const HgLevel &L = h->levels[0];
 	if (NRHS > 1 && L.n * NRHS * NRHS > HG_WALK) {
-		const int rc = hg_rows<NRHS>(L, x, L.n, HgSpmm<NRHS>{h->ap}, s);
-		return rc ? rc : hg_dot<NRHS>(h, x, h->ap, s);
+		const int rc = hg_rows<NRHS>(L, x, L.n, HgSpmm<NRHS>{h->ap}, s, active);
+		return rc ? rc : hg_dot<NRHS>(h, x, h->ap, s, active);
 	}
 	k_hpcg_spmm<NRHS><<<h->dot_blocks, HG_BLOCK, 0, s>>>(L.offsets, L.indices, L.values, x, h->ap,
-		L.n, h->partials);
+		L.n, h->partials, active);
 	ALPB_LAUNCHED();
 	return ALPB_SUCCESS;
 }
 
-// Iterations queued before the host looks whether any right-hand side is left
-// (the kernels of an iteration too many find none and return).
+// The host looks whether any right-hand side is left after the first and every
+// HG_QUEUE-th iteration: a look takes about 30 us, and the kernels of an iteration
+// too many find none and return.
 constexpr int64_t HG_QUEUE = 4;
 
 // algorithms::hpcg (hpcg.hpp:97-223) for NRHS right-hand sides at once
@@ -889,11 +899,11 @@ static int hg_solve(alpb_hpcg_s *h, const double *b, double *x, bool preconditio
 	ALPB_CUDA(cudaMemsetAsync(h->active, 0, 4, s));
 	// Ap = 0; r = 0; p = x; Ap = A x; r = b - Ap; norm = sqrt(r.r)
 	ALPB_CUDA(cudaMemcpyAsync(h->p, x, size_t(n) * NRHS * 8, cudaMemcpyDeviceToDevice, s));
-	int rc = hg_spmm<NRHS>(h, x, s);
+	int rc = hg_spmm<NRHS>(h, x, s, nullptr);
 	if (rc != ALPB_SUCCESS) return rc;
-	k_hpcg_axpby<NRHS><<<g, 256, 0, s>>>(L.r, h->ap, b, h->scalars, 0, n);
+	k_hpcg_axpby<NRHS><<<g, 256, 0, s>>>(L.r, h->ap, b, h->scalars, 0, n, nullptr);
 	ALPB_LAUNCHED();
-	rc = hg_dot<NRHS>(h, L.r, L.r, s);
+	rc = hg_dot<NRHS>(h, L.r, L.r, s, nullptr);
 	rc = rc ? rc : hg_finish<NRHS>(h, 0, 0, max_iter, tol, s);
 	if (rc != ALPB_SUCCESS) return rc;
 	HgScalars hs[NRHS];
@@ -908,29 +918,29 @@ static int hg_solve(alpb_hpcg_s *h, const double *b, double *x, bool preconditio
 			ALPB_CUDA(cudaMemcpyAsync(L.z, L.r, size_t(n) * NRHS * 8, cudaMemcpyDeviceToDevice, s));
 		}
 		// r.z, beta; p = z (first iteration) or p = beta p + z
-		rc = hg_dot<NRHS>(h, L.r, L.z, s);
+		rc = hg_dot<NRHS>(h, L.r, L.z, s, h->active);
 		rc = rc ? rc : hg_finish<NRHS>(h, 1, iter, max_iter, tol, s);
 		if (rc != ALPB_SUCCESS) return rc;
 		if (iter == 0) {
 			ALPB_CUDA(cudaMemcpyAsync(h->p, L.z, size_t(n) * NRHS * 8, cudaMemcpyDeviceToDevice, s));
 		} else {
 			// into Ap, then swapped with p (hpcg.hpp:193-196)
-			k_hpcg_axpby<NRHS><<<g, 256, 0, s>>>(h->ap, h->p, L.z, h->scalars, 1, n);
+			k_hpcg_axpby<NRHS><<<g, 256, 0, s>>>(h->ap, h->p, L.z, h->scalars, 1, n, h->active);
 			ALPB_LAUNCHED();
 			double *t = h->p;
 			h->p = h->ap;
 			h->ap = t;
 		}
 		// Ap = A p; alpha = r.z / p.Ap; x += alpha p; r -= alpha Ap; norm
-		rc = hg_spmm<NRHS>(h, h->p, s);
+		rc = hg_spmm<NRHS>(h, h->p, s, h->active);
 		rc = rc ? rc : hg_finish<NRHS>(h, 2, iter, max_iter, tol, s);
 		if (rc != ALPB_SUCCESS) return rc;
 		k_hpcg_update<NRHS><<<h->dot_blocks, HG_BLOCK, 0, s>>>(x, L.r, h->p, h->ap, h->scalars, n,
-			h->partials);
+			h->partials, h->active);
 		ALPB_LAUNCHED();
 		rc = hg_finish<NRHS>(h, 3, iter, max_iter, tol, s);
 		if (rc != ALPB_SUCCESS) return rc;
-		if (iter % queue != queue - 1 && iter + 1 < max_iter) continue;
+		if (iter >= 1 && iter % queue != queue - 1 && iter + 1 < max_iter) continue;
 		ALPB_CUDA(cudaMemcpyAsync(hs, h->scalars, sizeof(hs), cudaMemcpyDeviceToHost, s));
 		ALPB_CUDA(cudaMemcpyAsync(&hgs, h->gs, sizeof(hgs), cudaMemcpyDeviceToHost, s));
 		ALPB_CUDA(cudaStreamSynchronize(s));

@@ -175,3 +175,34 @@ def test_plain_iterations(cuda, nrhs, dims):
         p, rr = r + new / rr * p, new
     assert list(it) == [6] * nrhs
     assert np.abs(x.cpu().numpy().reshape(n, nrhs) - want).max() <= 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("precondition", [0, 1])
+@pytest.mark.parametrize("last", [1, 2, 3, 5])
+def test_solve_ends_where_it_converges(cuda, last, precondition):
+    """A solve that converges on iteration `last` leaves what that many iterations
+    leave, whatever was queued behind it."""
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    dims, nrhs = (24, 16, 32), 4
+    n = int(np.prod(dims))
+    b = torch.from_numpy(np.repeat(np.random.default_rng(last).standard_normal(n), nrhs)).cuda()
+
+    def solve(max_iter, tol):
+        h, x = C.c_void_p(), torch.zeros_like(b)
+        abi.call("alpb_hpcg_create", C.byref(h), *dims, 26.0, -1.0, 27, 4, 1, nrhs, dev.stream_ptr())
+        it, res = (C.c_int64 * nrhs)(), (C.c_double * nrhs)()
+        abi.call("alpb_hpcg_solve", h, dev.ptr(b), dev.ptr(x), precondition, 1, 1, max_iter, tol, it,
+                 res, dev.stream_ptr())
+        abi.lib().alpb_hpcg_destroy(h)
+        return x, list(it), list(res)
+
+    want = solve(last, 1e-30)
+    norm = float(b.view(n, nrhs)[:, 0].norm())
+    tol = want[2][0] / norm * 1.0001
+    for k in range(1, last):
+        assert solve(k, 1e-30)[2][0] / norm > tol
+    got = solve(100, tol)
+    assert got[1] == want[1] == [last] * nrhs
+    assert torch.equal(got[0], want[0]) and got[2] == want[2]
