@@ -269,15 +269,50 @@ static CgRowsShape cg_rows_shape(int64_t n, int maxlen) {
 	return c;
 }
 
+// Entries outside shared memory: 12 bytes each, a second copy of that part of
+// the matrix, padded to the longest row.
+static size_t cg_rows_ell(const CgRowsShape &c) {
+	return size_t(c.grid) * size_t(c.items - c.resident) * size_t(c.steps) * 32;
+}
+
+// Largest workspace: after alpb_init the stream-ordered pool keeps it for the next
+// solve, so it is bounded.  (To hand one back after every solve costs 10 ms per GB:
+// 27-point 160^3, 1.3 GB, 50 iterations 20.2 -> 28.3 ms, k_cg 31.1; 256^3, 5.4 GB,
+// 84 -> 142, k_cg 128.)
+constexpr size_t CGR_MAX = size_t(8) << 30;
+
+// Whether k_cg_rows is worth its set-up and its padding.  Measured us, k_cg /
+// k_cg_rows:
+//  - the rewriting takes longer than a few iterations win where most of it goes to
+//    memory and rows are long (27-point 64^3, 88 MB: 1 iteration 143 / 180, 2 180 / 192,
+//    4 274 / 229; 128^3: 1 627 / 1106, 4 1548 / 1692, 8 2785 / 2470; 256^3: 4 12359 /
+//    13250, 50 128344 / 84491; 5-point rows break even at one);
+//  - padded entries are read as the others are, and from some size on that is what
+//    an iteration costs (8 to 24 random columns a row, half as many again: 1 M rows,
+//    288 MB, 2990 / 2867 per 20 iterations, 3 M rows, 864 MB, 9153 / 10522).
+static bool cg_rows_pays(const CgRowsShape &c, int64_t nnz, int64_t max_iter) {
+	const size_t bytes = cg_rows_ell(c) * 12;
+	if (bytes == 0) return true;
+	if (bytes > CGR_MAX) return false;
+	if (c.steps * c.L > 8 && max_iter < (bytes > (size_t(128) << 20) ? 5 : 3)) return false;
+	const double padded = double(c.grid) * c.items * c.steps * 32;
+	return bytes <= (size_t(512) << 20) || padded <= 1.25 * double(nnz);
+}
+
 // The solve on k_cg_rows; ALPB_UNSUPPORTED (nothing launched) when its
-// workspace cannot be had, and the caller runs k_cg instead.
+// workspace cannot be had or its blocks cannot be resident together, and the
+// caller runs k_cg instead.
 template <int L>
 static int cg_rows_solve(const CgRowsShape &c, CgRowsArgs a, double *wk, cudaStream_t s,
 	CgState *h) {
 	static std::atomic<unsigned long long> allowed_in;
 	ALPB_CUDA(allow_smem(k_cg_rows<L>, CGR_SMEM, allowed_in));
+	if (cooperative_grid(k_cg_rows<L>, CGR_THREADS, c.smem, c.grid) < c.grid) {
+		cudaGetLastError();
+		return ALPB_UNSUPPORTED;
+	}
 	const int64_t n = a.n;
-	const size_t ell = size_t(c.grid) * size_t(c.items - c.resident) * size_t(c.steps) * 32;
+	const size_t ell = cg_rows_ell(c);
 	// one allocation: state, partials, the items outside shared memory, r
 	const size_t head = (sizeof(GridReduce) + sizeof(CgState) + 255) / 256 * 256;
 	const size_t bytes = head + ell * 12 + (c.vec_smem ? 0 : size_t(n) * 8);
@@ -302,8 +337,15 @@ static int cg_rows_solve(const CgRowsShape &c, CgRowsArgs a, double *wk, cudaStr
 	a.vec_smem = c.vec_smem;
 	ALPB_CUDA(cudaMemsetAsync(ws, 0, head, s));
 	void *args[] = {&a};
-	ALPB_CUDA(cudaLaunchCooperativeKernel((void *) k_cg_rows<L>, dim3(c.grid), dim3(CGR_THREADS),
-		args, c.smem, s));
+	const cudaError_t e = cudaLaunchCooperativeKernel((void *) k_cg_rows<L>, dim3(c.grid),
+		dim3(CGR_THREADS), args, c.smem, s);
+	if (e != cudaSuccess) {
+		cudaGetLastError();
+		cudaFreeAsync(ws, s);
+		if (e == cudaErrorCooperativeLaunchTooLarge) return ALPB_UNSUPPORTED;
+		set_error("alpb_cg_solve: %s", cudaGetErrorString(e));
+		return ALPB_PANIC;
+	}
 	ALPB_LAUNCHED();
 	ALPB_CUDA(cudaMemcpyAsync(h, a.st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
 	ALPB_CUDA(cudaFreeAsync(ws, s));
@@ -402,7 +444,7 @@ extern "C" int alpb_cg_solve(int64_t n, const int64_t *row_ptr, const uint32_t *
 	// 10^3 11.6 -> 7.7, 32^3 13.9 -> 7.6, 48^3 26 -> 11, 64^3 47 -> 17,
 	// 80^3 78 -> 50, 128^3 311 -> 199
 	const CgRowsShape c = plan->tile_d ? cg_rows_shape(n, int(plan->maxlen)) : CgRowsShape{};
-	if (c.grid > 0 && n < int64_t(CGR_NONE)) {
+	if (c.grid > 0 && n < int64_t(CGR_NONE) && cg_rows_pays(c, plan->nnz, max_iter)) {
 		CgRowsArgs a{};
 		a.offsets = row_ptr;
 		a.indices = col_idx;

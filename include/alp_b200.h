@@ -502,7 +502,12 @@ ALPB_API int alpb_reduce_f64(double *result, int op, int64_t n, const double *x,
  * x holds the initial guess on entry.  `work` is 4*n doubles of scratch
  * (16-byte aligned; otherwise, or when NULL, the solver allocates its own);
  * on return its first n doubles hold the final residual vector r.  Returns
- * ALPB_FAILED when not converged.  */
+ * ALPB_FAILED when not converged.  On short rows of similar length the solver
+ * takes up to 12 bytes per nonzero (rows padded to the longest), at most 8 GiB,
+ * from the device's stream-ordered pool, for the part of the matrix that does
+ * not stay on chip; it runs without them where they cannot be had.  After
+ * alpb_init the pool keeps them for the next solve (cudaMemPoolTrimTo gives
+ * them back).  */
 ALPB_API int alpb_cg_solve(int64_t n, const int64_t *row_ptr, const uint32_t *col_idx,
 	const double *values, const double *b, double *x, int64_t max_iter, double tol,
 	int64_t *iterations, double *residual, double *work, alpb_spmv_plan plan,

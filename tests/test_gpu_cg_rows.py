@@ -77,3 +77,45 @@ def test_cg_rows_budget_and_work_space(cuda, L, shift):
     assert abs(np.sqrt(rr) - float(r.norm())) <= 1e-13 * float(b.norm())
     if shift == 0:
         assert float((work - r).norm()) <= 1e-13 * float(b.norm())
+
+
+@pytest.mark.parametrize("steps", [1, 2, 3, 4, 5, 6])
+@pytest.mark.parametrize("sizes", [(40, 40, 40), (64, 64, 64), (80, 80, 80)])
+def test_few_iterations(cuda, sizes, steps):
+    """A handful of iterations runs on the matrix as it stands where rewriting it
+    would cost more than it saves: on both sides of that line the residual
+    belongs to x."""
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    A = dev.stencil(sizes, 27.0, -1.0)
+    b = dev.gen_values(A.m, abi.FP64, 7)
+    rc, x, it, rr, work = solve(A, b, steps, 1e-14)
+    assert rc == abi.FAILED and it == steps
+    r, nb = residual(A, b, x), float(b.norm())
+    assert abs(np.sqrt(rr) - float(r.norm())) <= 1e-13 * nb
+    assert float((work - r).norm()) <= 1e-13 * nb
+
+
+@pytest.mark.parametrize("sizes,rewritten", [((80, 80, 80), True), ((300, 300, 300), False)])
+def test_workspace_is_bounded(cuda, sizes, rewritten):
+    """The rewritten rows of an 80^3 grid come from the device's pool; those of
+    300^3 would be 8.7 GB, more than the 8 GiB that the solver takes, and it runs
+    without them."""
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    cu, pool = C.CDLL("libcuda.so.1"), C.c_void_p()
+    assert cu.cuDeviceGetDefaultMemPool(C.byref(pool), 0) == 0
+    A = dev.stencil(sizes, 27.0, -1.0)
+    b = dev.gen_values(A.m, abi.FP64, 7)
+    plan = dev.Plan(A, sched=abi.SCHED_MERGE_PATH)
+    torch.cuda.synchronize()
+    high = C.c_uint64(0)
+    assert cu.cuMemPoolTrimTo(pool, C.c_size_t(0)) == 0
+    assert cu.cuMemPoolSetAttribute(pool, 8, C.byref(high)) == 0    # USED_MEM_HIGH
+    rc, x, it, rr, work = solve(A, b, 8, 1e-14, plan=plan)
+    assert rc == abi.FAILED and it == 8
+    assert cu.cuMemPoolGetAttribute(pool, 8, C.byref(high)) == 0
+    assert (high.value > 12 * A.nnz // 2) == rewritten
+    assert abs(np.sqrt(rr) - float(work.norm())) <= 1e-13 * float(b.norm())
