@@ -1347,6 +1347,33 @@ static int launch_rows(const SpmvArgs &a, int maxlen, cudaStream_t s) {
 	return launch_rows_as<R, 2, 1, 7>(a, maxlen, s);
 }
 
+// Whether k_spmv_rows is the faster one, k_spmv_vector_dense's regular width being
+// the other.  Consecutive rows start a row's length apart in shared memory: even
+// lengths from 8 on meet in the same banks, and with differing lengths the lanes
+// wait for the longest row of the warp and the stages hold less.  The kernel's few
+// warps also gather with fewer loads in flight, which shows where the matrix is in
+// L2 or little beyond it.  Measured us, this / the other, FP64 unless said (L: row
+// length; matrices of diagonals and the stencils, Z: nonzeroes):
+//   L 5   8 M 32 / 25 (5-point 1200^2 31 / 25), 16 M 58 / 51, 24 M 82 / 105, 5-point
+//         2000^2 74 / 92, 3000^2 160 / 201; int32 8 M 19 / 23, 16 M 45 / 43, 48 M 117 / 168
+//   L 8   16 M 73 / 42, 48 M 195 / 181; random columns 78 / 47 (8 M)
+//   L 9   24 M 98 / 65, 48 M 189 / 201; pattern 16 M 52 / 45, 48 M 151 / 181
+//   L 13  24 M 86 / 69, 48 M 163 / 413; pattern 16 M 36 / 40
+//   L 19  8 M 26 / 33, 48 M 138 / 469; L 27 8 M 25 / 36, 48 M 135 / 186 (27-point
+//         130^3 165 / 242, int32 126 / 109, pattern 107 / 142); L 63 161 / 218
+//   8 to 24 random columns a row, 16 M 151 / 114; pattern 124 / 96
+template <class R>
+static bool rows_pay(const SpmvArgs &a, const alpb_spmv_plan_s &p) {
+	const int64_t len = int64_t(p.maxlen), vb = a.values ? int64_t(sizeof(typename R::T)) : 0;
+	if (!p.steady || (len >= 8 && len % 2 == 0)) return false;
+	if (len <= 2) return true;
+	const double bytes = double(a.nnz) * double(4 + vb) +
+		double(a.m_out) * double(8 + 3 * sizeof(typename R::T));
+	if (vb == 0) return len != 9 || bytes > 300e6;
+	if (vb <= 4) return len <= 7 && (bytes < 110e6 || bytes > 320e6);
+	return len > 16 || bytes > (len <= 7 ? 320e6 : 640e6);
+}
+
 static int default_width(double mean) {
 	int w = 1;
 	while (w < 32 && w * 2 <= mean * 0.75 + 1) w *= 2;
@@ -1388,7 +1415,7 @@ int run_spmv(const SpmvArgs &a, const alpb_spmv_plan_s *plan, int force_sched, c
 	}
 	// regular short rows: the row-streaming kernel (16-byte copies of the
 	// storage's ranges, so its arrays have to start on such a boundary)
-	if (fast && p && p->rows && !(reinterpret_cast<uintptr_t>(a.indices) & 15) &&
+	if (fast && p && p->can_rows && (p->rows < 0 ? rows_pay<R>(a, *p) : p->rows != 0) && !(reinterpret_cast<uintptr_t>(a.indices) & 15) &&
 		!(reinterpret_cast<uintptr_t>(a.values) & 15))
 		return launch_rows<R>(a, int(p->maxlen), s);
 	if (!fast) return launch_general<R>(a, p, W, s);
@@ -1542,7 +1569,7 @@ int alpb::plan_create_tiles(alpb_spmv_plan_s **plan, int64_t m, int64_t nnz,
 	p->small = sched == ALPB_SCHED_AUTO && !regular && nnz <= SMALL_NNZ && p->maxlen <= SMALL_ROW;
 	if (sched == ALPB_SCHED_AUTO) sched = regular ? ALPB_SCHED_VECTOR : ALPB_SCHED_MERGE_PATH;
 	p->sched = sched;
-	p->rows = regular && vector_width <= 0 && p->maxlen >= 1 && p->maxlen <= RS_MAX_LEN;
+	p->can_rows = regular && vector_width <= 0 && p->maxlen >= 1 && p->maxlen <= RS_MAX_LEN;
 	*plan = p;
 	return ALPB_SUCCESS;
 }
@@ -1724,12 +1751,13 @@ int alpb_spmv_autotune(alpb_spmv_plan p, int ring, int64_t n, const uint32_t *in
 	int nc = 0;
 	cands[nc++] = {ALPB_SCHED_MERGE_PATH, p->vw, false, false};
 	if (p->small) cands[nc++] = {ALPB_SCHED_MERGE_PATH, p->vw, false, true};
-	if (p->rows) cands[nc++] = {ALPB_SCHED_VECTOR, p->vw, true, false};
+	if (p->can_rows) cands[nc++] = {ALPB_SCHED_VECTOR, p->vw, true, false};
 	for (int w = 2; w <= 32; w *= 2) cands[nc++] = {ALPB_SCHED_VECTOR, w, false, false};
 	float best = 1e30f;
 	int best_i = 0;
 	const int saved_vw = p->vw;
-	const bool saved_rows = p->rows, saved_small = p->small;
+	const int saved_rows = p->rows;
+	const bool saved_small = p->small;
 	a.offsets = p->offsets;
 	for (int c = 0; c < nc; ++c) {
 		p->vw = cands[c].w;

@@ -10,7 +10,9 @@ struct alpb_spmv_plan_s {
 	int sched = ALPB_SCHED_VECTOR;
 	int vw = 8;
 	bool small = false;  // merge path by the plan's own choice: k_spmv_small instead
-	bool rows = false;   // vector schedule: short regular rows, streamed (rowstream.cuh)
+	// vector schedule: short regular rows, streamed (rowstream.cuh)
+	bool can_rows = false;   // the kernel holds this storage
+	int rows = -1;           // taken: 0 never, 1 always (tuned), -1 by rows_pay
 	bool steady = false;       // rows of nearly one length
 	bool hubs = false;         // some rows far longer than the others
 	bool given_width = false;  // vw is the caller's
