@@ -1566,7 +1566,9 @@ int alpb::plan_create_tiles(alpb_spmv_plan_s **plan, int64_t m, int64_t nnz,
 	// that no lane group should walk one: launch_general has the figures
 	p->steady = p->cv < 0.15;
 	p->hubs = !p->steady && p->maxlen > 256 && p->maxlen >= 8 * p->mean;
-	p->small = sched == ALPB_SCHED_AUTO && !regular && nnz <= SMALL_NNZ && p->maxlen <= SMALL_ROW;
+	p->own_vw = p->vw;
+	p->can_small = sched == ALPB_SCHED_AUTO && !regular && nnz <= SMALL_NNZ && p->maxlen <= SMALL_ROW;
+	p->small = p->can_small;
 	if (sched == ALPB_SCHED_AUTO) sched = regular ? ALPB_SCHED_VECTOR : ALPB_SCHED_MERGE_PATH;
 	p->sched = sched;
 	p->can_rows = regular && vector_width <= 0 && p->maxlen >= 1 && p->maxlen <= RS_MAX_LEN;
@@ -1746,11 +1748,14 @@ int alpb_spmv_autotune(alpb_spmv_plan p, int ring, int64_t n, const uint32_t *in
 	cudaEvent_t e0, e1;
 	ALPB_CUDA(cudaEventCreate(&e0));
 	ALPB_CUDA(cudaEventCreate(&e1));
-	// candidates: merge path, and vector widths around the mean row length
+	// candidates: merge path, and vector widths around the mean row length; the
+	// same ones whatever an earlier tuning chose
+	hot_release(p);
+	p->vw = p->own_vw;
 	struct Cand { int sched, w; bool rows, small; } cands[8];
 	int nc = 0;
 	cands[nc++] = {ALPB_SCHED_MERGE_PATH, p->vw, false, false};
-	if (p->small) cands[nc++] = {ALPB_SCHED_MERGE_PATH, p->vw, false, true};
+	if (p->can_small) cands[nc++] = {ALPB_SCHED_MERGE_PATH, p->vw, false, true};
 	if (p->can_rows) cands[nc++] = {ALPB_SCHED_VECTOR, p->vw, true, false};
 	for (int w = 2; w <= 32; w *= 2) cands[nc++] = {ALPB_SCHED_VECTOR, w, false, false};
 	float best = 1e30f;
@@ -1787,7 +1792,6 @@ int alpb_spmv_autotune(alpb_spmv_plan p, int ring, int64_t n, const uint32_t *in
 	p->small = cands[best_i].small;
 	// skewed rows on the merge path: try the hot-column cache at four sizes,
 	// up to what the shared memory left by the warps' tiles holds
-	hot_release(p);
 	if (p->sched == ALPB_SCHED_MERGE_PATH && p->tile == WM_TILE && n >= (int64_t(1) << 16) &&
 		p->nnz >= (int64_t(1) << 20)) {
 		constexpr int NH = 4;

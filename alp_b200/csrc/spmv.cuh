@@ -9,7 +9,9 @@ struct alpb_spmv_plan_s {
 	const int64_t *offsets = nullptr;  // storage the plan was made for
 	int sched = ALPB_SCHED_VECTOR;
 	int vw = 8;
-	bool small = false;  // merge path by the plan's own choice: k_spmv_small instead
+	int own_vw = 8;          // vw before any tuning
+	bool can_small = false;  // merge path by the plan's own choice: k_spmv_small holds it
+	bool small = false;      // and is taken
 	// vector schedule: short regular rows, streamed (rowstream.cuh)
 	bool can_rows = false;   // the kernel holds this storage
 	int rows = -1;           // taken: 0 never, 1 always (tuned), -1 by rows_pay

@@ -109,3 +109,32 @@ def test_structure_changed_in_place(cuda, kind, m, sparse):
         check(A, rp2, col2, vals, plan, rng, sparse)
         A.offsets.copy_(old[0])
         A.indices.copy_(old[1])
+
+
+@pytest.mark.parametrize("kind,m,n", [("skewed", 3000, 3000), ("skewed", 60, 20000), ("regular", 40, 500),
+                                      ("regular", 3000, 3000), ("regular", 200000, 200000)])
+def test_tuning_again_tries_the_same_kernels(cuda, kind, m, n):
+    """Whatever a tuning chose, the next one of the same plan, for another ring
+    too, launches the same candidates, and products stay right."""
+    import torch
+    from alp_b200 import _abi as abi
+    from alp_b200 import device as dev
+    rng = np.random.default_rng([m, n])
+    if kind == "skewed":
+        lens = np.minimum(rng.zipf(1.6, m), 4000)
+        lens[:3] = 4000, 300, 65
+    else:
+        lens = np.full(m, 5)
+    rp, col = storage(lens, n, rng)
+    vals = rng.random(len(col))
+    A = dev.from_host(m, n, rp, col, vals)
+    P = dev.CRS(m, n, A.nnz, A.offsets, A.indices, None, abi.VOID)
+    plan, counts = dev.Plan(A), []
+    for ring, M, dt in ((0, A, torch.float64), (2, P, torch.int32), (0, A, torch.float64)) * 3:
+        x, y = torch.ones(n, dtype=dt, device="cuda"), torch.zeros(m, dtype=dt, device="cuda")
+        before = abi.launches()
+        abi.call("alpb_spmv_autotune", plan.h, ring, n, dev.ptr(M.indices), dev.ptr(M.values), M.vtype,
+                 dev.ptr(x), dev.ptr(y), dev.stream_ptr())
+        counts.append(abi.launches() - before)
+        check(A, rp, col, vals, plan, rng, False)
+    assert len(set(counts)) == 1, counts
