@@ -411,7 +411,9 @@ __device__ __forceinline__ void chain_op(int op, T (&z)[B], const T (&a)[B], con
 // values wait in shared memory, [slot][batch][thread]: the steps name their
 // slots by number, and an array indexed so in registers went to local memory.
 // Two updates with a dot, a dot and two folds on 16e6 entries (1.3 GB): 791 us
-// then, 438 with one slot's loads waited for before the next, 391 now.
+// then, 438 with one slot's loads waited for before the next, 391 now.  Four
+// blocks per SM leave 64 registers: the 8-byte domains spill 116 to 132 bytes a
+// thread with B = VEC_BATCH, nothing with one entry.
 template <class T, int B>
 __global__ void __launch_bounds__(SCALAR_BLOCK, 4) k_vec_chain(ChainArgs<T> c, T init, VecOut out) {
 	extern __shared__ __align__(16) unsigned char chain_smem[];

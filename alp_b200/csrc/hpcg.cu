@@ -165,6 +165,8 @@ constexpr int HGC_CLUSTER = 16;     // blocks of a cluster launch
 // barrier is most of a step: 1.0 us there, 1.8 us through L2.  Measured us per
 // HPCG iteration, launches -> this: 16^3 with 8 right-hand sides 1451 -> 341,
 // 64^3 with 1 2499 -> 971, 64^3 with 8 4088 -> 1508, 128^3 with 8 10576 -> 8377.
+// 768 threads leave 80 registers each: two rows' entries in flight do not quite
+// fit, and 52 to 132 bytes a thread spill (what that costs was not measured apart).
 template <int NRHS, bool CLUSTER>
 __global__ void __launch_bounds__(HGC_THREADS, 1) k_hpcg_cycle(HgCycleArgs a) {
 	using Row = HgRow<NRHS>;

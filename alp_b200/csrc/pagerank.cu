@@ -317,13 +317,11 @@ __global__ void __launch_bounds__(32 * PRS_WARPS, 6) k_pr_step(PrStepArgs a, int
 	}
 }
 
-// residual and dangling mass in a fixed order; the next teleport term; stop
-// after an iteration whose residual is <= conv (:490) or at max_iter.
-// setup != 0: only the first term (no iteration has run).
-// The four sums of k_pr_finish in one pass: a thread's loads of all four
-// arrays are in flight together, and each sum keeps block_sum_array's order
-// (the thread's elements in stride order, then block_sum's tree), so the
+// The four sums that close an iteration in one pass: a thread's loads of all
+// four arrays are in flight together, and each sum keeps block_sum_array's
+// order (the thread's elements in stride order, then block_sum's tree), so the
 // values are those of four block_sum_array calls bit for bit.
+// setup != 0: the first teleport term only (no iteration has run).
 __device__ __forceinline__ void pr_finish_sums(const PrStepArgs &a, int setup,
 	double (*smem)[33], double out[4]) {
 	double v[4] = {0.0, 0.0, 0.0, 0.0};
@@ -356,7 +354,8 @@ __device__ __forceinline__ void pr_finish_sums(const PrStepArgs &a, int setup,
 	for (int q = 0; q < 4; ++q) out[q] = smem[q][32];
 }
 
-// One block: the sums, the next teleport term, and whether to stop.
+// One block: the sums, the next teleport term, and whether to stop: after an
+// iteration whose residual is <= conv (:490), or at max_iter.
 __device__ __forceinline__ void pr_finish(const PrStepArgs &a, int setup) {
 	__shared__ double red[4][33];
 	PrStepState *st = a.st;

@@ -17,9 +17,9 @@ struct alignas(128) GridSync {
 	unsigned int pad1[30];
 };
 
-// A few seconds of polls (each an L2 round trip of about 0.2 us): far beyond any
-// legitimate wait of a co-resident grid, short enough to keep the context
-// usable on a fault.
+// A few seconds of polls (each an L2 round trip of about 0.2 us; grid_reduce
+// waits an eighth of that): far beyond any legitimate wait of a co-resident
+// grid, short enough to keep the context usable on a fault.
 constexpr long long kSpinLimit = 1ll << 24;
 
 // All blocks of a cooperative launch call this the same number of times.

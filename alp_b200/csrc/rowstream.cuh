@@ -16,7 +16,8 @@
 namespace alpb {
 
 // Measured us per product (4 lanes per row before): 27-point 129 x 127 x 131
-// 299 -> 164, 5-point 2000^2 92 -> 74.  27-point with 10 / 14 / 20 warps per SM
+// 299 -> 164, 5-point 2000^2 92 -> 74; rows_pay (spmv.cu) says where the lanes
+// are the faster ones.  27-point with 10 / 14 / 20 warps per SM
 // 224 / 185 / 165 (24 are what the registers allow, about 20 what the stages
 // of 27-point rows allow), with one / four lanes a row 176 / 193, with three
 // stages 193.
