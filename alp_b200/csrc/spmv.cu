@@ -365,6 +365,7 @@ constexpr int LOR_CHUNK = 256;
 // general path (k_spmv_vector_general): rows longer than GEN_LONG run in
 // chunks of GEN_CHUNK, a lane's loads in batches of GEN_BATCH
 constexpr int GEN_LONG = 64;
+constexpr int64_t GEN_FEW = int64_t(1) << 15;   // see launch_general
 constexpr int GEN_CHUNK = 256;
 constexpr int GEN_BATCH = 4;
 constexpr int64_t GEN_NARROW = int64_t(1) << 20;   // see launch_general
@@ -778,39 +779,38 @@ struct GenRow {
 template <class R, int W, bool BITS = false, int BATCH = BITS ? GEN_BATCH_BITS : GEN_BATCH>
 __device__ __forceinline__ void gen_gather(const SpmvArgs &a, int64_t b, int64_t e, int lane,
 	typename R::T &acc, bool &set, const uint32_t *bits = nullptr) {
-	constexpr int GEN_BATCH = BATCH;
 	using T = typename R::T;
 	const T *__restrict__ values = reinterpret_cast<const T *>(a.values);
 	const T *__restrict__ x = reinterpret_cast<const T *>(a.v);
 	const bool use_index = (a.descr & ALPB_DESC_USE_INDEX) != 0;
 	const uint8_t *__restrict__ va = (a.descr & ALPB_DESC_DENSE) ? nullptr : a.v_assigned;
-	for (int64_t k0 = b + lane; k0 < e; k0 += GEN_BATCH * W) {
-		uint32_t j[GEN_BATCH];
-		bool on[GEN_BATCH];
-		T xv[GEN_BATCH], av[GEN_BATCH];
+	for (int64_t k0 = b + lane; k0 < e; k0 += BATCH * W) {
+		uint32_t j[BATCH];
+		bool on[BATCH];
+		T xv[BATCH], av[BATCH];
 #pragma unroll
-		for (int q = 0; q < GEN_BATCH; ++q) {
+		for (int q = 0; q < BATCH; ++q) {
 			on[q] = k0 + q * W < e;
 			j[q] = on[q] ? __ldcs(a.indices + k0 + q * W) : 0u;
 		}
 		if (BITS) {
 #pragma unroll
-			for (int q = 0; q < GEN_BATCH; ++q)
+			for (int q = 0; q < BATCH; ++q)
 				if (on[q]) on[q] = (bits[j[q] >> 5] >> (j[q] & 31)) & 1u;
 		}
 		if (!BITS && a.input_masked) {
 #pragma unroll
-			for (int q = 0; q < GEN_BATCH; ++q)
+			for (int q = 0; q < BATCH; ++q)
 				if (on[q])
 					on[q] = eval_mask(a.v_mask, a.v_mask_assigned, a.v_mask_type, a.descr, j[q]);
 		}
 		if (!BITS && va) {
 #pragma unroll
-			for (int q = 0; q < GEN_BATCH; ++q)
+			for (int q = 0; q < BATCH; ++q)
 				if (on[q]) on[q] = va[j[q]] != 0;
 		}
 #pragma unroll
-		for (int q = 0; q < GEN_BATCH; ++q) {
+		for (int q = 0; q < BATCH; ++q) {
 			xv[q] = R::zero();
 			av[q] = R::one();
 			if (on[q]) {
@@ -819,7 +819,7 @@ __device__ __forceinline__ void gen_gather(const SpmvArgs &a, int64_t b, int64_t
 			}
 		}
 #pragma unroll
-		for (int q = 0; q < GEN_BATCH; ++q)
+		for (int q = 0; q < BATCH; ++q)
 			if (on[q]) {
 				acc = R::add(a.left ? R::mull(xv[q], av[q]) : R::mulr(av[q], xv[q]), acc);
 				set = true;
@@ -916,9 +916,9 @@ __global__ void k_pack_present(SpmvArgs a, uint32_t *bits) {
 // How the general kernel runs.  GEN_CHUNKS: flags asked in memory, long rows in
 // chunks (or none listed).  GEN_BLOCKS: the same, but the first blocks take a listed
 // row each.  GEN_BITS: as GEN_CHUNKS, and every block copies the inputs' bits into its
-// shared memory first.  A nonzero then asks shared memory whether its input takes part (a warp's 32
-// random words are about four wavefronts there, and up to 32 in L1), and only
-// those that do gather x.
+// shared memory first.  A nonzero then asks shared memory whether its input takes
+// part (a warp's 32 random words are about four wavefronts there, and up to 32 in
+// L1), and only those that do gather x.
 enum { GEN_CHUNKS, GEN_BLOCKS, GEN_BITS };
 template <class R, int W, int MODE>
 __global__ void __launch_bounds__(MODE == GEN_BITS ? 1024 : 256)
@@ -1164,11 +1164,13 @@ int launch_vector_dense_w(const SpmvArgs &a, cudaStream_t s) {
 constexpr int64_t GEN_BITS_NNZ = int64_t(1) << 21;
 constexpr int64_t GEN_BITS_MAX = 200 * 1024 * 8;
 
-// Below this many nonzeroes the listed rows run a block each in the one launch:
-// the partials' memory and the finish pass cost a small product more than the
-// chip they fill (R-MAT, min-plus from a 20% sparse vector, us, blocks / chunks:
-// 20,000 vertices, 0.23 M nonzeroes, 16 / 23; 100,000, 1.4 M, 34 / 28).
+// Below this many nonzeroes, in rows of up to GEN_BLOCK_LEN, the listed rows run a
+// block each in the one launch: the partials' memory and the finish pass cost a
+// small product more than the chip they fill (us, blocks / chunks: R-MAT, min-plus
+// from a 20% sparse vector, 20,000 vertices, 0.23 M nonzeroes, 16 / 23, 100,000, 1.4 M,
+// 34 / 28; FP64, 4 to 64 rows of 1,000 12 / 16, of 8,000 19 / 16, of 100,000 172 / 18).
 constexpr int64_t GEN_SCRATCH_NNZ = int64_t(1) << 20;
+constexpr int64_t GEN_BLOCK_LEN = 6144;
 static_assert(GEN_SCRATCH_NNZ <= GEN_BITS_NNZ, "the kernel with the bits takes chunks");
 
 // A call under stream capture takes no scratch: its graph would hold allocation
@@ -1202,7 +1204,8 @@ int launch_general_w(const SpmvArgs &a, const alpb_spmv_plan_s *p, bool lists, c
 	uint32_t *bits = nullptr;
 	const bool want_bits = gen_filtered(a) && a.nnz >= GEN_BITS_NNZ && a.n_in <= GEN_BITS_MAX;
 	const size_t bit_bytes = want_bits ? size_t(a.n_in + 127) / 128 * 16 : 0;
-	const int64_t chunks = lists && a.nnz >= GEN_SCRATCH_NNZ ? p->gen_n : 0;
+	const int64_t chunks = lists && (a.nnz >= GEN_SCRATCH_NNZ || p->maxlen > GEN_BLOCK_LEN)
+		? p->gen_n : 0;
 	if ((bit_bytes || chunks) && !capturing(s)) {
 		// bits, then the partials of the long rows' chunks: this call's own
 		// (calls on other streams may use the same plan); without them the
@@ -1284,18 +1287,21 @@ static int with_width(int W, const F &f) {
 	}
 }
 
-// The general path.  Which kernel: k_spmv_vector_plain without a plan, for rows
-// of nearly one length, and for matrices without hub rows whose width the caller
-// gave or that are small; measured us, plain / the other, min-plus from a 20%
-// sparse vector unless said:
-//   hub rows, R-MAT 100,000 vertices 373 / 28, lognormal rows 300,000 118 / 50
-//   (under a mask, FP64, 2,000,000: 265 / 288); lists for rows that are merely
-//   longer than GEN_LONG cost more than they give (rows of 200: 82 / 93,
-//   of 0 to 100: 122 / 124, 74 without the lists);
-//   random rows, no hubs, from GEN_NARROW nonzeroes on: mean 16 and 1,000,000 rows
-//   110 / 70, mean 30 and 300,000 rows 74 / 45; where the inputs' flags do not fit as
-//   bits, mean 16 and 3,000,000 rows (2 lanes) 314 / 382 (478 / 344 in FP64), mean 30
-//   and 2,000,000 rows 462 / 528: from 8 lanes on the plain one;
+// The general path.  Which kernel: k_spmv_vector_plain without a plan and, where no
+// row is in the lists' way, for rows of nearly one length, small matrices, given
+// widths and rows of more than 128.  Measured us, plain / the other, min-plus from a
+// 20% sparse vector unless said:
+//   lists: R-MAT 100,000 vertices 373 / 28, lognormal rows 300,000 118 / 50 (under a
+//   mask, FP64, 2,000,000: 265 / 288); few rows or long ones, FP64 from all inputs:
+//   16 rows of 1,000 23 / 12, 1,000 rows of 8,000 278 / 54, 4,000 311 / 167, 16,000 rows
+//   of 1,000 119 / 101, 8,000 of up to 1,000 39 / 41, of up to 600 25 / 32; rows that are
+//   merely longer than GEN_LONG lose by them (100,000 rows of 200: 82 / 93, 300,000 of
+//   0 to 100: 122 / 124, 74 without the lists);
+//   random rows without lists, from GEN_NARROW nonzeroes on: mean 16 and 1,000,000 rows
+//   110 / 70, mean 30 and 300,000 rows 74 / 45, FP64 up to 300 and 8,000 rows 17 / 19, up
+//   to 600 25 / 42; where the inputs' flags do not fit as bits, mean 16 and 3,000,000
+//   rows (2 lanes) 314 / 382 (478 / 344 in FP64), mean 30 and 2,000,000 rows 462 / 528:
+//   from 8 lanes on the plain one;
 //   one length: 27-point 117^3 116 / 274, 5-point 1200^2 37 / 57, rows of 200 as above.
 // A lane waits for its row's chain of loads, so from GEN_NARROW nonzeroes on a
 // quarter of the lanes per row, and four times the rows in flight, is faster
@@ -1306,8 +1312,8 @@ static bool gen_no_bits(const SpmvArgs &a) { return gen_filtered(a) && a.n_in > 
 template <class R>
 int launch_general(const SpmvArgs &a, const alpb_spmv_plan_s *p, int W, cudaStream_t s) {
 	const bool lists = p && p->hubs && p->gen_n > 0;
-	if (!p || p->steady ||
-		(!lists && (p->given_width || a.nnz < GEN_NARROW || (W >= 8 && gen_no_bits(a)))))
+	if (!p || (!lists && (p->steady || p->given_width || a.nnz < GEN_NARROW || p->maxlen > 128 ||
+			(W >= 8 && gen_no_bits(a)))))
 		return with_width(W, [&](auto w) { return launch_plain_w<R, decltype(w)::value>(a, s); });
 	if (!p->given_width && a.nnz >= GEN_NARROW && W >= 4) W /= 4;
 	return with_width(W, [&](auto w) {
@@ -1562,10 +1568,12 @@ int alpb::plan_create_tiles(alpb_spmv_plan_s **plan, int64_t m, int64_t nnz,
 		p->vw = regular ? regular_width(p->mean) : default_width(p->mean);
 	}
 	p->given_width = vector_width > 0;
-	// rows of nearly one length (stencils with their boundaries), and rows so long
-	// that no lane group should walk one: launch_general has the figures
+	// rows of nearly one length (stencils with their boundaries), and rows that no
+	// lane group should walk: far longer than the others, long where a group per row
+	// leaves the chip idle, or long by themselves.  launch_general has the figures
 	p->steady = p->cv < 0.15;
-	p->hubs = !p->steady && p->maxlen > 256 && p->maxlen >= 8 * p->mean;
+	p->hubs = p->maxlen > 256 && ((!p->steady && p->maxlen >= 8 * p->mean) ||
+		p->m * p->vw < GEN_FEW || p->maxlen >= 768);
 	p->own_vw = p->vw;
 	p->can_small = sched == ALPB_SCHED_AUTO && !regular && nnz <= SMALL_NNZ && p->maxlen <= SMALL_ROW;
 	p->small = p->can_small;

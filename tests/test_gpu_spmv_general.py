@@ -317,3 +317,41 @@ def test_dense_descriptor_ignores_flags_at_every_size(cuda, oracle, ring):
         np.testing.assert_allclose(got.cpu().numpy(), want, rtol=3e-14, atol=0)
     else:
         np.testing.assert_array_equal(got.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("ring", [0, 1, 2])
+@pytest.mark.parametrize("m,length", [(4, 100000), (16, 1000), (64, 6144), (64, 6145), (2000, 767),
+                                      (2000, 768), (40, 256), (40, 257), (9000, 129)])
+def test_few_or_long_rows(cuda, oracle, ring, m, length):
+    """Long rows of one length: walked, a block each, or in chunks, at the edges
+    of those rules.  FP64 sums of n positive terms: 2 n 2^-53 relative."""
+    import torch
+    from alp_b200 import device as dev
+    vtype = {0: 3, 1: 1, 2: 2}[ring]
+    npt = {3: np.float64, 2: np.int32, 1: np.uint8}[vtype]
+    rng = np.random.default_rng([ring, m, length])
+    n = 30011
+    rp = (np.arange(m + 1) * length).astype(np.int64)
+    col = rng.integers(0, n, int(rp[-1])).astype(np.uint32)
+    value = lambda k: (rng.random(k) if vtype == 3 else rng.integers(0, 2 if vtype == 1 else 1000, k)).astype(npt)  # noqa: E731
+    vals, u, v = value(len(col)), value(m), value(n)
+    T = lambda a: torch.from_numpy(a.copy()).cuda()  # noqa: E731
+    A = dev.from_host(m, n, rp, col, vals, vtype)
+    plan = dev.Plan(A)
+    mask = (rng.random(m) < 0.7).astype(np.uint8)
+    for frontier in (0.001, 0.3):
+        va, ua = (rng.random(n) < frontier).astype(np.uint8), (rng.random(m) < 0.5).astype(np.uint8)
+        wu, wa = u.copy(), ua.copy()
+        kw = dict(u_mask_count=int(mask.sum()))
+        rc, wn = oracle.mxv(ring, 0, 0, m, n, rp, col, vals, vtype, wu, wa, v=v, v_assigned=va,
+                            u_mask=mask, u_mask_assigned=mask, **kw)
+        assert rc == 0
+        gu, ga, gn = T(u), T(ua), torch.tensor([int(ua.sum())], dtype=torch.int64, device="cuda")
+        dev.mxv(ring, A, gu, T(v), form=0, u_assigned=ga, u_nnz=gn, v_assigned=T(va), plan=plan,
+                u_mask=T(mask), u_mask_assigned=T(mask), **kw)
+        assert np.array_equal(ga.cpu().numpy() != 0, wa != 0) and int(gn) == wn
+        got, want = gu.cpu().numpy()[wa != 0], wu[wa != 0]
+        if vtype == 3:
+            np.testing.assert_allclose(got, want, rtol=2 * length * 2.0 ** -53, atol=0)
+        else:
+            np.testing.assert_array_equal(got, want)
