@@ -141,6 +141,8 @@ typedef struct alpb_spmv_plan_s *alpb_spmv_plan;
  * memory pool then keeps the stream-ordered scratch that entry points free
  * (its release threshold is raised), so that repeated calls reuse it. */
 ALPB_API int alpb_init(int device);
+/* Waits for the device, and gives back the reduction scratch (8 KB per thread
+ * that ever reduced at the same time as others) that no running thread holds. */
 ALPB_API int alpb_finalize(void);
 ALPB_API const char *alpb_last_error(void);
 ALPB_API int alpb_version(void);
