@@ -9,9 +9,10 @@
 //    list is cut in equal tiles (Merrill & Garland, "Merge-based parallel
 //    sparse matrix-vector multiplication", SC'16), so power-law rows cost the
 //    same as uniform ones; one launch, sums in a fixed order (deterministic).
-//  * vector: regular short rows stream through shared memory (rowstream.cuh),
-//    others take W lanes per row; the general path, W lanes per row with long
-//    rows cut in chunks, carries every ALP semantic of the reference gather:
+//  * vector: short rows of nearly one length stream through shared memory where
+//    that is faster (rowstream.cuh, rows_pay), others take W lanes per row; the
+//    general path (launch_general: W lanes walking a row, or batched with long
+//    rows cut in chunks) carries every ALP semantic of the reference gather:
 //    output/input masks (value or structural, inverted), sparse input and
 //    output vectors with assigned flags, add_identity, use_index,
 //    explicit_zero and the immutable-nonzero shortcut of lor.
